@@ -80,6 +80,8 @@ struct Geo {
   float fx_scale;    // 2^s: chord length -> fixed point units
   float fx_inv;      // 2^-s
   int fx_split;      // units = hi * 2^fx_split + lo, both parts summed in 32 bits
+  float inv_pitch[3];  // 1 / grid pitch (approximate)
+  bool check_window;   // grid too fine for the window's margin: every cell tested
 };
 
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }

@@ -10,6 +10,7 @@
 #include <curand_kernel.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "internal.h"
@@ -149,6 +150,26 @@ Geo make_geo(const epet_problem& p) {
   G.fx_scale = ldexpf(1.0f, s);
   G.fx_inv = ldexpf(1.0f, -s);
   G.fx_split = b;
+  for (int a = 0; a < 3; a++) G.inv_pitch[a] = 1.f / p.grid.d[a];
+  // The walk's windows leave a margin of 1e-3 voxel around the crystals'
+  // hull; a crossing's position carries a few roundings of the largest
+  // coordinate (2^-24 of it each).  Cells need no test against the window
+  // while 16 such roundings fit the margin (a pitch of 0.3 mm for heads
+  // 0.25 m away; the workloads' 2 mm leave a factor of 7).
+  double reach = 0.0;
+  for (double v : {(double)p.setup.pos0x, (double)p.setup.pos1x})
+    reach = std::max(reach, std::fabs(v) + p.setup.segx);
+  reach = std::max(reach, 0.5 * p.setup.segy * std::max(p.setup.n0y, p.setup.n1y));
+  reach = std::max(reach, 0.5 * p.setup.segz * std::max(p.setup.n0z, p.setup.n1z)) * 1.5;
+  double pitch = p.grid.d[0];
+  for (int a = 0; a < 3; a++) {
+    pitch = std::min(pitch, (double)p.grid.d[a]);
+    reach = std::max(reach, std::fabs((double)p.grid.o[a]));
+    reach = std::max(reach, std::fabs((double)p.grid.o[a] + (double)p.grid.n[a] * p.grid.d[a]));
+  }
+  // (cell indices from reciprocal pitches carry 2^-23 of their size: up to
+  // 2^11 cells along y; the walk takes at most 2^10 along x and z)
+  G.check_window = !(16.0 * std::ldexp(reach, -24) < 1e-3 * pitch) || p.grid.n[1] > 2048;
   return G;
 }
 

@@ -82,31 +82,40 @@ struct WalkArgs {
 };
 
 // Dynamic shared memory of the walk kernel: the grid-plane table, the per-row
-// z terms of the candidate test and the pool, each on a 256-byte boundary.
-// The pool holds, per channel, the window's column table (8 bytes per
-// column, border included) followed by the two 32-bit sum words of every
-// window cell and of the two trash cells (8 bytes per cell): a channel needs
-// columns + cells + 2 <= cap_cells.
+// z terms of the candidate test, the slab runs of every x and y (z slabs only)
+// and the pool, each on a 256-byte boundary.  The pool holds,
+// per channel, the window's column tables (8 bytes per column, border
+// included) followed by the two 32-bit sum words of every window cell and of
+// the two trash cells (8 bytes per cell): a channel needs columns + cells + 2
+// <= cap_cells.  Guard bands keep a ray's table and cell addresses inside the
+// pool wherever the walk can take them (walk_ray): `gcol` bytes before the
+// column tables (a row of the table and an entry, filled like empty columns)
+// and `gz` bytes (the z cells) before and after the cells.
 struct WalkLayout {
-  size_t planes, ztab, pool, pext, lines, slabs, total;
+  size_t planes, ztab, runs, pool, pext, lines, slabs, total;
+  int gcol, gz;
 };
-constexpr int kHullLines = 64;  // crystal-corner pair lines of the hull
-// nplanes: grid planes of all three axes (n0 + n1 + n2 + 3); nz: z cells.
-// The pool holds the column table and the cells.  Three arrays that die
-// early share it: the hull extents at the slab planes (pext, at its start)
-// and the hull lines' parameters after them are read only while the slab
-// windows are built, and the slab windows (slabs, at its end) only until the
-// column table is built, so the table must end before them and the cells,
-// written afterwards, may run over them.
-__host__ __device__ inline WalkLayout walk_layout(int nslab, int nplanes, int nz, int cap_cells) {
+constexpr int kHullLines = 16;  // lines of the hull joining the crystals' vertical edges
+// Three arrays that die early share the pool: the
+// hull extents at the slab planes (pext, at its start) and the hull lines'
+// parameters after them are read only while the slab windows are built, and
+// the slab windows (slabs, at its end) only until the column table is built,
+// so the table must end before them and the cells, written afterwards, may
+// run over them.
+__host__ __device__ inline WalkLayout walk_layout(const epet_grid& g, int cap_cells) {
+  const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
+  const int nslab = nx > nz ? nx : nz;
   WalkLayout L;
+  L.gcol = ((ny + 2) * 4 + 15) & ~15;
+  L.gz = ((nz + 4) * 4 + 15) & ~15;
   L.planes = 0;
-  L.ztab = L.planes + align256((size_t)(nplanes + 2) * 4);  // + a guard entry at each end
-  L.pool = L.ztab + align256((size_t)nz * 8);
+  L.ztab = L.planes + align256((size_t)(nx + ny + nz + 5) * 4);  // + a guard entry at each end
+  L.runs = L.ztab + align256((size_t)nz * 8);
+  L.pool = L.runs + align256((size_t)2 * (nx + ny) * 4);
   const size_t pext_b = ((size_t)(nslab + 1) * 16 + 15) & ~size_t(15);
-  const size_t slab_b = ((size_t)20 * nslab + 15) & ~size_t(15);
-  const size_t line_b = (size_t)6 * kHullLines * 4;
-  size_t pool_b = (size_t)cap_cells * 8;
+  const size_t slab_b = (size_t)16 * nslab;
+  const size_t line_b = (size_t)kHullLines * 16;
+  size_t pool_b = (size_t)cap_cells * 8 + L.gcol + 2 * L.gz;
   if (pool_b < pext_b + line_b + slab_b) pool_b = pext_b + line_b + slab_b;
   pool_b = (pool_b + 15) & ~size_t(15);
   L.pext = L.pool;
@@ -122,7 +131,6 @@ __host__ __device__ inline WalkLayout walk_layout(int nslab, int nplanes, int nz
 // rectangle [p0, p0+wp) x [q0, q0+wq) over the other two axes
 // (sa = 0: p = y, q = z; sa = 2: p = x, q = y).
 struct Slab {
-  int off;  // first cell
   int p0, wp;
   int q0, wq;
 };
@@ -131,22 +139,23 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) {
   return v < lo ? lo : (v > hi ? hi : v);
 }
 
-// Block-wide exclusive scan of one int per thread (kWalkThreads threads).
+// Block-wide exclusive scan of one int per thread (kWalkThreads threads) with
+// one barrier; warp_tot (kWalkThreads / 32 ints) is the call's own: it must
+// not be reused before another barrier.
 __device__ __forceinline__ int block_excl_scan(int v, int* warp_tot, int* total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  int inc = warp_incl_scan(v);
+  const int inc = warp_incl_scan(v);
   if (lane == 31) warp_tot[w] = inc;
   __syncthreads();
-  if (w == 0) {
-    int t = lane < (kWalkThreads / 32) ? warp_tot[lane] : 0;
-    int ti = warp_incl_scan(t);
-    if (lane < (kWalkThreads / 32)) warp_tot[lane] = ti - t;
-    if (lane == (kWalkThreads / 32) - 1) *total = ti;
+  int before = 0, all = 0;
+#pragma unroll
+  for (int k = 0; k < kWalkThreads / 32; k++) {
+    const int t = warp_tot[k];
+    before += k < w ? t : 0;
+    all += t;
   }
-  __syncthreads();
-  int r = warp_tot[w] + inc - v;
-  __syncthreads();
-  return r;
+  *total = all;
+  return before + inc - v;
 }
 
 // Order-preserving float <-> int keys for warp min/max reductions.
@@ -159,29 +168,32 @@ __device__ __forceinline__ float fval(int k) {
 }
 
 // Index window of slab i along axis sa from the hull's cross-sections at its
-// two planes (pext[k] = {pmin, pmax, qmin, qmax} keys at plane k) and the
-// hull vertices (crystal corners) inside the slab.  An index range is
-// widened by one only on a side whose extreme lies within kWinPad (in
-// voxels) of a grid plane, where the rounding of the hull's or a ray's
-// arithmetic could put a hit in the neighbouring cell (both are ~1e-6 voxel
-// here); the window then holds about 1.7x a row's non-zeros instead of 3.9x
-// with a voxel of padding on every side (channels of the full workload).
-// A hit outside the window is still counted and reported (hit_outside).
+// two planes (pext[k] = {pmin, pmax, qmin, qmax} keys at plane k) and, unless
+// the grid lies between the crystals (`spans`), the hull vertices (crystal
+// corners) inside the slab.  An index range is widened by one only on a side
+// whose extreme lies within kWinPad (in voxels) of a grid plane, where the
+// rounding of the hull's or a ray's arithmetic could put a hit in the
+// neighbouring cell (a few 1e-6 voxel here, a few 1e-4 at the largest index
+// counts: Geo::check_window); the window then holds about 1.7x a row's
+// non-zeros instead of 3.9x with a voxel of padding on every side (channels
+// of the full workload).
 __device__ void slab_window(const Geo& G, const float (*c0)[3], const float (*c1)[3],
-                            const int4* pext, int sa, int i, Slab* out) {
+                            const int4* pext, bool spans, int sa, int i, Slab* out) {
   const epet_grid& g = G.p.grid;
   const int pa = sa == 0 ? 1 : 0, qa = sa == 0 ? 2 : 1;
-  const float P0 = voxel_plane(g, sa, i), P1 = voxel_plane(g, sa, i + 1);
   int plo = min(pext[i].x, pext[i + 1].x), phi = max(pext[i].y, pext[i + 1].y);
   int qlo = min(pext[i].z, pext[i + 1].z), qhi = max(pext[i].w, pext[i + 1].w);
-  for (int k = 0; k < 8; k++) {
-    if (c0[k][sa] >= P0 && c0[k][sa] <= P1) {
-      plo = min(plo, fkey(c0[k][pa])); phi = max(phi, fkey(c0[k][pa]));
-      qlo = min(qlo, fkey(c0[k][qa])); qhi = max(qhi, fkey(c0[k][qa]));
-    }
-    if (c1[k][sa] >= P0 && c1[k][sa] <= P1) {
-      plo = min(plo, fkey(c1[k][pa])); phi = max(phi, fkey(c1[k][pa]));
-      qlo = min(qlo, fkey(c1[k][qa])); qhi = max(qhi, fkey(c1[k][qa]));
+  if (!spans) {
+    const float P0 = voxel_plane(g, sa, i), P1 = voxel_plane(g, sa, i + 1);
+    for (int k = 0; k < 8; k++) {
+      if (c0[k][sa] >= P0 && c0[k][sa] <= P1) {
+        plo = min(plo, fkey(c0[k][pa])); phi = max(phi, fkey(c0[k][pa]));
+        qlo = min(qlo, fkey(c0[k][qa])); qhi = max(qhi, fkey(c0[k][qa]));
+      }
+      if (c1[k][sa] >= P0 && c1[k][sa] <= P1) {
+        plo = min(plo, fkey(c1[k][pa])); phi = max(phi, fkey(c1[k][pa]));
+        qlo = min(qlo, fkey(c1[k][qa])); qhi = max(qhi, fkey(c1[k][qa]));
+      }
     }
   }
   out->p0 = out->q0 = 0;
@@ -197,10 +209,10 @@ __device__ void slab_window(const Geo& G, const float (*c0)[3], const float (*c1
     const float fl = floorf(f);
     return (int)fl + (f - fl > 1.f - kWinPad ? 1 : 0);
   };
-  int a0 = lo_index((pmin - g.o[pa]) / g.d[pa]);
-  int a1 = hi_index((pmax - g.o[pa]) / g.d[pa]);
-  int b0 = lo_index((qmin - g.o[qa]) / g.d[qa]);
-  int b1 = hi_index((qmax - g.o[qa]) / g.d[qa]);
+  int a0 = lo_index((pmin - g.o[pa]) * G.inv_pitch[pa]);
+  int a1 = hi_index((pmax - g.o[pa]) * G.inv_pitch[pa]);
+  int b0 = lo_index((qmin - g.o[qa]) * G.inv_pitch[qa]);
+  int b1 = hi_index((qmax - g.o[qa]) * G.inv_pitch[qa]);
   if (a1 < 0 || a0 > np - 1 || b1 < 0 || b0 > nq - 1) return;
   a0 = clampi(a0, 0, np - 1); a1 = clampi(a1, 0, np - 1);
   b0 = clampi(b0, 0, nq - 1); b1 = clampi(b1, 0, nq - 1);
@@ -216,44 +228,36 @@ __device__ void slab_window(const Geo& G, const float (*c0)[3], const float (*c1
 // hi * 2^fx_split + lo and the halves are summed separately with
 // fire-and-forget 32-bit shared atomics; the split is sized (make_geo) so
 // neither half can overflow.  The total (hi_sum << fx_split) + lo_sum is
-// exact and independent of the order of the adds.
+// exact and independent of the order of the adds.  The lo words and the hi
+// words are two arrays, so that a warp's adds spread over all 32 banks
+// (interleaved, each of the two adds had only 16).
 struct Window {
-  uint2* cell;  // per cell {lo, hi} sum words
-  // per column: {first cell, zlo | zn << 16}; empty: zn 0.  The table has
-  // (wbx + 1) x (wby + 1) entries (row stride wbyp = wby + 1): the last
-  // column of each row and the last row are empty and stand for every
-  // column outside the box.
-  const int2* cols;
-  const float* planes;  // grid planes: x at [0, n0], y at poff1 + [0, n1], z at poff2 + ...
+  uint32_t *lo, *hi;  // per cell sum words (lo, then hi, W + 2 each)
+  // per column k: the shared address of the lo word of its cell z = 0 (which
+  // need not be in the run), and zlo | zn << 16 (empty: zn 0).  The tables
+  // have (wbx + 1) x (wby + 1) entries (row stride wbyp = wby + 1); the last
+  // column of each row and the last row are empty.
+  const uint32_t* cbase;
+  const uint32_t* zrun;
+  uint32_t cbase_s;  // shared address of cbase
+  uint32_t hioff;    // bytes from a lo word to its hi word
+  // grid planes: x at [0, n0], y at poff1 + [0, n1], z at poff2 + [0, n2]
+  const float* planes;
+  uint32_t planes_s;  // shared address of planes
   int poff1, poff2;
   int bx0, by0, wbx, wby, wbyp;
   int split;
-  int trash;      // cell W: absorbs the adds of steps with nothing to add (never read)
-  int trash_out;  // cell W + 1: counts (in lo) hits outside the window (must stay 0)
+  int trash_out;  // cell W: counts (in lo) hits outside the window (must stay 0)
+  bool test_all;  // every ray's cells must be tested against the window
 };
-
-// A lane's cached column: first cell, first z, number of z cells.
-struct Col {
-  int off, zlo, zn;
-};
-// Column (cx, cy) relative to the box corner; outside the box: an empty
-// border entry (both indices clamped, unsigned, to the border).
-__device__ __forceinline__ Col load_col(const Window& w, int cx, int cy) {
-  const unsigned ux = min((unsigned)cx, (unsigned)w.wbx), uy = min((unsigned)cy, (unsigned)w.wby);
-  const int2 e = w.cols[ux * w.wbyp + uy];
-  Col c;
-  c.off = e.x;
-  c.zlo = e.y & 0xffff;
-  c.zn = e.y >> 16;
-  return c;
-}
 
 // One axis of a ray walk: the ray's parameter at grid plane k is the
 // reference's quotient (plane_k - r0)/(r1 - r0), correctly rounded.
 struct WalkAxis {
   const float* P;           // plane positions o + k*d, k = 0..n (the shared table)
-  float o, d, r0, dr, inv;  // ray at r0 + a*dr; inv = RN(1/dr)
-  int n, step;
+  float o, r0, dr, inv;     // ray at r0 + a*dr; inv = RN(1/dr)
+  float inv_d;              // 1 / d (approximate)
+  int n;
   float lo, hi;  // parameter interval of the current cell along this axis
   int kn;        // index of the plane at hi (cell + 1 ascending, cell descending)
   __device__ __forceinline__ float alpha(int k) const { return div_cr(fsub(P[k], r0), dr, inv); }
@@ -261,9 +265,9 @@ struct WalkAxis {
   // guess only starts the search, which corrects it either way; the
   // parameters of the cell's two planes are carried along the search
   __device__ __forceinline__ void enter(float a) {
-    int i = clampi((int)floorf(__fdividef(r0 + a * dr - o, d)), 0, n - 1);
+    int i = clampi((int)floorf((r0 + a * dr - o) * inv_d), 0, n - 1);
     float ai = alpha(i), ai1 = alpha(i + 1);
-    if (step > 0) {  // interval of cell i: [alpha(i), alpha(i+1)]
+    if (dr > 0.f) {  // interval of cell i: [alpha(i), alpha(i+1)]
       while (i > 0 && ai > a) { i--; ai1 = ai; ai = alpha(i); }
       while (i < n - 1 && ai1 <= a) { i++; ai = ai1; ai1 = alpha(i + 1); }
       lo = ai;
@@ -277,26 +281,42 @@ struct WalkAxis {
       kn = i;
     }
   }
+  __device__ __forceinline__ int cell() const { return kn - (dr > 0.f ? 1 : 0); }
 };
 
 // Walk one ray through the grid and add its chord lengths to the window.
 // Voxel interval = [max lo, min hi] over the axes; length = (aMax - aMin) *
-// |r1 - r0| (getSystemMatrixFromWorkqueue.cu:24-69).  The walk starts in the
-// cell containing the parameter fraction `frac` of the ray's grid range,
-// runs to the exit, re-enters at the entry and stops at the starting cell
-// (the first cell entered at or after its entry parameter), all in one loop:
-// the lanes of a warp walk rays of one channel, each from a different
-// starting point (fewer atomic collisions), and stay converged.  Each step
-// is branch-free: the axis whose plane comes first is selected and advanced
-// with one division.
+// |r1 - r0| (getSystemMatrixFromWorkqueue.cu:24-69).  Each step is
+// branch-free: the axis whose plane comes first is advanced with one
+// division.
+//
+// Every other ray is walked from its exit to its entry (`backward`): with
+// the negated parameters -a the quotients only change sign and the lengths
+// are the same, and the lanes of a warp, which walk rays of one channel, meet
+// in fewer cells at a time (their adds collide less).  Starting each lane at
+// another fraction of its ray, with a wrap at the exit, spread the lanes
+// further, but every lane's wrap was a divergent detour of the whole warp
+// and every ray entered the grid twice.
 //
 // With npieces > 1 the lane walks only piece `piece` of the ray: the cells
-// entered in [a_lo, a_hi), the piece's share of the grid range (no wrap).
-// The pieces of a ray compute their common bounds with the same expression,
-// so every cell belongs to exactly one piece.  Whole rays and pieces share
-// one loop (one copy of its code).
+// entered in [a_lo, a_hi), the piece's share of the grid range.  The pieces
+// of a ray compute their common bounds with the same expression, so every
+// cell belongs to exactly one piece.  Whole rays and pieces share one loop
+// (one copy of its code).
+//
+// Hits outside the window (a ray that is longer than its segment inside the
+// grid, an endpoint inside the grid) must be reported.  A ray that crosses
+// the grid between its two endpoints stays inside the crystals' convex hull,
+// which the window of a channel whose crystals lie on both sides of the grid
+// covers with kWinPad of a voxel to spare, so its cells need no test; every
+// other ray (`chk`, also when the grid is too fine for that margin,
+// Geo::check_window) tests each cell and stops at the first one outside.  An untested ray's addresses stay in the pool whatever the window
+// is: its columns lie between those of its entry and its exit, which are
+// checked against the table's box here (a column just off the box falls on
+// the border or the guard entries), and every table entry puts all z cells
+// into the pool.
 __device__ __forceinline__ void walk_ray(const Geo& G, const float* ray, const Window& w, int* needs_exact,
-                         float frac, int piece, int npieces) {
+                         bool backward, int piece, int npieces) {
   const epet_grid& g = G.p.grid;
   if (ray[0] == ray[3] && ray[1] == ray[4] && ray[2] == ray[5]) return;
   if (ray[0] == ray[3] || ray[1] == ray[4] || ray[2] == ray[5]) {
@@ -309,15 +329,17 @@ __device__ __forceinline__ void walk_ray(const Geo& G, const float* ray, const W
   }
   WalkAxis X, Y, Z;
   X.P = w.planes; Y.P = w.planes + w.poff1; Z.P = w.planes + w.poff2;
-  X.o = g.o[0]; X.d = g.d[0]; X.r0 = ray[0]; X.dr = fsub(ray[3], ray[0]); X.n = g.n[0];
-  Y.o = g.o[1]; Y.d = g.d[1]; Y.r0 = ray[1]; Y.dr = fsub(ray[4], ray[1]); Y.n = g.n[1];
-  Z.o = g.o[2]; Z.d = g.d[2]; Z.r0 = ray[2]; Z.dr = fsub(ray[5], ray[2]); Z.n = g.n[2];
+  X.o = g.o[0]; X.inv_d = G.inv_pitch[0]; X.r0 = ray[0]; X.n = g.n[0];
+  Y.o = g.o[1]; Y.inv_d = G.inv_pitch[1]; Y.r0 = ray[1]; Y.n = g.n[1];
+  Z.o = g.o[2]; Z.inv_d = G.inv_pitch[2]; Z.r0 = ray[2]; Z.n = g.n[2];
+  // backward: -(r1 - r0), so that the parameters are the negated ones
+  const float dir = backward ? -1.f : 1.f;
+  X.dr = fmul(dir, fsub(ray[3], ray[0]));
+  Y.dr = fmul(dir, fsub(ray[4], ray[1]));
+  Z.dr = fmul(dir, fsub(ray[5], ray[2]));
   X.inv = __frcp_rn(X.dr);
   Y.inv = __frcp_rn(Y.dr);
   Z.inv = __frcp_rn(Z.dr);
-  X.step = X.dr > 0.f ? 1 : -1;
-  Y.step = Y.dr > 0.f ? 1 : -1;
-  Z.step = Z.dr > 0.f ? 1 : -1;
   const float L = norm3(X.dr, Y.dr, Z.dr);
   // grid parameter range
   float a_in, a_out;
@@ -329,110 +351,149 @@ __device__ __forceinline__ void walk_ray(const Geo& G, const float* ray, const W
     a_out = fminf(fminf(fmaxf(x0, x1), fmaxf(y0, y1)), fmaxf(z0, z1));
   }
   if (!(a_in < a_out)) return;
-  const float span = fsub(a_out, a_in);
+  const float a_first = backward ? -a_out : a_in, a_last = backward ? -a_in : a_out;
+  bool chk = w.test_all || !(a_first >= 0.f && a_last <= 1.f);
+  {
+    // the (x, y) of the entry and the exit, in cells from the table's corner
+    const float bx = (X.r0 - X.o) * X.inv_d - (float)w.bx0, ux = X.dr * X.inv_d;
+    const float by = (Y.r0 - Y.o) * Y.inv_d - (float)w.by0, uy = Y.dr * Y.inv_d;
+    const float xi = bx + a_in * ux, xo = bx + a_out * ux;
+    const float yi = by + a_in * uy, yo = by + a_out * uy;
+    if (!(fminf(xi, xo) > -0.01f && fmaxf(xi, xo) < (float)w.wbx + 0.01f &&
+          fminf(yi, yo) > -0.01f && fmaxf(yi, yo) < (float)w.wby + 0.01f))
+      chk = true;
+  }
   // a_lim: the walk stops after the cell whose exit parameter reaches it
-  // (the grid's exit, the piece's end, or after the wrap the start cell's
-  // entry)
-  float a_s, a_lo = -INFINITY, a_lim = a_out;
-  // entry state of the second part: plane indices, their parameters, and
-  // the entry parameter of the grid's first cell
-  int ekpx = 0, ekpy = 0, ekpz = 0;
-  float ehx = 0.f, ehy = 0.f, ehz = 0.f, eamin = 0.f;
-  bool second;
+  // (the grid's exit or the piece's end)
+  float a_s = a_in, a_lo = -INFINITY, a_lim = a_out;
   if (npieces > 1) {
+    const float span = fsub(a_out, a_in);
     if (piece > 0) a_lo = fadd(a_in, fmul(span, (float)piece / (float)npieces));
     if (piece + 1 < npieces) a_lim = fadd(a_in, fmul(span, (float)(piece + 1) / (float)npieces));
-    a_s = piece > 0 ? a_lo : a_in;
+    if (piece > 0) a_s = a_lo;
     if (!(a_s < a_out) || !(a_lo < a_lim)) return;  // an empty piece (rounding)
-    second = true;  // no wrap
-  } else {
-    a_s = a_in + span * frac;
-    if (!(a_s >= a_in && a_s < a_out)) a_s = a_in;
-    // entry state of the second part (the cells before the starting cell),
-    // computed up front by all lanes together: the switch in the loop is
-    // then a register copy, not a divergent search
-    X.enter(a_in);
-    Y.enter(a_in);
-    Z.enter(a_in);
-    ekpx = X.kn; ekpy = w.poff1 + Y.kn; ekpz = w.poff2 + Z.kn;
-    ehx = X.hi; ehy = Y.hi; ehz = Z.hi;
-    eamin = fmaxf(fmaxf(X.lo, Y.lo), Z.lo);
-    second = !(a_s > a_in);  // nothing before the starting cell
   }
   X.enter(a_s);
   Y.enter(a_s);
   Z.enter(a_s);
-  const float a_start = fmaxf(fmaxf(X.lo, Y.lo), Z.lo);  // entry of the starting cell
-  // Per axis the walk keeps kp, the plane table index of the plane at which
-  // it leaves the current cell along that axis (the axis' table offset plus
-  // the plane index kn), and h, that plane's parameter; the cell index is
-  // kn - 1 (ascending) or kn (descending).  The entry parameter of the
-  // current cell is always the latest crossing (the largest of the axes'
-  // lo), so it is carried as one value; the cell whose exit parameter reaches
-  // a_out is the last before the grid's exit, so no axis steps past its last
-  // plane.
-  int kpx = X.kn, kpy = w.poff1 + Y.kn, kpz = w.poff2 + Z.kn;
+  // Per axis the walk keeps k, the address of the plane at which it leaves
+  // the current cell along that axis, and h, that plane's parameter.  The
+  // entry parameter of the current cell is always the latest crossing (the
+  // largest of the axes' lo), so it is carried as one value; the cell whose
+  // exit parameter reaches the grid's exit is the last one, so no axis steps
+  // past its last plane.
   float hx = X.hi, hy = Y.hi, hz = Z.hi;
-  float amin = a_start;
+  float amin = fmaxf(fmaxf(X.lo, Y.lo), Z.lo);
   // a piece's first cell entered before a_lo is the previous piece's: walked
   // as a zero-length cell (every later cell is entered at or after a_lo)
   if (amin < a_lo) amin = fminf(fminf(hx, hy), hz);
-  const int ox = (X.step > 0 ? 1 : 0) + w.bx0;  // column = (kp_x - ox, kp_y - oy)
-  const int oy = w.poff1 + (Y.step > 0 ? 1 : 0) + w.by0;
-  const int oz = w.poff2 + (Z.step > 0 ? 1 : 0);  // z cell = kp_z - oz
-  Col col = load_col(w, kpx - ox, kpy - oy);
+  const bool upx = X.dr > 0.f, upy = Y.dr > 0.f, upz = Z.dr > 0.f;
+  uint32_t kx = w.planes_s + 4u * (uint32_t)X.kn, ky = w.planes_s + 4u * (uint32_t)(w.poff1 + Y.kn),
+           kz = w.planes_s + 4u * (uint32_t)(w.poff2 + Z.kn);
+  const int sx = upx ? 4 : -4, sy = upy ? 4 : -4, sz = upz ? 4 : -4;
+  // (a tested ray looks its columns up itself: its table address stays put)
+  const int cx = chk ? 0 : (upx ? 4 * w.wbyp : -4 * w.wbyp), cy = chk ? 0 : sy;
+  uint32_t col = w.cbase_s;
+  if (!chk) col += 4u * (uint32_t)((X.cell() - w.bx0) * w.wbyp + (Y.cell() - w.by0));
+  // lo word of the cell: column base + kz + zl; hi word: + zl + hioff
+  const uint32_t zl = 0u - (w.planes_s + 4u * (uint32_t)w.poff2) - (upz ? 4u : 0u);
+  const uint32_t zh = zl + w.hioff;
+  const float nx_ = -X.dr, ny_ = -Y.dr, nz_ = -Z.dr;
+  // A tested ray's cell: false outside the window, else its column's base.
+  auto lookup = [&](uint32_t* base) -> bool {
+    const int ix = (int)((kx - w.planes_s) >> 2) - (upx ? 1 : 0) - w.bx0;
+    const int iy = (int)((ky - w.planes_s) >> 2) - w.poff1 - (upy ? 1 : 0) - w.by0;
+    if ((unsigned)ix >= (unsigned)w.wbx || (unsigned)iy >= (unsigned)w.wby) return false;
+    const int k = ix * w.wbyp + iy;
+    const uint32_t e = w.zrun[k];
+    *base = w.cbase[k];
+    return ((kz + zl) >> 2) - (e & 0xffffu) < (e >> 16);
+  };
+  uint32_t cb;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(cb) : "r"(col) : "memory");
   // chord units = RN((amax - amin) * L) * 2^s = RN((amax - amin) * (L * 2^s)):
   // scaling by a power of two is exact
   const float Ls = fmul(L, G.fx_scale);
   const uint32_t lo_mask = (1u << w.split) - 1u;
   const int budget = g.n[0] + g.n[1] + g.n[2] + 4;
-  for (int steps = 0; steps < budget; steps++) {
-    // the axis whose plane comes first (ties: x, then y, then z)
-    const float amax = fminf(fminf(hx, hy), hz);
-    const bool mx = hx == amax;
-    const bool my = !mx && hy == amax;
-    const bool mz = !mx && !my;
-    {
-      // Branch-free add: a step with nothing to add (a zero-length cell, the
-      // previous piece's cell) adds to the trash cell, a hit outside the
-      // window adds one to the outside cell's count.
-      const bool add = amin < amax;
-      const unsigned dz = (unsigned)(kpz - oz - col.zlo);
-      const bool inwin = dz < (unsigned)col.zn;
-      const int c = add ? (inwin ? col.off + (int)dz : w.trash_out) : w.trash;
-      // units = RN_int(max(len * scale, 1)) (< 2^64 by the choice of scale:
-      // a positive chord counts at least one unit), split as hi * 2^split + lo
-      const unsigned long long u = __float2ull_rn(fmaxf(fmul(fsub(amax, amin), Ls), 1.f));
-      const uint32_t h = (uint32_t)(u >> w.split);
-      const uint32_t l = inwin ? (uint32_t)u & lo_mask : 1u;
-      atomicAdd(&w.cell[c].x, l);
-      atomicAdd(&w.cell[c].y, h);
-    }
-    if (amax >= a_lim) {
-      // last cell: the part before the starting cell, if any
-      if (second || !(eamin < a_start)) break;
-      second = true;
-      a_lim = a_start;
-      kpx = ekpx; kpy = ekpy; kpz = ekpz;
-      hx = ehx; hy = ehy; hz = ehz;
-      amin = eamin;
-      col = load_col(w, kpx - ox, kpy - oy);
-      continue;
-    }
-    // advance the axis whose plane comes first: its next plane's parameter
-    // is the reference's quotient over the tabulated plane position
-    const int st = mx ? X.step : (my ? Y.step : Z.step);
-    const int kp = (mx ? kpx : (my ? kpy : kpz)) + st;
-    const float P = w.planes[kp];  // in the table or a guard entry
-    const float r0 = mx ? X.r0 : (my ? Y.r0 : Z.r0), dr = mx ? X.dr : (my ? Y.dr : Z.dr);
-    const float inv = mx ? X.inv : (my ? Y.inv : Z.inv);
-    const float h = div_cr(fsub(P, r0), dr, inv);
-    hx = mx ? h : hx; kpx = mx ? kp : kpx;
-    hy = my ? h : hy; kpy = my ? kp : kpy;
-    hz = mz ? h : hz; kpz = mz ? kp : kpz;
-    amin = amax;
-    col = load_col(w, kpx - ox, kpy - oy);
+  // every step of a tested ray takes the branch that only the last one of
+  // the others takes
+  const float a_stop = chk ? -INFINITY : a_lim;
+  // One step.  Instructions of the axis whose plane comes first are
+  // predicated instead of selected: the selects (six of them on the three
+  // axes' ray constants, six on the results) ran on the half-rate ALU pipe,
+  // which was the kernel's busiest (69 %); the predicated multiplies and
+  // adds run on the FMA pipe.  The column is looked up only when x or y is
+  // crossed.
+#define EPET_WALK_ADD                                                                           \
+  {                                                                                             \
+    /* units = RN_int(max(len * scale, 1)) (< 2^64 by the choice of scale: a positive chord    \
+       counts at least one unit), split as hi * 2^split + lo; a zero-length cell adds nothing */ \
+    const unsigned long long u = __float2ull_rn(fmaxf(fmul(fsub(amax, amin), Ls), 1.f));        \
+    const uint32_t h = (uint32_t)(u >> w.split), l = (uint32_t)u & lo_mask;                     \
+    asm volatile(                                                                               \
+        "{\n\t.reg .pred p;\n\t"                                                                \
+        "setp.lt.f32 p, %0, %1;\n\t"                                                            \
+        "@p red.shared.add.u32 [%2], %3;\n\t"                                                   \
+        "@p red.shared.add.u32 [%4], %5;\n\t}" ::"f"(amin),                                     \
+        "f"(amax), "r"(cb + kz + zl), "r"(l), "r"(cb + kz + zh), "r"(h)                         \
+        : "memory");                                                                            \
   }
+#define EPET_WALK_STEP                                                                          \
+  {                                                                                             \
+    const float amax = fminf(fminf(hx, hy), hz);                                                \
+    if (amax >= a_stop) {                                                                       \
+      if (chk && !lookup(&cb) && amin < amax) {                                                 \
+        atomicAdd(&w.lo[w.trash_out], 1u);                                                      \
+        break;                                                                                  \
+      }                                                                                         \
+      if (amax >= a_lim) {                                                                      \
+        EPET_WALK_ADD                                                                           \
+        break;                                                                                  \
+      }                                                                                         \
+    }                                                                                           \
+    EPET_WALK_ADD                                                                               \
+    /* ties: x, then y, then z */                                                               \
+    asm volatile(                                                                               \
+        "{\n\t.reg .pred px, py, pc;\n\t.reg .f32 P, t, q, r;\n\t"                              \
+        "setp.eq.f32 px, %0, %8;\n\t"                                                           \
+        "setp.eq.and.f32 py, %1, %8, !px;\n\t"                                                  \
+        "or.pred pc, px, py;\n\t"                                                               \
+        "@px add.s32 %3, %3, %9;\n\t"                                                           \
+        "@py add.s32 %4, %4, %10;\n\t"                                                          \
+        "@!pc add.s32 %5, %5, %11;\n\t"                                                         \
+        "@px ld.shared.f32 P, [%3];\n\t"                                                        \
+        "@py ld.shared.f32 P, [%4];\n\t"                                                        \
+        "@!pc ld.shared.f32 P, [%5];\n\t"                                                       \
+        "@px add.s32 %6, %6, %21;\n\t"                                                          \
+        "@py add.s32 %6, %6, %22;\n\t"                                                          \
+        "@pc ld.shared.u32 %7, [%6];\n\t"                                                       \
+        "@px sub.rn.f32 t, P, %12;\n\t"                                                         \
+        "@py sub.rn.f32 t, P, %13;\n\t"                                                         \
+        "@!pc sub.rn.f32 t, P, %14;\n\t"                                                        \
+        "@px mul.rn.f32 q, t, %15;\n\t"                                                         \
+        "@py mul.rn.f32 q, t, %16;\n\t"                                                         \
+        "@!pc mul.rn.f32 q, t, %17;\n\t"                                                        \
+        "@px fma.rn.f32 r, q, %18, t;\n\t"                                                      \
+        "@py fma.rn.f32 r, q, %19, t;\n\t"                                                      \
+        "@!pc fma.rn.f32 r, q, %20, t;\n\t"                                                     \
+        "@px fma.rn.f32 %0, r, %15, q;\n\t"                                                     \
+        "@py fma.rn.f32 %1, r, %16, q;\n\t"                                                     \
+        "@!pc fma.rn.f32 %2, r, %17, q;\n\t}"                                                   \
+        : "+f"(hx), "+f"(hy), "+f"(hz), "+r"(kx), "+r"(ky), "+r"(kz), "+r"(col), "+r"(cb)       \
+        : "f"(amax), "r"(sx), "r"(sy), "r"(sz), "f"(X.r0), "f"(Y.r0), "f"(Z.r0), "f"(X.inv),    \
+          "f"(Y.inv), "f"(Z.inv), "f"(nx_), "f"(ny_), "f"(nz_), "r"(cx), "r"(cy)                \
+        : "memory");                                                                            \
+    amin = amax;                                                                                \
+  }
+  // two steps per count of the loop's bound
+#pragma unroll 1
+  for (int steps = 0; steps < budget; steps += 2) {
+    EPET_WALK_STEP
+    EPET_WALK_STEP
+  }
+#undef EPET_WALK_STEP
+#undef EPET_WALK_ADD
 }
 
 // Per-channel geometry for the walk, one thread per channel: the 16 crystal
@@ -474,15 +535,20 @@ static epet_status launch_channel_geom(const Geo& G, const int32_t* rows, int64_
   return EPET_OK;
 }
 
+// Bound by instruction issue (80 % of the slots, 26 of 32 lanes active), not
+// by memory.  Forward projection of every 13th channel of the full workload
+// (395,460 rows, 100 rays): 14.8 -> 10.9 ms with the predicated step (a
+// select-based one: 52 instructions a step, ALU pipe 69 %), no wrap in a ray's
+// walk, lo and hi sums apart, the hull from 16 lines, the z runs of a column
+// from per-x and per-y slab runs, one barrier per scan.  Registers are held
+// to 64 for 8 CTAs per SM (9 with 56 registers: 11.4 ms, 10 with 48: 12.3).
 template <int kMode>
-__global__ void __launch_bounds__(kWalkThreads)
+__global__ void __launch_bounds__(kWalkThreads, 8)
 k_walk(WalkArgs args) {
   extern __shared__ __align__(16) unsigned char smem[];
   const Geo& G = args.G;
   const epet_grid& g = G.p.grid;
-  const int nx = g.n[0];
-  const int nplanes = g.n[0] + g.n[1] + g.n[2] + 3;
-  const WalkLayout lay = walk_layout(max(g.n[0], g.n[2]), nplanes, g.n[2], args.cap_cells);
+  const WalkLayout lay = walk_layout(g, args.cap_cells);
   Slab* slabs = reinterpret_cast<Slab*>(smem + lay.slabs);
   Window win;
   win.split = G.fx_split;
@@ -490,11 +556,12 @@ k_walk(WalkArgs args) {
   const float(*c0)[3] = reinterpret_cast<const float(*)[3]>(s_geom);
   const float(*c1)[3] = reinterpret_cast<const float(*)[3]>(s_geom + 24);
   const ChannelLine& line = *reinterpret_cast<const ChannelLine*>(s_geom + 48);
-  __shared__ int warp_tot[kWalkThreads / 32];
-  __shared__ int s_total, s_exact, s_box[4];
+  __shared__ int tot_cells[kWalkThreads / 32], tot_kept[kWalkThreads / 32];
+  __shared__ int s_exact, s_box[4], s_nospan;
   __shared__ double red_d[kWalkThreads / 32];
   __shared__ float red_f[kWalkThreads / 32];
   __shared__ float s_e;
+  __shared__ int s_col[kWalkThreads];
 
   if ((int64_t)blockIdx.x >= args.m) return;
   const int64_t row = args.sel ? (int64_t)args.sel[blockIdx.x] : (int64_t)blockIdx.x;
@@ -506,101 +573,112 @@ k_walk(WalkArgs args) {
         reinterpret_cast<const float4*>(args.geom + row * kGeomFloats)[threadIdx.x];
   if (threadIdx.x == 0) {
     s_exact = 0;
+    s_nospan = 0;
     s_box[0] = INT_MAX; s_box[1] = INT_MIN; s_box[2] = INT_MAX; s_box[3] = INT_MIN;
   }
   __syncthreads();
   // slabs along the axis the line follows more closely (x or z)
   const int sa = fabsf(line.ab[2]) > fabsf(line.ab[0]) ? 2 : 0;
-  const int pa = sa == 0 ? 1 : 0, qa = sa == 0 ? 2 : 1;
   const int ns = g.n[sa];  // slabs
 
-  // ---- hull cross-section at every slab plane: the 64 crystal-corner pair
-  // lines' parameters in shared memory (a thread per line), then two threads
-  // per plane, each taking the extremes over 32 of the lines, combined with
-  // one shuffle
+  // ---- hull cross-section at every slab plane.  A crystal's corners differ
+  // in y independently of x and z (the heads rotate about y), so the extremes
+  // over the 64 corner-pair lines come from the 16 lines that join the
+  // crystals' vertical edges: along the horizontal axis h from their points,
+  // along y from the smallest and the largest parameter t at the plane (the
+  // crystals' y faces are joined linearly in t).  A thread per line, then two
+  // threads per plane with 8 lines each, combined with shuffles (a quarter of
+  // the work of all 64 lines).
+  const int h = sa == 0 ? 2 : 0;  // the other horizontal axis
   int4* pext = reinterpret_cast<int4*>(smem + lay.pext);
+  bool spans;
   {
-    constexpr int kLines = kHullLines;
-    // ax, ay, az, inv (0: parallel to the planes), dy, dz of each line
-    float(*s_line)[kLines] = reinterpret_cast<float(*)[kLines]>(smem + lay.lines);
-    __shared__ int s_nospan;
-    if (threadIdx.x == 0) s_nospan = 0;
-    __syncthreads();
-    if (threadIdx.x < kLines) {
-      const int a = threadIdx.x >> 3, b = threadIdx.x & 7;
-      const float ax = c0[a][sa], ay = c0[a][pa], az = c0[a][qa];
-      const float dx = c1[b][sa] - ax;
-      const bool ok = dx != 0.f;
-      const float inv = ok ? __frcp_rn(dx) : 0.f;
-      s_line[0][threadIdx.x] = ax;
-      s_line[1][threadIdx.x] = ay;
-      s_line[2][threadIdx.x] = az;
-      s_line[3][threadIdx.x] = inv;
-      s_line[4][threadIdx.x] = c1[b][pa] - ay;
-      s_line[5][threadIdx.x] = c1[b][qa] - az;
+    // {edge 0 along sa, 1 / (edge 1 - edge 0) (0: parallel to the planes),
+    //  edge 0 along h, edge 1 - edge 0}
+    float4* s_line = reinterpret_cast<float4*>(smem + lay.lines);
+    if (threadIdx.x < kHullLines) {
+      // corner k = x + 2 y + 4 z: the edges are corners 0, 1, 4, 5
+      const int a = (threadIdx.x & 1) | ((threadIdx.x & 2) << 1);
+      const int b = ((threadIdx.x >> 2) & 1) | ((threadIdx.x >> 1) & 4);
+      const float as = c0[a][sa], ah = c0[a][h];
+      const float ds = c1[b][sa] - as;
+      const bool ok = ds != 0.f;
+      const float inv = ok ? __frcp_rn(ds) : 0.f;
+      s_line[threadIdx.x] = make_float4(as, inv, ah, c1[b][h] - ah);
       // t is monotone in the plane position: when every line meets the
       // first and the last plane within its segment it meets all of them
       // (the usual case, the grid lying between the heads), and the
       // per-plane tests drop
       const float X0 = voxel_plane(g, sa, 0), X1 = voxel_plane(g, sa, ns);
-      const float t0 = (X0 - ax) * inv, t1 = (X1 - ax) * inv;
+      const float t0 = (X0 - as) * inv, t1 = (X1 - as) * inv;
       if (!(ok && t0 >= 0.f && t0 <= 1.f && t1 >= 0.f && t1 <= 1.f)) s_nospan = 1;
     }
     __syncthreads();
-    const bool all_span = s_nospan == 0;
-    const int half = threadIdx.x & 1, l0 = half * (kLines / 2);
+    spans = s_nospan == 0;
+    const float ya0 = c0[0][1], yb0 = c0[2][1], dya = c1[0][1] - ya0, dyb = c1[2][1] - yb0;
+    const int half = threadIdx.x & 1, l0 = half * (kHullLines / 2);
     for (int k0 = 0; k0 <= ns; k0 += kWalkThreads / 2) {
       const int k = k0 + (threadIdx.x >> 1);
       const float X = voxel_plane(g, sa, min(k, ns));
-      float ylo = INFINITY, yhi = -INFINITY, zlo = INFINITY, zhi = -INFINITY;
-      bool any = false;
-      if (all_span) {
-#pragma unroll 8
-        for (int l = l0; l < l0 + kLines / 2; l++) {
-          const float t = (X - s_line[0][l]) * s_line[3][l];
-          const float y = s_line[1][l] + t * s_line[4][l], z = s_line[2][l] + t * s_line[5][l];
-          ylo = fminf(ylo, y); yhi = fmaxf(yhi, y);
-          zlo = fminf(zlo, z); zhi = fmaxf(zhi, z);
+      float tlo = INFINITY, thi = -INFINITY, hlo = INFINITY, hhi = -INFINITY;
+      if (spans) {
+#pragma unroll
+        for (int l = 0; l < kHullLines / 2; l++) {
+          const float4 q = s_line[l0 + l];
+          const float t = (X - q.x) * q.y, v = q.z + t * q.w;
+          tlo = fminf(tlo, t); thi = fmaxf(thi, t);
+          hlo = fminf(hlo, v); hhi = fmaxf(hhi, v);
         }
-        any = true;
       } else {
-        for (int l = l0; l < l0 + kLines / 2; l++) {
-          const float inv = s_line[3][l];
-          const float t = (X - s_line[0][l]) * inv;
-          if (inv != 0.f && t >= 0.f && t <= 1.f) {
-            const float y = s_line[1][l] + t * s_line[4][l], z = s_line[2][l] + t * s_line[5][l];
-            ylo = fminf(ylo, y); yhi = fmaxf(yhi, y);
-            zlo = fminf(zlo, z); zhi = fmaxf(zhi, z);
-            any = true;
+        for (int l = 0; l < kHullLines / 2; l++) {
+          const float4 q = s_line[l0 + l];
+          const float t = (X - q.x) * q.y;
+          if (q.y != 0.f && t >= 0.f && t <= 1.f) {
+            const float v = q.z + t * q.w;
+            tlo = fminf(tlo, t); thi = fmaxf(thi, t);
+            hlo = fminf(hlo, v); hhi = fmaxf(hhi, v);
           }
         }
       }
-      ylo = fminf(ylo, __shfl_xor_sync(0xffffffffu, ylo, 1));
-      yhi = fmaxf(yhi, __shfl_xor_sync(0xffffffffu, yhi, 1));
-      zlo = fminf(zlo, __shfl_xor_sync(0xffffffffu, zlo, 1));
-      zhi = fmaxf(zhi, __shfl_xor_sync(0xffffffffu, zhi, 1));
-      // (every lane takes part in the shuffle: no short-circuit around it)
-      const int any_pair = __shfl_xor_sync(0xffffffffu, (int)any, 1);
-      any = any || any_pair != 0;
-      if (half == 0 && k <= ns)
-        pext[k] = any ? make_int4(fkey(ylo), fkey(yhi), fkey(zlo), fkey(zhi))
-                      : make_int4(INT_MAX, INT_MIN, INT_MAX, INT_MIN);
+      // (every lane takes part in the shuffles)
+      tlo = fminf(tlo, __shfl_xor_sync(0xffffffffu, tlo, 1));
+      thi = fmaxf(thi, __shfl_xor_sync(0xffffffffu, thi, 1));
+      hlo = fminf(hlo, __shfl_xor_sync(0xffffffffu, hlo, 1));
+      hhi = fmaxf(hhi, __shfl_xor_sync(0xffffffffu, hhi, 1));
+      if (half == 0 && k <= ns) {
+        if (tlo <= thi) {
+          const float u0 = ya0 + tlo * dya, u1 = ya0 + thi * dya;
+          const float w0 = yb0 + tlo * dyb, w1 = yb0 + thi * dyb;
+          const int ylo = fkey(fminf(fminf(u0, u1), fminf(w0, w1)));
+          const int yhi = fkey(fmaxf(fmaxf(u0, u1), fmaxf(w0, w1)));
+          pext[k] = sa == 0 ? make_int4(ylo, yhi, fkey(hlo), fkey(hhi))
+                            : make_int4(fkey(hlo), fkey(hhi), ylo, yhi);
+        } else {
+          pext[k] = make_int4(INT_MAX, INT_MIN, INT_MAX, INT_MIN);
+        }
+      }
     }
+  }
+  // z slabs: the first and the last slab whose rectangle holds each x and
+  // each y (x at runs[0 ..], y at runs[2 nx ..]: firsts, then lasts)
+  int* xr0 = reinterpret_cast<int*>(smem + lay.runs);
+  int* xr1 = xr0 + g.n[0];
+  int* yr0 = xr1 + g.n[0];
+  int* yr1 = yr0 + g.n[1];
+  if (sa == 2) {
+    for (int i = threadIdx.x; i < g.n[0]; i += kWalkThreads) { xr0[i] = INT_MAX; xr1[i] = INT_MIN; }
+    for (int i = threadIdx.x; i < g.n[1]; i += kWalkThreads) { yr0[i] = INT_MAX; yr1[i] = INT_MIN; }
   }
   __syncthreads();
 
-  // ---- per-slab windows (rectangles over the other two axes), their
-  // flattened offsets, and the (x, y) bounding box of all of them
-  int my_cells = 0;
-  const int per = (ns + kWalkThreads - 1) / kWalkThreads;
-  const int sbeg = threadIdx.x * per, send = min(ns, sbeg + per);
+  // ---- per-slab windows (rectangles over the other two axes) and the (x, y)
+  // bounding box of all of them
   {
     int xlo = INT_MAX, xhi = INT_MIN, ylo = INT_MAX, yhi = INT_MIN;
-    for (int i = sbeg; i < send; i++) {
+    for (int i = threadIdx.x; i < ns; i += kWalkThreads) {
       Slab sl;
-      slab_window(G, c0, c1, pext, sa, i, &sl);
+      slab_window(G, c0, c1, pext, spans, sa, i, &sl);
       slabs[i] = sl;
-      my_cells += sl.wp * sl.wq;
       if (sl.wp > 0 && sl.wq > 0) {
         if (sa == 0) {  // slab = x, rectangle over (y, z)
           xlo = min(xlo, i); xhi = max(xhi, i);
@@ -608,6 +686,14 @@ k_walk(WalkArgs args) {
         } else {        // slab = z, rectangle over (x, y)
           xlo = min(xlo, sl.p0); xhi = max(xhi, sl.p0 + sl.wp - 1);
           ylo = min(ylo, sl.q0); yhi = max(yhi, sl.q0 + sl.wq - 1);
+          for (int j = sl.p0; j < sl.p0 + sl.wp; j++) {
+            atomicMin(&xr0[j], i);
+            atomicMax(&xr1[j], i);
+          }
+          for (int j = sl.q0; j < sl.q0 + sl.wq; j++) {
+            atomicMin(&yr0[j], i);
+            atomicMax(&yr1[j], i);
+          }
         }
       }
     }
@@ -616,117 +702,79 @@ k_walk(WalkArgs args) {
       atomicMin(&s_box[2], ylo); atomicMax(&s_box[3], yhi);
     }
   }
-  int n_rect = 0;  // cells of all slab rectangles (z slabs only: offsets for the table)
-  if (sa == 2) {   // uniform across the block
-    const int excl = block_excl_scan(my_cells, warp_tot, &s_total);
-    int o = excl;
-    for (int i = sbeg; i < send; i++) {
-      slabs[i].off = o;
-      o += slabs[i].wp * slabs[i].wq;
-    }
-  }
   __syncthreads();
-  if (sa == 2) n_rect = s_total;
   win.bx0 = s_box[0];
   win.by0 = s_box[2];
   win.wbx = s_box[1] >= s_box[0] ? s_box[1] - s_box[0] + 1 : 0;
   win.wby = s_box[3] >= s_box[2] ? s_box[3] - s_box[2] + 1 : 0;
   win.wbyp = win.wby + 1;
   const int A = (win.wbx + 1) * win.wbyp;  // table entries (with the empty border)
-  // z range of column k = (ix, iy): for x slabs the range of slab ix's
-  // rectangle at iy; for z slabs the first and last slab whose rectangle
-  // holds (ix, iy)
-  auto col_range_scan = [&](int k, int* zlo, int* zhi) {  // z slabs, no storage
-    const int ix = win.bx0 + k / win.wbyp, iy = win.by0 + k % win.wbyp;
-    int lo = INT_MAX, hi = INT_MIN;
-    for (int iz = 0; iz < ns; iz++) {
-      const Slab sl = slabs[iz];
-      if ((unsigned)(ix - sl.p0) < (unsigned)sl.wp && (unsigned)(iy - sl.q0) < (unsigned)sl.wq) {
-        lo = min(lo, iz);
-        hi = iz;
-      }
-    }
-    *zlo = lo;
-    *zhi = hi;
-  };
-  auto col_range_x = [&](int k, int* zlo, int* zhi) {  // x slabs
-    const int cx = k / win.wbyp, cy = k % win.wbyp;
-    const int ix = win.bx0 + cx, iy = win.by0 + cy;
-    const Slab sl = slabs[cx < win.wbx ? ix : win.bx0];  // the border column is empty
-    if (cx < win.wbx && cy < win.wby && (unsigned)(iy - sl.p0) < (unsigned)sl.wp) {
-      *zlo = sl.q0;
-      *zhi = sl.q0 + sl.wq - 1;
-    } else {
-      *zlo = INT_MAX;
-      *zhi = INT_MIN;
-    }
-  };
   const int kper = (A + kWalkThreads - 1) / kWalkThreads;
   const int kbeg = min(A, (int)threadIdx.x * kper), kend = min(A, kbeg + kper);
+  // The z runs of the thread's columns k = (ix, iy), f(k, first, last) in
+  // order (empty: last < first): for x slabs the range of slab ix's rectangle
+  // at iy; for z slabs the slabs whose rectangle holds ix and those whose
+  // rectangle holds iy (of a convex bundle, both without gaps).
+  auto for_cols = [&](auto&& f) {
+    if (kbeg >= kend) return;
+    int cx = kbeg / win.wbyp, cy = kbeg - cx * win.wbyp;
+    for (int k = kbeg; k < kend; k++) {
+      int zlo = 0, zhi = -1;
+      if (cx < win.wbx && cy < win.wby) {  // not the border
+        const int ix = win.bx0 + cx, iy = win.by0 + cy;
+        if (sa == 0) {
+          const int4 sl = reinterpret_cast<const int4*>(slabs)[ix];
+          if ((unsigned)(iy - sl.x) < (unsigned)sl.y) {
+            zlo = sl.z;
+            zhi = sl.z + sl.w - 1;
+          }
+        } else if (spans) {
+          zlo = max(xr0[ix], yr0[iy]);
+          zhi = max(min(xr1[ix], yr1[iy]), -1);
+          if (zhi < zlo) zlo = 0, zhi = -1;
+        } else {
+          // the rectangles of a bundle that ends inside the grid need not
+          // shrink steadily: the first and the last slab that holds (ix, iy)
+          zlo = 0, zhi = -1;
+          for (int iz = ns - 1; iz >= 0; iz--) {
+            const int4 sl = reinterpret_cast<const int4*>(slabs)[iz];
+            if ((unsigned)(ix - sl.x) < (unsigned)sl.y && (unsigned)(iy - sl.z) < (unsigned)sl.w) {
+              if (zhi < 0) zhi = iz;
+              zlo = iz;
+            }
+          }
+        }
+      }
+      f(k, zlo, zhi);
+      if (++cy == win.wbyp) {
+        cy = 0;
+        ++cx;
+      }
+    }
+  };
   if (kMode == kModeWindow) {
     // columns + cells, computed without the table
-    int n = 0;
-    for (int k = kbeg; k < kend; k++) {
-      int zlo, zhi;
-      if (sa == 0) col_range_x(k, &zlo, &zhi);
-      else col_range_scan(k, &zlo, &zhi);
-      if (zhi >= zlo) n += zhi - zlo + 1;
-    }
-    block_excl_scan(n, warp_tot, &s_total);
-    // + the two trash cells
-    if (threadIdx.x == 0) args.win_cells[row] = A + s_total + 2;
+    int n = 0, W;
+    for_cols([&](int, int zlo, int zhi) { n += max(zhi - zlo + 1, 0); });
+    block_excl_scan(n, tot_cells, &W);
+    // + the cell that counts hits outside, and one
+    if (threadIdx.x == 0) args.win_cells[row] = A + W + 2;
     return;
   }
-  int2* cols = reinterpret_cast<int2*>(smem + lay.pool);
-  const bool table_fits = (size_t)A * 8 <= lay.slabs - lay.pool;  // ends before the slabs
-  if (table_fits) {
-    if (sa == 0) {
-      for (int k = kbeg; k < kend; k++) {
-        int zlo, zhi;
-        col_range_x(k, &zlo, &zhi);
-        cols[k] = make_int2(zlo, zhi);
-      }
-    } else {
-      for (int k = threadIdx.x; k < A; k += kWalkThreads) cols[k] = make_int2(INT_MAX, INT_MIN);
-      __syncthreads();
-      // every rectangle cell widens its column's range (shared atomics)
-      const int rpt = (n_rect + kWalkThreads - 1) / kWalkThreads;
-      const int rbeg = min(n_rect, (int)threadIdx.x * rpt), rend = min(n_rect, rbeg + rpt);
-      if (rbeg < rend) {
-        int lo_s = 0, hi_s = ns - 1;  // last slab with off <= rbeg
-        while (lo_s < hi_s) {
-          const int mid = (lo_s + hi_s + 1) >> 1;
-          if (slabs[mid].off <= rbeg) lo_s = mid;
-          else hi_s = mid - 1;
-        }
-        int iz = lo_s;
-        Slab sl = slabs[iz];
-        int jp = (rbeg - sl.off) / max(sl.wq, 1), jq = rbeg - sl.off - jp * sl.wq;
-        for (int r = rbeg; r < rend; r++) {
-          while (r >= sl.off + sl.wp * sl.wq) {
-            sl = slabs[++iz];
-            jp = 0;
-            jq = 0;
-          }
-          const int k = (sl.p0 + jp - win.bx0) * win.wbyp + (sl.q0 + jq - win.by0);
-          atomicMin(&cols[k].x, iz);
-          atomicMax(&cols[k].y, iz);
-          if (++jq == sl.wq) {
-            jq = 0;
-            ++jp;
-          }
-        }
-      }
-    }
-  }
-  __syncthreads();
-  // column lengths -> first cells (exclusive scan), packed ranges
+  // (while it is built, the table holds each column's first and last z)
+  int* cz0 = reinterpret_cast<int*>(smem + lay.pool + lay.gcol);
+  int* cz1 = cz0 + A;
+  const bool table_fits = (size_t)A * 8 + lay.gcol <= lay.slabs - lay.pool;  // ends before the slabs
   int n_mine = 0;
   if (table_fits)
-    for (int k = kbeg; k < kend; k++)
-      if (cols[k].y >= cols[k].x) n_mine += cols[k].y - cols[k].x + 1;
-  const int cexcl = block_excl_scan(n_mine, warp_tot, &s_total);
-  const int W = s_total;  // window cells
+    for_cols([&](int k, int zlo, int zhi) {
+      cz0[k] = zlo;
+      cz1[k] = zhi;
+      n_mine += max(zhi - zlo + 1, 0);
+    });
+  // column lengths -> first cells (exclusive scan)
+  int W;  // window cells
+  const int cexcl = block_excl_scan(n_mine, tot_cells, &W);
   if (!table_fits || A + W + 2 > args.cap_cells) {
     if (threadIdx.x == 0) {
       int k = atomicAdd(args.overflow_count, 1);
@@ -735,26 +783,41 @@ k_walk(WalkArgs args) {
     }
     return;
   }
+  // 8A + 8(W + 2) and the guard bands <= pool
+  win.lo = reinterpret_cast<uint32_t*>(smem + lay.pool + lay.gcol + (size_t)A * 8 + lay.gz);
+  win.hi = win.lo + W + 2;
+  win.hioff = 4u * (uint32_t)(W + 2);
+  const uint32_t lo_s = (uint32_t)__cvta_generic_to_shared(win.lo);
+  // Extraction: thread t takes the cells [t cpt, (t + 1) cpt) (an odd count:
+  // the lanes' concurrent reads fall in distinct shared-memory banks), from
+  // column s_col[t] on.
+  const int cpt = ((W + kWalkThreads - 1) / kWalkThreads) | 1;
+  const float inv_cpt = __fdividef(1.f, (float)cpt);
+  auto first_thread = [&](int o) { return (int)(((float)(o + cpt) - 0.5f) * inv_cpt); };  // ceil(o / cpt)
   {
     int o = cexcl;
     for (int k = kbeg; k < kend; k++) {
-      const int2 r = cols[k];
-      if (r.y >= r.x) {
-        cols[k] = make_int2(o, r.x | ((r.y - r.x + 1) << 16));
-        o += r.y - r.x + 1;
-      } else {
-        cols[k] = make_int2(o, 0);  // empty: zn 0
-      }
+      const int z0 = cz0[k], z1 = cz1[k];
+      const int zn = max(z1 - z0 + 1, 0);
+      cz0[k] = (int)(lo_s + 4u * (uint32_t)(zn > 0 ? o - z0 : o));  // (o - z0 may be < 0)
+      cz1[k] = zn > 0 ? z0 | (zn << 16) : 0;
+      // the threads whose cells start in this column
+      for (int t = first_thread(o); t < kWalkThreads && t * cpt < o + zn; t++) s_col[t] = k;
+      o += zn;
     }
+    uint32_t* guard = reinterpret_cast<uint32_t*>(smem + lay.pool);
+    for (int i = threadIdx.x; i < lay.gcol / 4; i += kWalkThreads) guard[i] = lo_s;
   }
-  win.cols = cols;
-  // 8A + 8(W + 2) <= pool
-  win.cell = reinterpret_cast<uint2*>(smem + lay.pool + (size_t)A * 8);
-  win.trash = W;
-  win.trash_out = W + 1;
+  win.cbase = reinterpret_cast<const uint32_t*>(cz0);
+  win.zrun = reinterpret_cast<const uint32_t*>(cz1);
+  win.cbase_s = (uint32_t)__cvta_generic_to_shared(cz0);
+  win.trash_out = W;
+  win.test_all = G.check_window || !spans;
   // grid planes o + k d of the three axes (the walk's quotients read them)
+  const int nplanes = g.n[0] + g.n[1] + g.n[2] + 3;
   float* planes = reinterpret_cast<float*>(smem + lay.planes) + 1;  // guards at -1 and nplanes
   win.planes = planes;
+  win.planes_s = (uint32_t)__cvta_generic_to_shared(planes);
   win.poff1 = g.n[0] + 1;
   win.poff2 = g.n[0] + g.n[1] + 2;
   if (threadIdx.x == 0) planes[-1] = planes[nplanes] = 0.f;
@@ -770,9 +833,8 @@ k_walk(WalkArgs args) {
     ztab[iz] = make_float2(fmul(line.ab[1], ap2), fmul(line.ab[0], ap2));
   }
   // ---- zero the window, walk the rays
-  for (int i = threadIdx.x; i <= W + 1; i += kWalkThreads) {  // the window and the trash cells
-    win.cell[i] = make_uint2(0u, 0u);
-  }
+  for (int i = threadIdx.x; i < W + 2; i += kWalkThreads)  // lo, then hi words
+    reinterpret_cast<uint2*>(win.lo)[i] = make_uint2(0u, 0u);
   __syncthreads();
   const int R = G.p.nrays;
   const float* rays = args.rays + row * (int64_t)R * 6;
@@ -786,9 +848,7 @@ k_walk(WalkArgs args) {
       const float2* rp = reinterpret_cast<const float2*>(rays + 6 * r);
       const float2 a = rp[0], b = rp[1], c = rp[2];
       ray[0] = a.x; ray[1] = a.y; ray[2] = b.x; ray[3] = b.y; ray[4] = c.x; ray[5] = c.y;
-      // golden-ratio spread of the starting points of whole rays
-      const float frac = (float)r * 0.6180339887f - floorf((float)r * 0.6180339887f);
-      walk_ray(G, ray, win, &s_exact, frac, piece, np);
+      walk_ray(G, ray, win, &s_exact, (r & 1) != 0, piece, np);
     };
     // one call site, so each form of the walk loop is compiled once
     const int t = threadIdx.x;
@@ -814,7 +874,7 @@ k_walk(WalkArgs args) {
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && win.cell[win.trash_out].x != 0u) atomicAdd(args.hit_outside, 1);
+  if (threadIdx.x == 0 && win.lo[win.trash_out] != 0u) atomicAdd(args.hit_outside, 1);
   if (s_exact) {  // uniform across the block
     if (threadIdx.x == 0) {
       int k = atomicAdd(args.exact_count, 1);
@@ -824,26 +884,17 @@ k_walk(WalkArgs args) {
     return;
   }
 
-  // ---- ordered extraction: the cells are stored in voxel-id order, thread
-  // t takes a contiguous range of them (odd length: the lanes' concurrent
-  // reads fall in distinct shared-memory banks)
-  const int cpt = ((W + kWalkThreads - 1) / kWalkThreads) | 1;
+  // ---- ordered extraction: the cells are stored in voxel-id order
   const int cbeg = min(W, (int)threadIdx.x * cpt), cend = min(W, cbeg + cpt);
   // Visits the thread's range in order: fcol(ix, iy) on entering a column,
   // f(cell, ix, iy, iz) per cell.
   auto for_cells = [&](auto&& fcol, auto&& f) {
     if (cbeg >= cend) return;
-    int lo_k = 0, hi_k = A - 1;  // last column with first cell <= cbeg
-    while (lo_k < hi_k) {
-      const int mid = (lo_k + hi_k + 1) >> 1;
-      if (cols[mid].x <= cbeg) lo_k = mid;
-      else hi_k = mid - 1;
-    }
-    int k = lo_k;
-    int2 e = cols[k];
-    int zhi = (e.y & 0xffff) + (e.y >> 16) - 1;
+    int k = s_col[threadIdx.x];
+    uint32_t e = win.zrun[k];
+    int zhi = (int)(e & 0xffffu) + (int)(e >> 16) - 1;
     int cx = k / win.wbyp, cy = k - cx * win.wbyp;
-    int iz = (e.y & 0xffff) + (cbeg - e.x);
+    int iz = cbeg - (int)(win.cbase[k] - lo_s) / 4;
     fcol(win.bx0 + cx, win.by0 + cy);
     for (int cidx = cbeg; cidx < cend; cidx++) {
       if (iz > zhi) {
@@ -853,9 +904,9 @@ k_walk(WalkArgs args) {
             cy = 0;
             ++cx;
           }
-          e = cols[k];
-          iz = e.y & 0xffff;
-          zhi = iz + (e.y >> 16) - 1;
+          e = win.zrun[k];
+          iz = (int)(e & 0xffffu);
+          zhi = iz + (int)(e >> 16) - 1;
         } while (iz > zhi);
         fcol(win.bx0 + cx, win.by0 + cy);
       }
@@ -886,8 +937,8 @@ k_walk(WalkArgs args) {
         colvox = ix * G.nyz + iy * g.n[2];
       },
       [&](int cidx, int ix, int iy, int iz) {
-    const uint2 cu = win.cell[cidx];
-    const unsigned long long u = ((unsigned long long)cu.y << win.split) + (unsigned long long)cu.x;
+    const unsigned long long u =
+        ((unsigned long long)win.hi[cidx] << win.split) + (unsigned long long)win.lo[cidx];
     const float2 zt = ztab[iz];
     const float c0 = fsub(zt.x, K0), c1 = fsub(K1, zt.y);
     // not a candidate: dropped
@@ -897,7 +948,8 @@ k_walk(WalkArgs args) {
     if (kMode == kModeCsr || kMode == kModeMlem) {
       // kept entries compacted at the start of the thread's range: the slot
       // written is this cell's or an earlier one, already read
-      win.cell[cbeg + cnt] = make_uint2(__float_as_uint(v), (uint32_t)(colvox + iz));
+      win.lo[cbeg + cnt] = __float_as_uint(v);
+      win.hi[cbeg + cnt] = (uint32_t)(colvox + iz);
     }
     cnt += keep ? 1 : 0;
     if (kMode != kModeCsr && keep) {
@@ -911,15 +963,15 @@ k_walk(WalkArgs args) {
     }
   });
   if (kMode == kModeCsr) {
-    const int pos = block_excl_scan(cnt, warp_tot, &s_total);
+    int kept;
+    const int pos = block_excl_scan(cnt, tot_kept, &kept);
     const int64_t o = slot * args.stride + pos;
     for (int j = 0; j < cnt; j++) {
-      const uint2 e = win.cell[cbeg + j];
-      args.stage_col[o + j] = (int32_t)e.y;
-      args.stage_val[o + j] = __uint_as_float(e.x);
+      args.stage_col[o + j] = (int32_t)win.hi[cbeg + j];
+      args.stage_val[o + j] = __uint_as_float(win.lo[cbeg + j]);
     }
     if (threadIdx.x == 0) {
-      args.row_len[row] = s_total;
+      args.row_len[row] = kept;
       if (args.sel) args.ovf_idx[row] = (int32_t)slot;
     }
   } else if (kMode == kModeForward || kMode == kModeMlem) {
@@ -943,8 +995,8 @@ k_walk(WalkArgs args) {
       const float ev = s_e;
       if (ev != 0.f)
         for (int j = 0; j < cnt; j++) {
-          const uint2 en = win.cell[cbeg + j];
-          atomicAdd(&args.c64[en.y], (double)fmul(__uint_as_float(en.x), ev));
+          atomicAdd(&args.c64[win.hi[cbeg + j]],
+                    (double)fmul(__uint_as_float(win.lo[cbeg + j]), ev));
         }
     }
   }
@@ -1003,10 +1055,8 @@ __global__ void k_offset_rowptr(int64_t* rp, int64_t n, const int64_t* base) {
 // ------------------------------------------------------------------ host
 
 static size_t walk_smem(const Geo& G, int cap_cells) {
-  static_assert(sizeof(Slab) == 20, "walk_layout assumes 20-byte slabs");
-  return walk_layout(std::max(G.p.grid.n[0], G.p.grid.n[2]),
-                     G.p.grid.n[0] + G.p.grid.n[1] + G.p.grid.n[2] + 3, G.p.grid.n[2], cap_cells)
-      .total;
+  static_assert(sizeof(Slab) == 16, "walk_layout assumes 16-byte slabs");
+  return walk_layout(G.p.grid, cap_cells).total;
 }
 
 // Dynamic shared memory a walk CTA may use on the current device (cached per
