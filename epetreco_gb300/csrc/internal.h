@@ -34,13 +34,15 @@ epet_status launch_workqueue_count(const Geo& G, const int32_t* rows, int64_t m,
 epet_status launch_workqueue_fill(const Geo& G, const int32_t* rows, int64_t m,
                                   const int64_t* row_off, int32_t* cnl, int32_t* vxl,
                                   cudaStream_t st);
-epet_status launch_values(const Geo& G, const float* rays, int64_t m,
+// (ray_row, optional: the rays of row i are those at row ray_row[i])
+epet_status launch_values(const Geo& G, const float* rays, const int32_t* ray_row, int64_t m,
                           const int64_t* row_ptr, const int32_t* col, float* val,
                           bool exact, cudaStream_t st);
 // Rows left to the per-candidate path: in CSR mode (mode 0) each row's kept
 // entries go to compact buffers (row i of the list at off[i], any length),
 // row_len[row] is set and src_idx[row] = -2 - i tells the row gather to read
 // them there; the caller frees the buffers (release()) after that gather.
+// rays: the rays of all of `rows`, generated for the walk.
 struct ExactRows {
   int64_t* off = nullptr;
   int32_t* col = nullptr;
@@ -48,8 +50,8 @@ struct ExactRows {
   void release(cudaStream_t st);
 };
 epet_status exact_rows_apply(const Geo& G, const int32_t* rows, const int32_t* ex_rows,
-                             int64_t n_ex, int mode, int32_t* row_len, int32_t* src_idx,
-                             ExactRows* keep, const float* x, float* y, const float* e,
+                             int64_t n_ex, const float* rays, int mode, int32_t* row_len,
+                             int32_t* src_idx, ExactRows* keep, const float* x, float* y, const float* e,
                              float* c, double* s64, const float* ycnt, double* c64,
                              cudaStream_t st);
 epet_status column_sums(const epet_problem* p, const int32_t* rows_d, int64_t m,

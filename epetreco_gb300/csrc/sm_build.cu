@@ -1069,7 +1069,7 @@ static int max_dyn_smem() {
   int v = slot ? slot->load(std::memory_order_relaxed) : 0;
   if (v == 0) {
     cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    v -= 4096;  // static shared memory of the kernel
+    v -= 1024;  // static shared memory of the kernel
     if (slot) slot->store(v, std::memory_order_relaxed);
   }
   return v;
@@ -1140,16 +1140,18 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
   dev_free(d_cells, st);
   dev_free(d_geom, st);
   if (rc != EPET_OK) return rc;
-  // Sized for the 90th percentile of the sample, not its maximum: every CTA
-  // reserves the capacity in shared memory, so a smaller one keeps more
-  // channels resident per SM; the few larger windows are redone with their
-  // exact size (redo_overflow).
-  std::sort(cells.begin(), cells.end());
-  const int p90 = cells.empty() ? 0 : cells[(cells.size() * 9) / 10];
+  // Sized for the 90th percentile of the sample first: every CTA reserves the
+  // capacity in shared memory, so a smaller one can keep more channels
+  // resident per SM; larger windows are redone with their exact size
+  // (redo_overflow).
+  auto percentile = [&](int q) -> int {
+    if (cells.empty()) return 0;
+    const size_t i = cells.size() * q / 100;
+    std::nth_element(cells.begin(), cells.begin() + i, cells.end());
+    return cells[i];
+  };
+  const int p90 = percentile(90);
   int cap = std::max(256, (int)(p90 * 1.10) + 64);
-  // If a capacity at most 15 % smaller keeps one more CTA resident per SM,
-  // take the largest such: the occupancy gain outweighs the few more rows
-  // redone.
   auto resident = [&](int c) {
     int n = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_walk<kModeCsr>, kWalkThreads,
@@ -1157,15 +1159,27 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
       n = 0;
     return n;
   };
-  const int n0 = resident(cap), lo = std::max(256, (int)(cap * 0.85));
-  if (n0 > 0 && resident(lo) > n0) {
-    int a = lo, b = cap;  // resident(a) > n0 >= resident(b)
+  // Largest capacity in [a, b) that keeps `n` CTAs resident (a does).
+  auto largest = [&](int a, int b, int n) {
     while (b - a > 1) {
       const int mid = (a + b) / 2;
-      if (resident(mid) > n0) a = mid;
+      if (resident(mid) >= n) a = mid;
       else b = mid;
     }
-    cap = a;
+    return a;
+  };
+  const int n0 = resident(cap), lo = std::max(256, (int)(cap * 0.85));
+  if (n0 > 0 && resident(lo) > n0) {
+    // a capacity at most 15 % smaller keeps one more CTA resident per SM:
+    // the occupancy gain outweighs the few more rows redone
+    cap = largest(lo, cap, n0 + 1);
+  } else if (n0 > 0) {
+    // room up to the sample's 98th percentile that costs no resident CTA (at
+    // 52^3 voxels and 100 rays the registers allow 8 CTAs, which leaves each
+    // 28 KB): fewer rows redone (3.8 % of them, 1.0 of 10.9 ms, at the lower
+    // capacity), while a few very wide windows do not size all rows' staging
+    const int top = percentile(98);
+    if (top > cap) cap = resident(top) >= n0 ? top : largest(cap, top, n0);
   }
   *cap_out = cap;
   return EPET_OK;
@@ -1258,6 +1272,9 @@ static epet_status redo_overflow(WalkArgs a, const int32_t* ovf_rows, int n, int
   if (walk_smem(a.G, *cap2) > (size_t)max_dyn_smem())
     return set_error(EPET_ERR_UNSUPPORTED, "per-row window of %d cells exceeds shared memory",
                      *cap2);
+  // the column table must end before the slab windows, whatever the window
+  const int room = *cap2 + 2 * std::max(a.G.p.grid.n[0], a.G.p.grid.n[2]);
+  if (walk_smem(a.G, room) <= (size_t)max_dyn_smem()) *cap2 = room;
   WalkArgs b = a;
   b.sel = sel;
   b.m = n;
@@ -1396,12 +1413,14 @@ static epet_status run_walk(const Geo& G, const int32_t* rows, int64_t m,
                                       st));
       n_overflow_rows_ += fl[0];
       // the redone rows can add to the list of rows with an axis-parallel ray
-      EPET_CUDA(cudaMemcpyAsync(&fl[2], flags + 2, 4, cudaMemcpyDeviceToHost, st));
+      EPET_CUDA(cudaMemcpyAsync(fl, flags, 12, cudaMemcpyDeviceToHost, st));
       EPET_CUDA(cudaStreamSynchronize(st));
+      if (fl[0] > 0)
+        return set_error(EPET_ERR_UNSUPPORTED, "%d per-row windows exceed shared memory", fl[0]);
     }
     if (fl[2] > 0) {
       // rows with an axis-parallel ray: per-candidate path
-      EPET_CHECK(exact_rows_apply(G, rows + c0, ex_rows, fl[2], kMode, row_len,
+      EPET_CHECK(exact_rows_apply(G, rows + c0, ex_rows, fl[2], rays, kMode, row_len,
                                   csr ? ovf_idx : nullptr, &exr, a.x, a.y, a.e, a.c, a.s64,
                                   a.ycnt, a.c64, st));
       n_exact_rows_ += fl[2];

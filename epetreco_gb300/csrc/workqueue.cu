@@ -115,6 +115,69 @@ k_workqueue(Geo G, const int32_t* __restrict__ rows, int64_t m,
   if (!kFill && lane == 0) row_count[row] = count;
 }
 
+// The same with a CTA of kWqBlock threads per channel, for lists too short to
+// fill the device with a warp each: a warp takes a channel's ny*nx columns 32
+// at a time, one round after the other (85 rounds at 52^3: 59 us for the
+// count and 118 us for the pairs of a single row); a CTA takes kWqBlock at a
+// time and orders them with a block scan.
+constexpr int kWqBlock = 1024;
+template <bool kFill>
+__global__ void __launch_bounds__(kWqBlock)
+k_workqueue_block(Geo G, const int32_t* __restrict__ rows, int64_t* __restrict__ row_count,
+                  const int64_t* __restrict__ row_off, int32_t* __restrict__ out_cnl,
+                  int32_t* __restrict__ out_vxl) {
+  __shared__ int tot[2][kWqBlock / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t row = blockIdx.x;
+  const int cnl = rows[row];
+  ChannelLine L;
+  CrystalMat m0, m1;
+  channel_line(G, cnl, &L, nullptr, &m0, &m1);
+  float u[3];
+  line_unit(L, u);
+  const float Reff = G.sum_radii * 1.01f + 1e-6f;
+  const float R2 = Reff * Reff;
+  const epet_grid& g = G.p.grid;
+  const int ny = g.n[1];
+  const int ncol = g.n[0] * ny;
+  const int64_t base = kFill ? row_off[row] : 0;
+  int64_t count = 0;
+  for (int q0 = 0, buf = 0; q0 < ncol; q0 += kWqBlock, buf ^= 1) {
+    const int q = q0 + threadIdx.x;
+    int zlo = 1, zhi = 0, ix = 0, iy = 0;
+    int c = 0;
+    if (q < ncol) {
+      ix = q / ny;
+      iy = q - ix * ny;
+      column_z_range(G, L, u, R2, ix, iy, &zlo, &zhi);
+      for (int iz = zlo; iz <= zhi; iz++) c += is_candidate(G, L, ix, iy, iz);
+    }
+    const int inc = warp_incl_scan(c);
+    if (lane == 31) tot[buf][w] = inc;
+    __syncthreads();  // (the other buffer is free again: its readers are past it)
+    const int t = tot[buf][lane];  // kWqBlock / 32 = 32 warps
+    const int tinc = warp_incl_scan(t);
+    const int before = __shfl_sync(0xffffffffu, tinc - t, w);
+    const int all = __shfl_sync(0xffffffffu, tinc, 31);
+    if (kFill && c > 0) {
+      int64_t o = base + count + before + (inc - c);
+      const int vb = ix * G.nyz + iy * g.n[2];
+      for (int iz = zlo; iz <= zhi; iz++)
+        if (is_candidate(G, L, ix, iy, iz)) {
+          out_cnl[o] = cnl;
+          out_vxl[o] = vb + iz;
+          o++;
+        }
+    }
+    count += all;
+  }
+  if (!kFill && threadIdx.x == 0) row_count[row] = count;
+}
+
+// A CTA per row up to four rows per SM: beyond that a warp per row has enough
+// warps to hide its rounds.
+static bool workqueue_by_block(int64_t m) { return m <= 4 * (int64_t)num_sms(); }
+
 // Slab chord length of a ray in the box of voxel (ix,iy,iz), as
 // intersectionLength (getSystemMatrixFromWorkqueue.cu:24-69): axes where the
 // ray's two points coincide are left out of the entry/exit max/min.
@@ -163,7 +226,7 @@ constexpr int kValThreads = 128;
 // the walk hands to this path get values of the same definition.
 template <bool Exact>
 __global__ void __launch_bounds__(kValThreads)
-k_values(Geo G, const float* __restrict__ rays, int64_t m,
+k_values(Geo G, const float* __restrict__ rays, const int32_t* __restrict__ ray_row, int64_t m,
          const int64_t* __restrict__ row_ptr, const int32_t* __restrict__ col,
          float* __restrict__ val) {
   extern __shared__ float sray[];
@@ -173,7 +236,7 @@ k_values(Geo G, const float* __restrict__ rays, int64_t m,
   const int64_t first = b + (int64_t)blockIdx.y * kValThreads;
   if (first >= e) return;  // uniform across the block
   const int R = G.p.nrays;
-  const float* src = rays + row * (int64_t)R * 6;
+  const float* src = rays + (ray_row ? (int64_t)ray_row[row] : row) * R * 6;
   for (int i = threadIdx.x; i < R * 6; i += kValThreads) sray[i] = src[i];
   __syncthreads();
   const epet_grid& g = G.p.grid;
@@ -272,6 +335,12 @@ __global__ void k_expand_rows(const int64_t* __restrict__ row_ptr, int64_t m,
 epet_status launch_workqueue_count(const Geo& G, const int32_t* rows, int64_t m,
                                    int64_t* row_count, cudaStream_t st) {
   if (m == 0) return EPET_OK;
+  if (workqueue_by_block(m)) {
+    k_workqueue_block<false><<<(unsigned)m, kWqBlock, 0, st>>>(G, rows, row_count, nullptr, nullptr,
+                                                               nullptr);
+    EPET_LAUNCHED();
+    return EPET_OK;
+  }
   k_workqueue<false><<<ceil_div(m, kWqWarps), 32 * kWqWarps, 0, st>>>(
       G, rows, m, row_count, nullptr, nullptr, nullptr);
   EPET_LAUNCHED();
@@ -282,13 +351,18 @@ epet_status launch_workqueue_fill(const Geo& G, const int32_t* rows, int64_t m,
                                   const int64_t* row_off, int32_t* cnl, int32_t* vxl,
                                   cudaStream_t st) {
   if (m == 0) return EPET_OK;
+  if (workqueue_by_block(m)) {
+    k_workqueue_block<true><<<(unsigned)m, kWqBlock, 0, st>>>(G, rows, nullptr, row_off, cnl, vxl);
+    EPET_LAUNCHED();
+    return EPET_OK;
+  }
   k_workqueue<true><<<ceil_div(m, kWqWarps), 32 * kWqWarps, 0, st>>>(
       G, rows, m, nullptr, row_off, cnl, vxl);
   EPET_LAUNCHED();
   return EPET_OK;
 }
 
-epet_status launch_values(const Geo& G, const float* rays, int64_t m,
+epet_status launch_values(const Geo& G, const float* rays, const int32_t* ray_row, int64_t m,
                           const int64_t* row_ptr, const int32_t* col, float* val,
                           bool exact, cudaStream_t st) {
   if (m == 0) return EPET_OK;
@@ -300,11 +374,11 @@ epet_status launch_values(const Geo& G, const float* rays, int64_t m,
   if (exact) {
     EPET_CUDA(cudaFuncSetAttribute(k_values<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
-    k_values<true><<<grid, kValThreads, smem, st>>>(G, rays, m, row_ptr, col, val);
+    k_values<true><<<grid, kValThreads, smem, st>>>(G, rays, ray_row, m, row_ptr, col, val);
   } else {
     EPET_CUDA(cudaFuncSetAttribute(k_values<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)smem));
-    k_values<false><<<grid, kValThreads, smem, st>>>(G, rays, m, row_ptr, col, val);
+    k_values<false><<<grid, kValThreads, smem, st>>>(G, rays, ray_row, m, row_ptr, col, val);
   }
   EPET_LAUNCHED();
   return EPET_OK;
@@ -321,8 +395,8 @@ void ExactRows::release(cudaStream_t st) {
 
 // Per-candidate path for a few rows (list ex_rows of indices into rows).
 epet_status exact_rows_apply(const Geo& G, const int32_t* rows, const int32_t* ex_rows,
-                             int64_t n_ex, int mode, int32_t* row_len, int32_t* src_idx,
-                             ExactRows* keep, const float* x, float* y, const float* e,
+                             int64_t n_ex, const float* rays, int mode, int32_t* row_len,
+                             int32_t* src_idx, ExactRows* keep, const float* x, float* y, const float* e,
                              float* c, double* s64, const float* ycnt, double* c64,
                              cudaStream_t st) {
   if (n_ex == 0) return EPET_OK;
@@ -352,18 +426,16 @@ epet_status exact_rows_apply(const Geo& G, const int32_t* rows, const int32_t* e
   EPET_CUDA(cudaStreamSynchronize(st));
   const int64_t tt = std::max<int64_t>(total, 1);
   Scratch t2;
-  EPET_CHECK(t2.init(nullptr, 0, 2 * align256((size_t)tt * 4) +
-                                     align256((size_t)n_ex * G.p.nrays * 24), st));
+  EPET_CHECK(t2.init(nullptr, 0, 2 * align256((size_t)tt * 4), st));
   int32_t* wv = t2.take<int32_t>(tt);
   float* wval = t2.take<float>(tt);
-  float* rays = t2.take<float>((size_t)n_ex * G.p.nrays * 6);
   if (t2.overrun) return set_error(EPET_ERR_INVALID, "internal: exact-row workspace size");
   // candidate channels; in CSR mode the kept columns then overwrite them
   EPET_CUDA(dev_alloc((void**)&out.col, tt * 4, st));
   if (mode == 0) EPET_CUDA(dev_alloc((void**)&out.val, tt * 4, st));
   EPET_CHECK(launch_workqueue_fill(G, cnl, n_ex, out.off, out.col, wv, st));
-  EPET_CHECK(launch_rays(G, cnl, n_ex, rays, false, st));
-  EPET_CHECK(launch_values(G, rays, n_ex, out.off, wv, wval, true, st));
+  // (the walk's rays: generating one row's again took 217 us, a serial stream)
+  EPET_CHECK(launch_values(G, rays, ex_rows, n_ex, out.off, wv, wval, true, st));
   const int T = 128;
   const int nb = ceil_div(n_ex * 32, T);
 #define EPET_APPLY(K)                                                                    \
@@ -449,7 +521,7 @@ epet_status epet_sm_values(const epet_problem* p, const int32_t* rows_d,
   for (int64_t c0 = 0; c0 < m; c0 += ch) {
     const int64_t mc = std::min(ch, m - c0);
     EPET_CHECK(launch_rays(G, rows_d + c0, mc, rays, false, st));
-    EPET_CHECK(launch_values(G, rays, mc, row_ptr_d + c0, col_d, val_d, false, st));
+    EPET_CHECK(launch_values(G, rays, nullptr, mc, row_ptr_d + c0, col_d, val_d, false, st));
   }
   return EPET_OK;
 }
