@@ -127,7 +127,7 @@ struct epet_mlem_batch {
   bool grouped = false;
   void* gdesc = nullptr;      // device, nprob descriptors of the pass
   int64_t* gstart = nullptr;  // device, prefix of the problems' group counts
-  int64_t total_groups = 0;
+  BatchGroups total;
   int32_t* gwide = nullptr;   // device, global ids of the wide groups
   int64_t nwide = 0;
   int graph_kernels = 0;      // kernels in the captured iteration
@@ -176,7 +176,7 @@ epet_status launch_batch_rows(const epet_mlem_batch* h, const RowPlan& plan, boo
 
 epet_status batch_iteration(const epet_mlem_batch* h, cudaStream_t st) {
   if (h->grouped)
-    EPET_CHECK(grouped_pass_batch(h->gdesc, h->gstart, h->np(), h->total_groups, h->gwide,
+    EPET_CHECK(grouped_pass_batch(h->gdesc, h->gstart, h->np(), h->total, h->gwide,
                                   h->nwide, st));
   else
     EPET_CHECK(launch_batch_rows(h, h->plan_fwd, true, st));
@@ -289,8 +289,13 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
   if (all_grouped) {
     ALLOC(h->gdesc, gd_h.size());
     ALLOC(h->gstart, (np + 1) * 8);
-    h->total_groups = gs_h[np];
-    if (h->total_groups > INT32_MAX)
+    for (const epet_mlem* p : h->probs) {
+      h->total.groups += p->G.ngroups;
+      h->total.strips += p->G.nstrips;
+      h->total.entries += p->G.nent;
+      h->total.max_nd = std::max(h->total.max_nd, p->G.max_nd);
+    }
+    if (h->total.groups > INT32_MAX)
       return fail(set_error(EPET_ERR_UNSUPPORTED, "batch: more than 2^31 row groups"));
     h->nwide = (int64_t)gw_h.size();
     if (h->nwide > 0) ALLOC(h->gwide, h->nwide * 4);
@@ -323,7 +328,7 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
       // one pass fills the slots (unless the plan is cached); the slot
       // sums' candidates rerun the (idempotent) update epilogue
       if (!tune_lookup(7, h->voxels, nslots, np, &h->plan_bwd))
-        rc = grouped_pass_batch(h->gdesc, h->gstart, np, h->total_groups, h->gwide, h->nwide,
+        rc = grouped_pass_batch(h->gdesc, h->gstart, np, h->total, h->gwide, h->nwide,
                                 st);
       if (rc == EPET_OK)
         rc = tune_rows(

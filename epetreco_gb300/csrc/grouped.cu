@@ -4,25 +4,24 @@
 // The rows (in the reconstruction's crystal-pair order) are cut into groups
 // of consecutive rows whose distinct columns fit a per-warp table in shared
 // memory.  Consecutive rows in that order are a fan of lines through nearly
-// one point, so a group touches few voxels: at 52^3 voxels a group of 32
-// rows (~14k entries) touches ~1000.  Each entry keeps only its value and a
-// 2-byte rank of its column among the group's sorted distinct columns (the
-// group's table), 6 bytes per entry in FP32 and 4 in BF16/FP16 instead of a
-// CSR plus a column-major copy (16 bytes).  Rows start on 4-entry boundaries
-// and are padded to whole 4-entry chunks with zero values whose rank is a
-// trash slot (past the table), so the pass reads 16-byte chunks with no
-// per-entry bounds tests.
+// one point, so a group touches few voxels, and four consecutive rows (a
+// strip) touch few more than one of them.  A strip is stored as the merged list
+// of its rows' columns: per entry the four rows' values (zero where a row
+// does not touch the column) and a 2-byte rank of the column among the
+// group's sorted distinct columns (the group's table), 18 bytes in FP32 for
+// about 3 non-zeros and 10 in the 16-bit forms, instead of a CSR plus a
+// column-major copy (16 bytes per non-zero).
 //
 // One iteration reads every entry once (k_group_mlem): a warp takes a group,
-// gathers x at the table into shared memory, and row by row forms A x from
-// the shared copy, e = y / (A x) and adds the row times e into the group's
-// shared correction; a row's columns are distinct, so the lanes never write
-// the same word (padding goes to the trash slot, which is never read) and
-// each column's sum runs in row order.  The group's corrections go to one
-// slot per (group, column); the slots of each column, listed in group order
-// (built once: the column-major order of the table's entries), are summed in
-// that order by the slot-sum kernel (k_sums), whose epilogue applies x*c/s.
-// Every sum has an input-determined order, so results are deterministic.
+// gathers x at the table into shared memory, and strip by strip forms A x from
+// the shared copy, e = y / (A x) and adds the strip times e into the group's
+// shared correction; a strip's columns are distinct, so the lanes never write
+// the same word and each column's sum runs in row order.  The group's
+// corrections go to one slot per (group, column); the slots of each column,
+// listed in group order (built once: the column-major order of the table's
+// entries), are summed in that order by the slot-sum kernel (k_sums), whose
+// epilogue applies x*c/s.  Every sum has an input-determined order, so
+// results are deterministic (where an entry lies in memory does not matter).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -39,20 +38,22 @@ namespace epet {
 
 constexpr int kGroupFirstRows = 32;  // rows of a first-cut group (split while too wide)
 constexpr int kGroupThreads = 256;   // threads of the table-building kernels
-constexpr int kTrash = kGroupCap;    // rank of the padding entries
-// Shared tables are indexed by rank (the word of rank r sits in bank r % 32).
-// A row's entries are stored so that each warp-wide shared access of the
-// pass takes 32 consecutive entries of the row (k_group_tables): their ranks
-// ascend by a few, which spreads them over the banks better than the fixed
-// swizzles of the ranks tried: 2.05 distinct-address wavefronts per 32
-// entries on rows of the full workload, against 2.94 with a lane taking 4
-// consecutive entries and the ranks swizzled as r + r / 32 (the pass 7 %
-// faster).  A layout balancing each row over the banks (1.27 wavefronts)
-// was no faster: the pass is bound by the latency of its entry stream.
-__host__ __device__ constexpr int sw_rank(int r) { return r; }
-constexpr int kGroupStride = sw_rank(kGroupCap) + 4;  // floats per shared table (trash included)
-constexpr size_t kGroupSmem = (size_t)kGroupWarps * 2 * kGroupStride * 4;
-static_assert(kGroupSmem <= 227 * 1024, "grouped tables exceed shared memory");
+// Shared tables are indexed by rank (the word of rank r sits in bank r % 32);
+// a group's padding entries have the rank after its last column.
+constexpr int kColsumWarps = 8;  // warps of the column-sum kernel
+constexpr int kMaxStride = kGroupCap + 4;  // floats of the largest shared table
+constexpr size_t kMaxPassSmem = 227 * 1024;
+// Floats of each of a warp's two tables with `warps` warps in a block: fixed, so
+// that a rank's place in the second is the first's plus a constant (with a
+// run-time stride the full-size iteration took 79 ms instead of 73), and no
+// larger than the matrices with that many warps need: what is left of the
+// SM's memory caches the gathers of x (17.1 -> 16.0 ms for 16 small problems).
+__host__ __device__ constexpr int pass_stride(int warps) {
+  return warps == 20 ? 1088 : warps == 16 ? 1312 : kMaxStride;
+}
+constexpr size_t kColsumSmem = (size_t)kColsumWarps * kMaxStride * 4;
+static_assert(kGroupFirstRows <= 64 && kGroupFirstRows % kStrip == 0, "row masks, strips");
+constexpr int kGroupStrips = kGroupFirstRows / kStrip;  // strips of a first cut
 
 // Row r of the source: its columns and values, and its length.
 struct RowSpan {
@@ -71,13 +72,12 @@ __device__ __forceinline__ RowSpan row_span(const RowSource& A, int64_t r) {
   return RowSpan{A.col + b, A.val + b, A.rp[r + 1] - b};
 }
 
-// The spans of rows r0 .. r1 - 1 (at most kGroupFirstRows) in shared memory,
-// with their exclusive prefix off[] (off[nr] = the group's entries); the
-// loads run in parallel, a thread per row.  Ends with a block barrier.
+// The spans of rows r0 .. r1 - 1 (at most kGroupFirstRows) in shared memory;
+// the loads run in parallel, a thread per row.  Ends with a block barrier.
 struct GroupSpans {
   const int32_t* col[kGroupFirstRows];
   const float* val[kGroupFirstRows];
-  int off[kGroupFirstRows + 1];
+  int n[kGroupFirstRows];
 };
 __device__ __forceinline__ void load_spans(const RowSource& A, int r0, int r1, GroupSpans* S) {
   const int nr = r1 - r0;
@@ -88,30 +88,68 @@ __device__ __forceinline__ void load_spans(const RowSource& A, int r0, int r1, G
     S->val[threadIdx.x] = rs.val;
     n = (int)rs.n;
   }
-  if (threadIdx.x < 32) {  // nr <= 32: one warp's scan
-    const int inc = warp_incl_scan(n);
-    if ((int)threadIdx.x < nr) S->off[threadIdx.x + 1] = inc;
-    if (threadIdx.x == 0) S->off[0] = 0;
-  }
+  if ((int)threadIdx.x < nr) S->n[threadIdx.x] = n;
   __syncthreads();
 }
 
-// Sets the group's columns in the bitmap bm: a warp per row, its lanes
-// along the row, four column loads issued before their atomics.
-__device__ __forceinline__ void set_group_columns(const GroupSpans& S, int nr, unsigned* bm) {
+// A warp's walk along a row's columns, four consecutive ones per lane (16-byte
+// loads): f(c, k) gets k of them, ascending.  Neighbouring columns fall into
+// the same bitmap word, so a lane ORs its four together before it touches
+// shared memory, and the lanes of a warp spread over a few words more: with a
+// column per lane a dozen lanes hit one word at a time, and these atomics'
+// replays held the table kernel at 71 % of the L1's throughput.
+template <class F>
+__device__ __forceinline__ void for_row4(const int32_t* __restrict__ col, int n, F&& f) {
   const int lane = threadIdx.x & 31;
-  for (int r = threadIdx.x >> 5; r < nr; r += kGroupThreads / 32) {
-    const int32_t* col = S.col[r];
-    const int n = S.off[r + 1] - S.off[r];
-    for (int j0 = lane; j0 < n; j0 += 128) {
-      int v[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++) v[u] = j0 + 32 * u < n ? col[j0 + 32 * u] : -1;
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (v[u] >= 0) atomicOr(&bm[v[u] >> 5], 1u << (v[u] & 31));
+  // entries before the first 16-byte boundary, whole 16-byte pieces, the rest
+  const int head = min(n, (int)((0u - (unsigned)(reinterpret_cast<uintptr_t>(col) >> 2)) & 3u));
+  const int nv = (n - head) >> 2, tail = n - head - 4 * nv;
+  const int4* v = reinterpret_cast<const int4*>(col + head);
+  if (lane < 2 && (lane ? tail : head) > 0) {
+    const int32_t* p = lane ? col + n - tail : col;
+    const int k = lane ? tail : head;
+    const int c[4] = {p[0], k > 1 ? p[1] : 0, k > 2 ? p[2] : 0, 0};
+    f(c, k);
+  }
+  for (int j = lane; j < nv; j += 64) {
+    const bool two = j + 32 < nv;
+    const int4 q = v[j];
+    int4 r = q;
+    if (two) r = v[j + 32];
+    {
+      const int c[4] = {q.x, q.y, q.z, q.w};
+      f(c, 4);
+    }
+    if (two) {
+      const int c[4] = {r.x, r.y, r.z, r.w};
+      f(c, 4);
     }
   }
+}
+
+// ORs the bits of k ascending positions into a bitmap.
+__device__ __forceinline__ void or_bits(const int* c, int k, unsigned* words) {
+  int w = c[0] >> 5;
+  unsigned m = 1u << (c[0] & 31);
+#pragma unroll
+  for (int t = 1; t < 4; t++) {
+    if (t < k) {
+      const int wt = c[t] >> 5;
+      if (wt != w) {
+        atomicOr(&words[w], m);
+        w = wt;
+        m = 0u;
+      }
+      m |= 1u << (c[t] & 31);
+    }
+  }
+  atomicOr(&words[w], m);
+}
+
+// Sets the group's columns in the bitmap bm, a warp per row.
+__device__ __forceinline__ void set_group_columns(const GroupSpans& S, int nr, unsigned* bm) {
+  for (int r = threadIdx.x >> 5; r < nr; r += kGroupThreads / 32)
+    for_row4(S.col[r], S.n[r], [&](const int* c, int k) { or_bits(c, k, bm); });
 }
 
 // Distinct columns of the candidate groups cand[g] = {r0, r1}: a bitmap over
@@ -139,64 +177,145 @@ k_group_distinct(RowSource A, const int2* __restrict__ cand, int nwords,
   }
 }
 
-// Storage order of a row of nq 4-entry chunks (its entries j in CSR order,
-// then padding): the pass hands chunk 32 u + l to lane l in round u and
-// reads position t of every lane's chunk with one shared access, so the
-// entries are placed for this access to take consecutive entries: round u
-// (cq = min(32, nq - 32 u) chunks) holds entry j = 128 u + t cq + l at chunk
-// l, position t, i.e. at 128 u + 4 l + t.
+// Words of a row's or strip's bitmap over the group's ranks.
+constexpr int kRankWords = kGroupCap / 32;
+static_assert(kGroupCap % 32 == 0, "rank bitmaps");
 
-// Tables and the padded layout of the final groups (one block per group):
-// the group's distinct columns, ascending, at table[tb ..]; every row r's
-// entries at ptr[r] (a multiple of 4) onwards in the storage order above,
-// each as its value and its column's rank among the group's columns, then
-// zero values on the trash rank up to the next multiple of 4.  A single row
-// wider than the shared tables (a "wide" group) keeps its own columns as its
-// table (padded like the row with column 0) and the CSR order; its padding
-// points past the row in that table.
+// A warp's strip while its entries are made: per row and for the strip the
+// bitmap over the ranks and the exclusive prefix of its words.
+struct StripBits {
+  uint32_t row[kStrip][kRankWords];
+  uint16_t rpre[kStrip][kRankWords], apre[kRankWords];
+  __device__ uint32_t all(int w) const { return row[0][w] | row[1][w]; }
+};
+static_assert(kStrip == 2, "StripBits::all");
+constexpr int kListEntries = 1024;  // ranks of a warp's strip, in order, that many at a time
+static_assert(kListEntries % 128 == 0, "whole rounds of the pass");
+
+// Sets a row's ranks in its bitmap.
+__device__ __forceinline__ void set_row_ranks(const int32_t* __restrict__ col, int n,
+                                              const unsigned* bm, const uint16_t* pre,
+                                              uint32_t* words) {
+  for_row4(col, n, [&](const int* c, int k) {
+    int rk[4];
+#pragma unroll
+    for (int t = 0; t < 4; t++) {
+      const unsigned v = (unsigned)c[t];
+      rk[t] = t < k ? pre[v >> 5] + __popc(bm[v >> 5] & ((1u << (v & 31)) - 1u)) : 0;
+    }
+    or_bits(rk, k, words);
+  });
+}
+
+// Exclusive prefixes of the popcounts of the rows' words and of their unions
+// over the first `words` words, packed in one scan (each below 2^10 a round);
+// returns the union's total.
+__device__ __forceinline__ int rank_prefixes(StripBits& Q, int words) {
+  const int lane = threadIdx.x & 31;
+  int run = 0, run0 = 0, run1 = 0;
+  for (int w0 = 0; w0 < words; w0 += 32) {
+    const int w = w0 + lane;
+    const bool ok = w < words;
+    const uint32_t r0 = ok ? Q.row[0][w] : 0u, r1 = ok ? Q.row[1][w] : 0u;
+    // (a round's totals are at most 1024 each: 10 + 1 bits)
+    const int n0 = __popc(r0), n1 = __popc(r1), n = __popc(r0 | r1);
+    const int inc01 = warp_incl_scan(n0 | (n1 << 16)), inc = warp_incl_scan(n);
+    if (ok) {
+      Q.rpre[0][w] = (uint16_t)(run0 + (inc01 & 0xffff) - n0);
+      Q.rpre[1][w] = (uint16_t)(run1 + (inc01 >> 16) - n1);
+      Q.apre[w] = (uint16_t)(run + inc - n);
+    }
+    const int t01 = __shfl_sync(0xffffffffu, inc01, 31);
+    run0 += t01 & 0xffff;
+    run1 += t01 >> 16;
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
+  return run;
+}
+
+// Strips are padded to whole 4-entry chunks.  Chunk 32 r + l is lane l's in
+// round r of the pass, and an access takes one entry of every lane's chunk,
+// so the entries are stored for it to take consecutive ones (ascending
+// ranks): round r (cq = min(32, chunks left) chunks) holds entry 128 r + t cq
+// + l at chunk l, position t.  FP32 values of a round: the first two entries
+// of every chunk (16 bytes each), then the last two, so that each of a lane's
+// two loads is part of one contiguous run (side by side, every 32-byte sector
+// was fetched twice).  Padding: zero values on the group's spare rank.  A wide row's
+// strip (n > kGroupCap) is a plain list.
+__host__ __device__ constexpr int strip_pad(int n) { return (n + 3) & ~3; }
+
+// Where the entries go: the arrays' capacity and the cursor (entries
+// reserved so far: each block takes its strips' share with one atomic add, so
+// the place of a group's entries in memory varies, their contents do not).
+struct EntryOut {
+  unsigned long long* cursor;
+  int64_t cap;
+  StripF* val;
+  uint16_t* loc;
+  StripDesc* strips;
+};
+
+// Tables and entries of groups (one block per group, a warp per strip): the
+// group's distinct columns, ascending, at table[tb ..]; per strip its entries
+// in column order.
 //
-// Two launches.  The first (nd_out set, groups null, table the scratch
-// ftab) takes the first cuts, block b the rows [32 b, min(m, 32 b + 32)): it
-// writes each cut's count of distinct columns to nd_out[b] and, for a cut
-// that fits the shared tables, its table at ftab + b * kGroupCap and its
-// entries.  The second takes the final groups: a first cut kept whole
-// copies its table from ftab to its slots; the groups made by splitting
-// wider cuts are laid out in full.
-__global__ void __launch_bounds__(kGroupThreads, 8)
+// Three uses.  Counting (entries.val null): block b takes the first cut
+// b * every and only adds its strips' entries to the cursor.  First cuts
+// (nd_out set): block b takes the rows [R b, min(m, R b + R)), writes the
+// cut's count of distinct columns to nd_out[b] and, for a cut that fits the
+// shared tables, its table to ftab + b * kGroupCap and its entries, with the
+// strip descriptors at [R / kStrip * b ..] (scratch, like ftab).  Final groups: a
+// first cut kept whole copies its table and strip descriptors to their
+// places; a group made by splitting a wider cut is laid out in full; a
+// single row wider than the shared tables (a "wide" group) keeps its own
+// columns as its table, its entries in that order (ranks unused).
+__global__ void __launch_bounds__(kGroupThreads)
 k_group_tables(RowSource A, const GroupDesc* __restrict__ groups, int64_t m, int nwords,
-               const int64_t* __restrict__ ptr, int32_t* __restrict__ table,
-               const int32_t* __restrict__ ftab, int32_t* __restrict__ nd_out,
-               float* __restrict__ pval, uint16_t* __restrict__ ploc) {
-  extern __shared__ unsigned gsh[];
-  unsigned* bm = gsh;
-  // per bitmap word the rank of its first column (< kGroupCap where read):
-  // 16 bits keep the block at 6 bytes per word (8 blocks per SM at 52^3)
-  uint16_t* pre = reinterpret_cast<uint16_t*>(gsh + nwords);
-  __shared__ int wtot[kGroupThreads / 32];
+               int64_t every, int32_t* __restrict__ table, const int32_t* __restrict__ ftab,
+               const StripDesc* __restrict__ fstrips, int32_t* __restrict__ nd_out, EntryOut out) {
+  extern __shared__ __align__(16) unsigned gsh[];
+  StripBits* sbits = reinterpret_cast<StripBits*>(gsh);
+  unsigned* bm = gsh + sizeof(StripBits) * kGroupStrips / 4;
+  // per bitmap word the rank of its first column (< kGroupCap where read)
+  uint16_t* pre = reinterpret_cast<uint16_t*>(bm + nwords);
+  __shared__ int wtot[kGroupThreads / 32], sn[kGroupStrips];
   __shared__ int s_nd;
-  const bool first = nd_out != nullptr;
+  __shared__ unsigned long long s_base;
+  const bool count = out.val == nullptr, first = count || nd_out != nullptr;
   GroupDesc gd;
   if (first) {
-    const int64_t r0 = (int64_t)blockIdx.x * kGroupFirstRows;
-    gd = GroupDesc{(int32_t)r0, (int32_t)min(m, r0 + kGroupFirstRows), 0, 0};
+    const int64_t r0 = (int64_t)blockIdx.x * every * kGroupFirstRows;
+    gd = GroupDesc{(int32_t)r0, (int32_t)min(m, r0 + kGroupFirstRows), 0, 0,
+                   (int32_t)(blockIdx.x * kGroupStrips)};
   } else {
     gd = groups[blockIdx.x];
     if (gd.nd <= kGroupCap && gd.r0 % kGroupFirstRows == 0 &&
         gd.r1 == min(m, (int64_t)gd.r0 + kGroupFirstRows)) {
       // a first cut kept whole: laid out by the first launch
-      const int32_t* src = ftab + (int64_t)(gd.r0 / kGroupFirstRows) * kGroupCap;
+      const int64_t cut = gd.r0 / kGroupFirstRows;
+      const int32_t* src = ftab + cut * kGroupCap;
       for (int j = threadIdx.x; j < gd.nd; j += kGroupThreads) table[gd.tb + j] = src[j];
+      if ((int)threadIdx.x < (gd.r1 - gd.r0 + kStrip - 1) / kStrip)
+        out.strips[gd.qb + threadIdx.x] = fstrips[cut * kGroupStrips + threadIdx.x];
       return;
     }
   }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (!first && gd.nd > kGroupCap) {  // wide: one row
     const RowSpan rs = row_span(A, gd.r0);
-    const int64_t d = ptr[gd.r0], pn = ptr[gd.r0 + 1] - d;
-    for (int64_t j = threadIdx.x; j < gd.nd; j += kGroupThreads)
-      table[gd.tb + j] = j < rs.n ? rs.col[j] : 0;
-    for (int64_t j = threadIdx.x; j < pn; j += kGroupThreads) {
-      pval[d + j] = j < rs.n ? rs.val[j] : 0.f;
-      ploc[d + j] = 0;  // (unused: a wide row reads its table by position)
+    const int np = strip_pad((int)rs.n);
+    if (threadIdx.x == 0) s_base = atomicAdd(out.cursor, (unsigned long long)np);
+    __syncthreads();
+    const int64_t base = (int64_t)s_base;
+    if (threadIdx.x == 0) out.strips[gd.qb] = StripDesc{base, (int32_t)rs.n, gd.r0};
+    for (int64_t j = threadIdx.x; j < np; j += kGroupThreads) {
+      if (j < rs.n) table[gd.tb + j] = rs.col[j];
+      if (base + np <= out.cap) {
+        StripF v = {};
+        v.v[0] = j < rs.n ? rs.val[j] : 0.f;
+        out.val[base + j] = v;
+        out.loc[base + j] = 0;
+      }
     }
     return;
   }
@@ -212,7 +331,6 @@ k_group_tables(RowSource A, const GroupDesc* __restrict__ groups, int64_t m, int
   const int wb = min(nwords, (int)threadIdx.x * per), we = min(nwords, wb + per);
   int cnt = 0;
   for (int w = wb; w < we; w++) cnt += __popc(bm[w]);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int inc = warp_incl_scan(cnt);
   if (lane == 31) wtot[wid] = inc;
   __syncthreads();
@@ -223,69 +341,122 @@ k_group_tables(RowSource A, const GroupDesc* __restrict__ groups, int64_t m, int
     if (lane == kGroupThreads / 32 - 1) s_nd = ti;
   }
   __syncthreads();
-  if (first) {  // (uniform across the block)
-    if (threadIdx.x == 0) nd_out[blockIdx.x] = s_nd;
-    if (s_nd > kGroupCap) return;  // split by the host, laid out by the second launch
+  const int nd = s_nd;  // (uniform across the block)
+  if (first && !count && threadIdx.x == 0) nd_out[blockIdx.x] = nd;
+  if (nd > kGroupCap) {
+    // split by the host, laid out by the last launch; while counting, taken
+    // as if each row had its own entries
+    if (count) {
+      for (int r = threadIdx.x; r < nr; r += kGroupThreads)
+        atomicAdd(out.cursor, (unsigned long long)strip_pad(S.n[r]));
+    }
+    return;
   }
   // (the first launch's table is its cut's share of the scratch ftab)
   int32_t* const tab = first ? table + (int64_t)blockIdx.x * kGroupCap : table + gd.tb;
   int run = wtot[wid] + inc - cnt;
   for (int w = wb; w < we; w++) {
     pre[w] = (uint16_t)run;
-    unsigned word = bm[w];
-    while (word) {
-      const int bit = __ffs(word) - 1;
-      tab[run] = w * 32 + bit;
-      run++;
-      word &= word - 1u;
-    }
+    run += __popc(bm[w]);
+  }
+  const int words = (nd + 31) / 32;  // of the ranks
+  for (int i = threadIdx.x; i < kGroupStrips * kStrip * kRankWords; i += kGroupThreads) {
+    const int s = i / (kStrip * kRankWords);
+    (&sbits[s].row[0][0])[i - s * kStrip * kRankWords] = 0u;
   }
   __syncthreads();
-  // the padded layout a 4-entry chunk at a time, a warp per row: lane l
-  // takes chunk l of every round u, which holds the row's entries j = 128 u
-  // + t cq + l (t = 0..3, the storage order above), padding (j past the row)
-  // as zero values on the trash rank; a chunk's values and ranks are
-  // written with one 16-byte and one 8-byte store
-  for (int r = wid; r < nr; r += kGroupThreads / 32) {
-    const int32_t* col = S.col[r];
-    const float* val = S.val[r];
-    const int n = S.off[r + 1] - S.off[r];
-    const int64_t d = ptr[gd.r0 + r];
-    const int nq = (int)((ptr[gd.r0 + r + 1] - d) >> 2);
-    for (int c = lane; c < nq; c += 32) {
-      const int u = c >> 5;
-      const int cq = min(32, nq - 32 * u);
-      int cc[4];
-      float vv[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const int j = 128 * u + t * cq + lane;
-        cc[t] = j < n ? col[j] : -1;
-        vv[t] = j < n ? val[j] : 0.f;
+  if (!count) {
+    // the table, 32 words at a time per warp: a lane per column of each word
+    // that has any
+    for (int w0 = 32 * wid; w0 < nwords; w0 += kGroupThreads) {
+      const unsigned mine = w0 + lane < nwords ? bm[w0 + lane] : 0u;
+      unsigned left = __ballot_sync(0xffffffffu, mine != 0u);
+      while (left) {
+        const int l = __ffs(left) - 1;
+        left &= left - 1u;
+        const unsigned word = __shfl_sync(0xffffffffu, mine, l);
+        if ((word >> lane) & 1u)
+          tab[pre[w0 + l] + __popc(word & ((1u << lane) - 1u))] = (w0 + l) * 32 + lane;
       }
-      unsigned rk[4];
+    }
+  }
+  // the strips' rows as bitmaps over the ranks, and their unions, a warp per
+  // strip
+  const int ns = (nr + kStrip - 1) / kStrip;
+  for (int s = wid; s < kGroupStrips; s += kGroupThreads / 32) {
+    StripBits& Q = sbits[s];
+    int n = 0;
+    if (s < ns) {  // (uniform in the warp)
+      for (int r = 0; r < kStrip && kStrip * s + r < nr; r++)
+        set_row_ranks(S.col[kStrip * s + r], S.n[kStrip * s + r], bm, pre, Q.row[r]);
+      __syncwarp();
+      n = rank_prefixes(Q, words);
+    }
+    if (lane == 0) sn[s] = n;
+  }
+  __syncthreads();
+  int total = 0;
+  for (int s = 0; s < kGroupStrips; s++) total += strip_pad(sn[s]);
+  if (threadIdx.x == 0) s_base = atomicAdd(out.cursor, (unsigned long long)total);
+  if (count) return;
+  __syncthreads();
+  int64_t base = (int64_t)s_base;
+  const bool fits = base + total <= out.cap;  // (else the host sees the cursor and starts again)
+  const unsigned below = (1u << lane) - 1u;
+  // (the columns' bitmap is not needed any more: the lists take its place)
+  uint16_t* list = reinterpret_cast<uint16_t*>(bm) + wid * kListEntries;
+  for (int s = 0; s < ns; base += strip_pad(sn[s]), s++) {
+    if (s % (kGroupThreads / 32) != wid) continue;
+    const int n = sn[s], np = strip_pad(n);
+    if (lane == 0) out.strips[gd.qb + s] = StripDesc{base, n, gd.r0 + kStrip * s};
+    if (!fits) continue;
+    const StripBits& Q = sbits[s];
+    const float* val[kStrip];
 #pragma unroll
-      for (int t = 0; t < 4; t++) {
-        const unsigned v = (unsigned)cc[t];
-        rk[t] = cc[t] >= 0
-                    ? (unsigned)sw_rank(pre[v >> 5] + __popc(bm[v >> 5] & ((1u << (v & 31)) - 1u)))
-                    : (unsigned)sw_rank(kTrash);
+    for (int r = 0; r < kStrip; r++) val[r] = kStrip * s + r < nr ? S.val[kStrip * s + r] : nullptr;
+    for (int e0 = 0; e0 < n; e0 += kListEntries) {
+      for (int w = 0; w < words; w++) {
+        const uint32_t all = Q.all(w);
+        const unsigned i = Q.apre[w] + __popc(all & below) - e0;
+        if (((all >> lane) & 1u) && i < (unsigned)kListEntries) list[i] = (uint16_t)(32 * w + lane);
       }
-      *reinterpret_cast<float4*>(pval + d + 4 * c) = make_float4(vv[0], vv[1], vv[2], vv[3]);
-      *reinterpret_cast<uint2*>(ploc + d + 4 * c) = make_uint2(rk[0] | (rk[1] << 16),
-                                                               rk[2] | (rk[3] << 16));
+      __syncwarp();
+      // a chunk per lane, in the storage order
+      for (int c = e0 / 4 + lane; c < min(np, e0 + kListEntries) / 4; c += 32) {
+        const int first_e = c & ~31, cq = min(32, np / 4 - first_e);  // chunks of this round
+        StripF v[4];
+        unsigned rk[4];
+  #pragma unroll
+        for (int t = 0; t < 4; t++) {
+          const int i = 4 * first_e + t * cq + lane;
+          rk[t] = i < n ? list[i - e0] : nd;
+          const int w = min((int)rk[t] >> 5, kRankWords - 1), bit = rk[t] & 31;
+          const uint32_t lower = (1u << bit) - 1u;
+  #pragma unroll
+          for (int r = 0; r < kStrip; r++) {
+            const uint32_t mine = Q.row[r][w];
+            const bool has = i < n && ((mine >> bit) & 1u);
+            v[t].v[r] = has ? val[r][Q.rpre[r][w] + __popc(mine & lower)] : 0.f;
+          }
+        }
+        float4* q = reinterpret_cast<float4*>(out.val + base + 4 * first_e) + lane;
+        q[0] = make_float4(v[0].v[0], v[0].v[1], v[1].v[0], v[1].v[1]);
+        q[cq] = make_float4(v[2].v[0], v[2].v[1], v[3].v[0], v[3].v[1]);
+        *reinterpret_cast<uint2*>(out.loc + base + 4 * c) =
+            make_uint2(rk[0] | (rk[1] << 16), rk[2] | (rk[3] << 16));
+      }
+      __syncwarp();
     }
   }
 }
 
-// Dynamic shared memory of k_group_tables: the bitmap and the word ranks.
-static size_t table_smem(int nwords) { return (size_t)nwords * 6; }
+constexpr int64_t kSampleCuts = 2048;  // first cuts counted to size the entries' arrays
 
-__global__ void k_padded_len(RowSource A, int64_t m, int64_t* __restrict__ len) {
-  const int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= m) return;
-  const int64_t q = A.segs ? A.idx[r] : r;
-  len[r] = (A.rp[q + 1] - A.rp[q] + 3) & ~int64_t(3);
+// Dynamic shared memory of k_group_tables: the strips' bitmaps, the group's
+// bitmap and its word ranks, later a list of ranks per warp.
+static size_t table_smem(int nwords) {
+  return sizeof(StripBits) * kGroupStrips +
+         std::max((size_t)nwords * 6, (size_t)(kGroupThreads / 32) * kListEntries * 2);
 }
 
 __global__ void k_fill_f32(float* __restrict__ p, int64_t n, float v) {
@@ -317,67 +488,88 @@ __device__ __forceinline__ float gq_from(uint32_t q) {
   return __half2float(__ushort_as_half((unsigned short)q));
 }
 
+// 16-bit values of a strip's rows and their scales, a warp per strip.
 template <int FMT>
-__global__ void k_group_quantise(const int64_t* __restrict__ ptr, const float* __restrict__ val,
-                                 int64_t m, float* __restrict__ scale, uint16_t* __restrict__ q) {
-  const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+__global__ void k_group_quantise(const StripDesc* __restrict__ strips, int64_t nstrips,
+                                 const StripF* __restrict__ val, int64_t m,
+                                 float* __restrict__ scale, StripH* __restrict__ q) {
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (r >= m) return;
-  const int64_t b = ptr[r], e = ptr[r + 1];
-  float mx = 0.f;
-  for (int64_t k = b + lane; k < e; k += 32) mx = fmaxf(mx, fabsf(val[k]));
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-  const float sc = mx > 0.f ? mx : 1.f;
-  if (lane == 0) scale[r] = sc;
-  for (int64_t k = b + lane; k < e; k += 32) q[k] = gq_to<FMT>(__fdiv_rn(val[k], sc));
-}
-
-// A row's entries as the pass holds them: 4-entry chunks, chunk u of lane l
-// the (l + 32 u)-th chunk of the (padded) row; values raw (FP32: float4,
-// 16-bit: 4 x 16 bits) and column ranks as 4 x 16 bits.
-constexpr int kGroupRounds = 4;  // chunks per lane held in registers (512 entries a row)
-template <int FMT>
-struct RowBuf {
-  using V = typename std::conditional<FMT == 0, float4, uint2>::type;
-  V v[kGroupRounds];
-  uint2 l[kGroupRounds];
-};
-
-__device__ __forceinline__ float gval4(const float4& c, int t) {
-  return t == 0 ? c.x : t == 1 ? c.y : t == 2 ? c.z : c.w;
-}
-template <int FMT>
-__device__ __forceinline__ float gval(const typename RowBuf<FMT>::V& c, int t) {
-  if constexpr (FMT == 0) {
-    return gval4(c, t);
-  } else {
-    const uint32_t w = t < 2 ? c.x : c.y;
-    return gq_from<FMT>((t & 1) ? (w >> 16) : (w & 0xffffu));
+  if (i >= nstrips) return;
+  const StripDesc d = strips[i];
+  // (strips are in row order: this one ends where the next begins)
+  const int nr = (int)((i + 1 < nstrips ? strips[i + 1].r0 : m) - d.r0);
+  const bool wide = d.n > kGroupCap;
+  float mx[kStrip] = {};
+  for (int64_t k = d.start + lane; k < d.start + strip_pad(d.n); k += 32) {
+    // (pairs of values: the same two rows whatever the order of the entries)
+    const StripF v = val[k];
+#pragma unroll
+    for (int j = 0; j < kStrip; j++) mx[j] = fmaxf(mx[j], fabsf(v.v[j]));
+  }
+  float sc[kStrip];
+#pragma unroll
+  for (int j = 0; j < kStrip; j++) {
+    for (int o = 16; o > 0; o >>= 1) mx[j] = fmaxf(mx[j], __shfl_xor_sync(0xffffffffu, mx[j], o));
+    sc[j] = mx[j] > 0.f ? mx[j] : 1.f;
+    if (lane == 0 && j < nr) scale[d.r0 + j] = sc[j];
+  }
+  for (int k = lane; k < strip_pad(d.n); k += 32) {
+    const StripF v = val[d.start + k];
+    StripH b;
+#pragma unroll
+    for (int j = 0; j < kStrip; j++) b.v[j] = gq_to<FMT>(__fdiv_rn(v.v[j], sc[j]));
+    // FP32 position k of round u: half h, chunk l, entry 2 h + e of it; the
+    // 16-bit values of a chunk lie together
+    int to = k;
+    if (!wide) {
+      const int u = k >> 7, cq = min(32, strip_pad(d.n) / 4 - 32 * u);
+      const int i = k & 127, h = i >= 2 * cq ? 1 : 0, r = i - 2 * cq * h;
+      to = 128 * u + 4 * (r >> 1) + 2 * h + (r & 1);
+    }
+    q[d.start + to] = b;
   }
 }
-__device__ __forceinline__ int grank(const uint2& c, int t) {
+
+// A strip's entries as the pass holds them: chunk 32 r + lane in slot r (up to
+// 128 ROUNDS entries of a strip), four
+// entries of two values (FP32: two float4, 16-bit: 8 x 16 bits) and their
+// ranks (4 x 16 bits).
+static_assert(kStrip == 2, "a chunk's loads");
+struct Chunk32 {
+  float4 a, b;
+};
+template <int FMT>
+using ChunkV = typename std::conditional<FMT == 0, Chunk32, uint4>::type;
+template <int FMT, int ROUNDS>
+struct StripBuf {
+  ChunkV<FMT> v[ROUNDS];
+  uint2 l[ROUNDS];
+};
+// Row j's value of entry t.
+template <int FMT>
+__device__ __forceinline__ float cvalue(const ChunkV<FMT>& c, int t, int j) {
+  if constexpr (FMT == 0) {
+    const float4& q = t < 2 ? c.a : c.b;
+    const int k = 2 * (t & 1) + j;
+    return k == 0 ? q.x : k == 1 ? q.y : k == 2 ? q.z : q.w;
+  } else {
+    const uint32_t w = t == 0 ? c.x : t == 1 ? c.y : t == 2 ? c.z : c.w;
+    return gq_from<FMT>(j ? w >> 16 : w & 0xffffu);
+  }
+}
+__device__ __forceinline__ int crank(const uint2& c, int t) {
   const uint32_t w = t < 2 ? c.x : c.y;
   return (int)((t & 1) ? (w >> 16) : (w & 0xffffu));
-}
-
-template <int FMT>
-__device__ __forceinline__ void gload_chunk(const void* __restrict__ val,
-                                            const uint16_t* __restrict__ loc, int64_t k4,
-                                            typename RowBuf<FMT>::V* v, uint2* l) {
-  if constexpr (FMT == 0)
-    *v = __ldcs(reinterpret_cast<const float4*>(static_cast<const float*>(val) + k4));
-  else
-    *v = __ldcs(reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(val) + k4));
-  *l = __ldcs(reinterpret_cast<const uint2*>(loc + k4));
 }
 
 struct GroupIterArgs {
   const GroupDesc* groups;
   int64_t ngroups;
-  const int64_t* row_ptr;  // padded (multiples of 4)
-  const void* val;         // float (FP32) or 16-bit bits, padded
-  const float* scale;      // per row (16-bit forms)
-  const uint16_t* loc;     // padded
+  const StripDesc* strips;
+  const void* val;     // StripF (FP32) or StripH (16-bit) per entry
+  const float* scale;  // per row (16-bit forms)
+  const uint16_t* loc;
   const int32_t* table;
   const float* x;
   const float* y;
@@ -385,12 +577,30 @@ struct GroupIterArgs {
   float* partial;
 };
 
-// What a group's pass needs before its first row: its row pointers, counts
-// and scales, one row per lane (a group has at most 32 rows), loaded one
-// group ahead.
+// The chunk of lane `lane` in round u of the strip of nq chunks at `start`.
+template <int FMT>
+__device__ __forceinline__ void gload(const void* val, const uint16_t* loc, int64_t start, int nq,
+                                      int u, int lane, ChunkV<FMT>* v, uint2* l) {
+  const int64_t k = start + 128 * u;
+  if constexpr (FMT == 0) {
+    const float4* p =
+        reinterpret_cast<const float4*>(static_cast<const StripF*>(val) + k) + lane;
+    v->a = __ldcs(p);
+    v->b = __ldcs(p + min(32, nq - 32 * u));
+  } else {
+    *v = __ldcs(reinterpret_cast<const uint4*>(static_cast<const StripH*>(val) + k) + lane);
+  }
+  *l = __ldcs(reinterpret_cast<const uint2*>(loc + k) + lane);
+}
+
+// What a group's pass needs before its first strip: its counts and scales, a
+// row per lane, and its strips, one per lane (a group has at most 32 rows),
+// loaded one group ahead.
+static_assert(kGroupFirstRows <= 32, "a row per lane");
 struct GroupHead {
   GroupDesc gd;
-  int64_t rp, rp_end;
+  int64_t qs;
+  int qn;
   float y, sc;
 };
 
@@ -400,174 +610,240 @@ __device__ __forceinline__ GroupHead group_head(const GroupIterArgs& a, const Gr
   GroupHead h;
   h.gd = gd;
   const int nr = gd.r1 - gd.r0;
-  h.rp = lane <= nr ? a.row_ptr[gd.r0 + lane] : 0;
-  h.rp_end = a.row_ptr[gd.r1];
+  h.qs = 0;
+  h.qn = 0;
+  if (lane < (nr + kStrip - 1) / kStrip) {
+    const StripDesc q = a.strips[gd.qb + lane];
+    h.qs = q.start;
+    h.qn = q.n;
+  }
   h.y = lane < nr ? a.y[gd.r0 + lane] : 0.f;
   h.sc = FMT != 0 && lane < nr ? a.scale[gd.r0 + lane] : 1.f;
   return h;
 }
 
 // One group of the MLEM pass (a warp): per row ybar = A x, e = y / ybar (0
-// where ybar == 0, the fused epilogue's guard) and the row's share of A^T e
-// added, row after row, to the group's shared correction, written to
-// partial[slot] at the end.  The next row's entries are in flight while a
-// row is reduced and scattered.
-// Which groups a pass instantiation handles: kOrdinary (tables in shared
-// memory), kWide (one row wider than the shared tables, its own columns as
-// its table, read from global memory), or kAny (decided per group).  The
-// ordinary groups' kernel carries none of the wide path's instructions:
-// with them (kAny) the full-size iteration took 4.85 ms instead of 4.16.
-enum GroupKind { kOrdinary = 0, kWide = 1, kAny = 2 };
-
-template <int FMT, int KIND>
-__device__ __forceinline__ void group_pass_as(const GroupIterArgs& a, const GroupHead& H,
-                                              float* xs, float* cs, int lane) {
+// where ybar == 0, the fused epilogue's guard) and the strip's share of A^T e
+// added, strip after strip, to the group's shared correction, written to
+// partial[slot] at the end.
+//
+// Merging two rows per entry cuts what the pass issues per non-zero: one read
+// of x and one read and write of the correction per entry (0.6 per non-zero),
+// the ranks' decoding, and one warp sum, division and broadcast per two rows.
+// The next strip's entries are in flight while a strip is reduced and added.
+// Bound by the latency of those loads and of the chain from a strip's sums to
+// its corrections.  One row at a time: 120 M instructions, 279 us for the
+// first 400,000 channels of the full workload, 4.24 ms an iteration at full
+// size (the slot sums included); in strips of two 87 M, 255 us, 3.66 ms.
+// Tried: strips of four (more registers than a thread has), a ring in shared
+// memory filled by asynchronous copies ahead of the pass (5.2 ms: a third of
+// the tables' room and twice the instructions).
+template <int FMT, int ROUNDS>
+__device__ __forceinline__ void group_pass(const GroupIterArgs& a, const GroupHead& H, float* xs,
+                                           float* cs, int lane) {
   const GroupDesc& gd = H.gd;
-  const int nr = gd.r1 - gd.r0;  // <= 32
-  const bool wide = KIND == kAny ? gd.nd > kGroupCap : KIND == kWide;
-  float yb_l = 0.f;
-  auto row_begin = [&](int i) -> int64_t { return __shfl_sync(0xffffffffu, H.rp, i); };
-  auto row_end = [&](int i) -> int64_t {
-    const int64_t t = __shfl_sync(0xffffffffu, H.rp, (i + 1) & 31);
-    return i + 1 < 32 ? t : H.rp_end;
+  const int nr = gd.r1 - gd.r0;
+  const int ns = (nr + kStrip - 1) / kStrip;
+  using V = ChunkV<FMT>;
+  // (a batch's descriptors are read where they lie: held in registers, they
+  // would push entries out)
+  const void* const val = a.val;
+  const uint16_t* const loc = a.loc;
+  auto load_strip = [&](int k, StripBuf<FMT, ROUNDS>& B) {
+    const int64_t start = __shfl_sync(0xffffffffu, H.qs, k);
+    const int nq = (__shfl_sync(0xffffffffu, H.qn, k) + 3) >> 2;
+#pragma unroll
+    for (int u = 0; u < ROUNDS; u++)
+      if (lane + 32 * u < nq) gload<FMT>(val, loc, start, nq, u, lane, &B.v[u], &B.l[u]);
   };
-  if (!wide) {
-    // x at the table: batches of 8 independent table loads, then their x
-    // gathers
-    for (int j0 = 0; j0 < gd.nd; j0 += 8 * 32) {
-      int col[8];
+  StripBuf<FMT, ROUNDS> b0, b1;
+  load_strip(0, b0);
+  // x at the table: batches of 8 independent table loads, then their x
+  // gathers.  An entry's zeros (a row that does not touch its column) must
+  // not meet an infinite x or ratio: such groups or strips take the tested
+  // form below.
+  bool odd = false;
+  for (int j0 = 0; j0 < gd.nd; j0 += 8 * 32) {
+    int col[8];
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int j = j0 + 32 * k + lane;
-        col[k] = j < gd.nd ? __ldg(a.table + gd.tb + j) : 0;
+    for (int k = 0; k < 8; k++) {
+      const int j = j0 + 32 * k + lane;
+      col[k] = j < gd.nd ? __ldg(a.table + gd.tb + j) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int j = j0 + 32 * k + lane;
+      const float xv = __ldg(a.x + col[k]);
+      if (j < gd.nd) {
+        xs[j] = xv;
+        cs[j] = 0.f;
+        odd = odd || !(fabsf(xv) <= 3.402823466e38f);
       }
+    }
+  }
+  if (lane == 0) xs[gd.nd] = 0.f;  // (the padding's rank)
+  odd = __any_sync(0xffffffffu, odd);
+  __syncwarp();
+  float yb_l = 0.f;
+  auto process = [&](int k, const StripBuf<FMT, ROUNDS>& B) {
+    const int n = __shfl_sync(0xffffffffu, H.qn, k);
+    const int nq = (n + 3) >> 2;
+    float s0[2] = {0.f, 0.f}, s1[2] = {0.f, 0.f};
+    auto dot = [&](const V& v, const uint2& l) {
+      float xv[4];
 #pragma unroll
-      for (int k = 0; k < 8; k++) {
-        const int j = j0 + 32 * k + lane;
-        const float xv = __ldg(a.x + col[k]);
-        if (j < gd.nd) {
-          xs[sw_rank(j)] = xv;
-          cs[sw_rank(j)] = 0.f;
+      for (int t = 0; t < 4; t++) xv[t] = xs[crank(l, t)];
+#pragma unroll
+      for (int t = 0; t < 4; t++) {
+        s0[t & 1] = fmaf(cvalue<FMT>(v, t, 0), xv[t], s0[t & 1]);
+        s1[t & 1] = fmaf(cvalue<FMT>(v, t, 1), xv[t], s1[t & 1]);
+      }
+    };
+    if (!odd) {
+#pragma unroll
+      for (int u = 0; u < ROUNDS; u++)
+        if (lane + 32 * u < nq) dot(B.v[u], B.l[u]);
+      if (nq > 32 * ROUNDS) {
+        const int64_t start = __shfl_sync(0xffffffffu, H.qs, k);
+        for (int u = ROUNDS; 32 * u + lane < nq; u++) {
+          V v;
+          uint2 l;
+          gload<FMT>(val, loc, start, nq, u, lane, &v, &l);
+          dot(v, l);
+        }
+      }
+    } else {
+      const int64_t start = __shfl_sync(0xffffffffu, H.qs, k);
+      for (int u = 0; 32 * u + lane < nq; u++) {
+        V v;
+        uint2 l;
+        gload<FMT>(val, loc, start, nq, u, lane, &v, &l);
+        for (int t = 0; t < 4; t++) {
+          const float xv = xs[crank(l, t)];
+          const float v0 = cvalue<FMT>(v, t, 0), v1 = cvalue<FMT>(v, t, 1);
+          if (v0 != 0.f) s0[0] = fmaf(v0, xv, s0[0]);
+          if (v1 != 0.f) s1[0] = fmaf(v1, xv, s1[0]);
         }
       }
     }
-    if (lane == 0) xs[sw_rank(kTrash)] = 0.f;
-    __syncwarp();
-  }
-  auto load_row = [&](int i, RowBuf<FMT>& B) {
-    const int64_t b = row_begin(i);
-    const int nq = (int)((row_end(i) - b) >> 2);
+    // both rows' sums over the warp: lane l gets that of row l % 2
+    const float a0 = fadd(s0[0], s0[1]), a1 = fadd(s1[0], s1[1]);
+    const bool odd_lane = lane & 1;
+    float d = fadd(odd_lane ? a1 : a0, __shfl_xor_sync(0xffffffffu, odd_lane ? a0 : a1, 1));
 #pragma unroll
-    for (int u = 0; u < kGroupRounds; u++) {
-      const int q = lane + 32 * u;
-      if (q < nq) gload_chunk<FMT>(a.val, a.loc, b + 4 * q, &B.v[u], &B.l[u]);
-    }
-  };
-  auto process_row = [&](int i, const RowBuf<FMT>& B) {
-    const int64_t b = row_begin(i);
-    const int nq = (int)((row_end(i) - b) >> 2);
-    // dot product: four accumulators (entry position t in its chunk), the
-    // shared x loads independent; padding entries are zero
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    auto dot = [&](const typename RowBuf<FMT>::V& vv, const uint2& ll, int q) {
-      float xv[4];
-#pragma unroll
-      for (int t = 0; t < 4; t++)
-        xv[t] = wide ? __ldg(a.x + a.table[gd.tb + 4 * q + t]) : xs[grank(ll, t)];
-#pragma unroll
-      for (int t = 0; t < 4; t++) acc[t] = fmaf(gval<FMT>(vv, t), xv[t], acc[t]);
-    };
-#pragma unroll
-    for (int u = 0; u < kGroupRounds; u++) {
-      const int q = lane + 32 * u;
-      if (q < nq) dot(B.v[u], B.l[u], q);
-    }
-    for (int q = lane + 32 * kGroupRounds; q < nq; q += 32) {  // rows over 512 entries
-      typename RowBuf<FMT>::V vv;
-      uint2 ll;
-      gload_chunk<FMT>(a.val, a.loc, b + 4 * q, &vv, &ll);
-      dot(vv, ll, q);
-    }
-    float d = fadd(fadd(acc[0], acc[1]), fadd(acc[2], acc[3]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-    const float sc = __shfl_sync(0xffffffffu, H.sc, i);
+    for (int o = 2; o < 32; o <<= 1) d = fadd(d, __shfl_xor_sync(0xffffffffu, d, o));
+    const int rl = kStrip * k + (lane & 1);
+    const float sc = FMT == 0 ? 1.f : __shfl_sync(0xffffffffu, H.sc, rl);
     const float yb = FMT == 0 ? d : fmul(d, sc);
-    if (lane == i) yb_l = yb;
     // e = y / (A x) (mlemOperations.hpp:22-32; 0 where A x == 0)
-    const float yr = __shfl_sync(0xffffffffu, H.y, i);
+    const float yr = __shfl_sync(0xffffffffu, H.y, rl);
     const float er = yb > 0.f ? __fdiv_rn(yr, yb) : 0.f;
     const float f = FMT == 0 ? er : fmul(er, sc);
-    // scatter into the group's correction, a chunk at a time: its four
-    // columns are distinct (as all of a row's; padding goes to the trash
-    // slot), so the four sums are read before any is written
-    auto scatter = [&](const typename RowBuf<FMT>::V& vv, const uint2& ll, int q) {
-      if (wide) {
+    if (lane / kStrip == k) yb_l = yb;  // lane = row of the group
+    const float f0 = __shfl_sync(0xffffffffu, f, 0), f1 = __shfl_sync(0xffffffffu, f, 1);
+    // the strip's rows added, in row order, to the group's correction, a
+    // chunk at a time: its four columns are distinct (as all of a strip's;
+    // padding goes to the trash slot), so the four sums are read before any
+    // is written
+    auto add = [&](const V& v, const uint2& l) {
+      float c[4];
 #pragma unroll
-        for (int t = 0; t < 4; t++) a.partial[gd.tb + 4 * q + t] = fmul(gval<FMT>(vv, t), f);
-        return;
-      }
-      float old[4];
+      for (int t = 0; t < 4; t++) c[t] = cs[crank(l, t)];
 #pragma unroll
-      for (int t = 0; t < 4; t++) old[t] = cs[grank(ll, t)];
-#pragma unroll
-      for (int t = 0; t < 4; t++) cs[grank(ll, t)] = fmaf(gval<FMT>(vv, t), f, old[t]);
+      for (int t = 0; t < 4; t++)
+        cs[crank(l, t)] = fmaf(cvalue<FMT>(v, t, 1), f1, fmaf(cvalue<FMT>(v, t, 0), f0, c[t]));
     };
+    if (!odd && fabsf(f0) <= 3.402823466e38f && fabsf(f1) <= 3.402823466e38f) {
 #pragma unroll
-    for (int u = 0; u < kGroupRounds; u++) {
-      const int q = lane + 32 * u;
-      if (q < nq) scatter(B.v[u], B.l[u], q);
-    }
-    for (int q = lane + 32 * kGroupRounds; q < nq; q += 32) {
-      typename RowBuf<FMT>::V vv;
-      uint2 ll;
-      gload_chunk<FMT>(a.val, a.loc, b + 4 * q, &vv, &ll);
-      scatter(vv, ll, q);
+      for (int u = 0; u < ROUNDS; u++)
+        if (lane + 32 * u < nq) add(B.v[u], B.l[u]);
+      if (nq > 32 * ROUNDS) {
+        const int64_t start = __shfl_sync(0xffffffffu, H.qs, k);
+        for (int u = ROUNDS; 32 * u + lane < nq; u++) {
+          V v;
+          uint2 l;
+          gload<FMT>(val, loc, start, nq, u, lane, &v, &l);
+          add(v, l);
+        }
+      }
+    } else {
+      const int64_t start = __shfl_sync(0xffffffffu, H.qs, k);
+      for (int u = 0; 32 * u + lane < nq; u++) {
+        V v;
+        uint2 l;
+        gload<FMT>(val, loc, start, nq, u, lane, &v, &l);
+        for (int t = 0; t < 4; t++) {
+          const float v0 = cvalue<FMT>(v, t, 0), v1 = cvalue<FMT>(v, t, 1);
+          float c = cs[crank(l, t)];
+          if (v0 != 0.f) c = fmaf(v0, f0, c);
+          if (v1 != 0.f) c = fmaf(v1, f1, c);
+          cs[crank(l, t)] = c;
+        }
+      }
     }
     __syncwarp();
   };
-  RowBuf<FMT> b0, b1;
-  if (nr > 0) load_row(0, b0);
-  for (int i = 0; i < nr; i += 2) {
-    if (i + 1 < nr) load_row(i + 1, b1);
-    process_row(i, b0);
-    if (i + 1 < nr) {
-      if (i + 2 < nr) load_row(i + 2, b0);
-      process_row(i + 1, b1);
+  for (int k = 0; k < ns; k += 2) {
+    if (k + 1 < ns) load_strip(k + 1, b1);
+    process(k, b0);
+    if (k + 1 < ns) {
+      if (k + 2 < ns) load_strip(k + 2, b0);
+      process(k + 1, b1);
     }
   }
   if (lane < nr) a.ybar[gd.r0 + lane] = yb_l;
-  if (!wide) {
-    for (int j = lane; j < gd.nd; j += 32) a.partial[gd.tb + j] = cs[sw_rank(j)];
-    __syncwarp();
-  }
+  for (int j = lane; j < gd.nd; j += 32) a.partial[gd.tb + j] = cs[j];
+  __syncwarp();
 }
 
+// Entry k of a wide row.
+template <int FMT>
+__device__ __forceinline__ float evalue(const GroupIterArgs& a, int64_t k) {
+  if constexpr (FMT == 0) return static_cast<const StripF*>(a.val)[k].v[0];
+  else return gq_from<FMT>(static_cast<const StripH*>(a.val)[k].v[0]);
+}
 
+// A wide group (one row, its own columns as its table, in the entries' order).
+template <int FMT>
+__device__ __forceinline__ void wide_pass(const GroupIterArgs& a, const GroupDesc& gd, int lane) {
+  const StripDesc q = a.strips[gd.qb];
+  float s = 0.f;
+  for (int i = lane; i < q.n; i += 32)
+    s = fmaf(evalue<FMT>(a, q.start + i), __ldg(a.x + a.table[gd.tb + i]), s);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s = fadd(s, __shfl_xor_sync(0xffffffffu, s, o));
+  const float sc = FMT == 0 ? 1.f : a.scale[gd.r0];
+  const float yb = FMT == 0 ? s : fmul(s, sc);
+  const float er = yb > 0.f ? __fdiv_rn(a.y[gd.r0], yb) : 0.f;
+  const float f = FMT == 0 ? er : fmul(er, sc);
+  if (lane == 0) a.ybar[gd.r0] = yb;
+  for (int i = lane; i < q.n; i += 32)
+    a.partial[gd.tb + i] = fmul(evalue<FMT>(a, q.start + i), f);
+}
 
 // A warp per group, a persistent grid striding over the groups; each warp
-// holds its group's tables (x and the correction at the distinct columns)
-// in its share of the block's shared memory.  The next group's head is
-// loaded one group ahead, descriptors two ahead.
-template <int FMT>
-__global__ void __launch_bounds__(kGroupWarps * 32, 1)
+// holds its group's tables (x and the correction at the distinct columns) in
+// its share of the block's shared memory.  The next group's head is loaded one group ahead, descriptors two ahead.
+template <int FMT, int ROUNDS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 k_group_mlem(GroupIterArgs a) {
   extern __shared__ __align__(16) float gsm[];
+  constexpr int kStride = pass_stride(WARPS);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* xs = gsm + (size_t)w * 2 * kGroupStride;
-  float* cs = xs + kGroupStride;
-  const int64_t step = (int64_t)gridDim.x * kGroupWarps;
-  int64_t g = (int64_t)blockIdx.x * kGroupWarps + w;
+  float* xs = gsm + (size_t)w * 2 * kStride;
+  float* cs = xs + kStride;
+  const int64_t step = (int64_t)gridDim.x * WARPS;
+  int64_t g = (int64_t)blockIdx.x * WARPS + w;
   if (g >= a.ngroups) return;
   GroupHead cur = group_head<FMT>(a, a.groups[g], lane);
-  GroupDesc nxt = g + step < a.ngroups ? a.groups[g + step] : GroupDesc{0, 0, 0, 0};
+  GroupDesc nxt = g + step < a.ngroups ? a.groups[g + step] : GroupDesc{0, 0, 0, 0, 0};
   for (; g < a.ngroups; g += step) {
     const GroupDesc nn =
-        g + 2 * step < a.ngroups ? a.groups[g + 2 * step] : GroupDesc{0, 0, 0, 0};
+        g + 2 * step < a.ngroups ? a.groups[g + 2 * step] : GroupDesc{0, 0, 0, 0, 0};
     GroupHead head_next{};
     if (g + step < a.ngroups) head_next = group_head<FMT>(a, nxt, lane);
     // (wide groups: k_group_mlem_wide)
-    if (cur.gd.nd <= kGroupCap) group_pass_as<FMT, kOrdinary>(a, cur, xs, cs, lane);
+    if (cur.gd.nd <= kGroupCap) group_pass<FMT, ROUNDS>(a, cur, xs, cs, lane);
     cur = head_next;
     nxt = nn;
   }
@@ -580,21 +856,22 @@ k_group_mlem_wide(GroupIterArgs a, const int32_t* __restrict__ wide, int64_t nwi
   const int lane = threadIdx.x & 31;
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (i >= nwide) return;
-  const GroupHead h = group_head<FMT>(a, a.groups[wide[i]], lane);
-  group_pass_as<FMT, kWide>(a, h, nullptr, nullptr, lane);
+  wide_pass<FMT>(a, a.groups[wide[i]], lane);
 }
 
 // The same over the groups of many reconstructions (batched form): global
 // group g belongs to problem p with gstart[p] <= g < gstart[p + 1].
-__global__ void __launch_bounds__(kGroupWarps * 32, 1)
+template <int ROUNDS, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 k_group_mlem_batch(const GroupIterArgs* __restrict__ desc, const int64_t* __restrict__ gstart,
                    int np) {
   extern __shared__ __align__(16) float gsm[];
+  constexpr int kStride = pass_stride(WARPS);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* xs = gsm + (size_t)w * 2 * kGroupStride;
-  float* cs = xs + kGroupStride;
+  float* xs = gsm + (size_t)w * 2 * kStride;
+  float* cs = xs + kStride;
   const int64_t total = gstart[np];
-  const int64_t step = (int64_t)gridDim.x * kGroupWarps;
+  const int64_t step = (int64_t)gridDim.x * WARPS;
   auto locate = [&](int64_t g) {  // gstart[lo] <= g < gstart[lo + 1]
     int lo = 0, hi = np;
     while (hi - lo > 1) {
@@ -604,13 +881,11 @@ k_group_mlem_batch(const GroupIterArgs* __restrict__ desc, const int64_t* __rest
     }
     return lo;
   };
-  int64_t g = (int64_t)blockIdx.x * kGroupWarps + w;
+  int64_t g = (int64_t)blockIdx.x * WARPS + w;
   if (g >= total) return;
-  // the problem's descriptor held by value; the next group's problem and
-  // head loaded one group ahead
+  // the next group's problem and head loaded one group ahead
   int p = locate(g);
-  GroupIterArgs a = desc[p];
-  GroupHead cur = group_head<0>(a, a.groups[g - gstart[p]], lane);
+  GroupHead cur = group_head<0>(desc[p], desc[p].groups[g - gstart[p]], lane);
   for (; g < total; g += step) {
     int pn = p;
     GroupHead hn{};
@@ -620,11 +895,8 @@ k_group_mlem_batch(const GroupIterArgs* __restrict__ desc, const int64_t* __rest
       hn = group_head<0>(an, an.groups[g + step - gstart[pn]], lane);
     }
     // (wide groups: k_group_mlem_batch_wide)
-    if (cur.gd.nd <= kGroupCap) group_pass_as<0, kOrdinary>(a, cur, xs, cs, lane);
-    if (pn != p) {
-      p = pn;
-      a = desc[p];
-    }
+    if (cur.gd.nd <= kGroupCap) group_pass<0, ROUNDS>(desc[p], cur, xs, cs, lane);
+    p = pn;
     cur = hn;
   }
 }
@@ -644,42 +916,58 @@ k_group_mlem_batch_wide(const GroupIterArgs* __restrict__ desc, const int64_t* _
     else hi = mid;
   }
   const GroupIterArgs a = desc[lo];
-  const GroupHead h = group_head<0>(a, a.groups[g - gstart[lo]], lane);
-  group_pass_as<0, kWide>(a, h, nullptr, nullptr, lane);
+  wide_pass<0>(a, a.groups[g - gstart[lo]], lane);
 }
 
 // Column sums of the grouped matrix's values (the 16-bit forms dequantised)
 // over its rows, by the same group / slot structure as the pass: a warp per
-// group adds its rows' values, row after row, into the group's shared sums
+// group adds its strips' values, in row order, into the group's shared sums
 // (the slots); the slot sums per column then run on the slot-sum kernel.
 template <int FMT>
-__global__ void __launch_bounds__(kGroupWarps * 32, 1)
+__global__ void __launch_bounds__(kColsumWarps * 32)
 k_group_colsum(GroupIterArgs a) {
   extern __shared__ __align__(16) float gsm[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* cs = gsm + (size_t)w * 2 * kGroupStride;
-  for (int64_t g = (int64_t)blockIdx.x * kGroupWarps + w; g < a.ngroups;
-       g += (int64_t)gridDim.x * kGroupWarps) {
+  float* cs = gsm + (size_t)w * kMaxStride;
+  for (int64_t g = (int64_t)blockIdx.x * kColsumWarps + w; g < a.ngroups;
+       g += (int64_t)gridDim.x * kColsumWarps) {
     const GroupDesc gd = a.groups[g];
     const bool wide = gd.nd > kGroupCap;
     if (!wide) {
-      for (int j = lane; j < gd.nd; j += 32) cs[sw_rank(j)] = 0.f;
+      for (int j = lane; j < gd.nd; j += 32) cs[j] = 0.f;
       __syncwarp();
     }
-    for (int r = gd.r0; r < gd.r1; r++) {
-      const int64_t b = a.row_ptr[r], e = a.row_ptr[r + 1];
-      const float sc = FMT == 0 ? 1.f : a.scale[r];
-      for (int64_t k = b + lane; k < e; k += 32) {
-        float v;
-        if constexpr (FMT == 0) v = static_cast<const float*>(a.val)[k];
-        else v = fmul(gq_from<FMT>(static_cast<const uint16_t*>(a.val)[k]), sc);
-        if (wide) a.partial[gd.tb + (k - b)] = v;
-        else cs[a.loc[k]] = fadd(cs[a.loc[k]], v);  // padding: the trash slot
+    for (int r = gd.r0, q = gd.qb; r < gd.r1; r += kStrip, q++) {
+      const StripDesc d = a.strips[q];
+      float sc[kStrip];
+#pragma unroll
+      for (int j = 0; j < kStrip; j++) sc[j] = FMT != 0 && r + j < gd.r1 ? a.scale[r + j] : 1.f;
+      auto with = [&](float c, const float* v) {
+#pragma unroll
+        for (int j = 0; j < kStrip; j++) c = fadd(c, FMT == 0 ? v[j] : fmul(v[j], sc[j]));
+        return c;
+      };
+      if (wide) {
+        for (int i = lane; i < d.n; i += 32) {
+          const float v[kStrip] = {evalue<FMT>(a, d.start + i), 0.f};
+          a.partial[gd.tb + i] = with(0.f, v);
+        }
+      } else {
+        const int nq = strip_pad(d.n) / 4;
+        for (int u = 0; 32 * u + lane < nq; u++) {
+          ChunkV<FMT> vv;
+          uint2 l;
+          gload<FMT>(a.val, a.loc, d.start, nq, u, lane, &vv, &l);
+          for (int t = 0; t < 4; t++) {  // (padding: the trash slot)
+            const float v[kStrip] = {cvalue<FMT>(vv, t, 0), cvalue<FMT>(vv, t, 1)};
+            cs[crank(l, t)] = with(cs[crank(l, t)], v);
+          }
+        }
       }
       __syncwarp();
     }
     if (!wide) {
-      for (int j = lane; j < gd.nd; j += 32) a.partial[gd.tb + j] = cs[sw_rank(j)];
+      for (int j = lane; j < gd.nd; j += 32) a.partial[gd.tb + j] = cs[j];
       __syncwarp();
     }
   }
@@ -690,7 +978,7 @@ k_group_colsum(GroupIterArgs a) {
 static int bitmap_words(int64_t V) { return (int)((V + 31) / 32); }
 
 bool grouped_supported(int64_t V, int64_t m) {
-  // two V-bit maps in a table block's shared memory; int32 rows
+  // a V-bit map and its prefix in a table block's shared memory; int32 rows
   return V > 0 && (size_t)bitmap_words(V) * 8 <= (size_t)200 * 1024 && m < INT32_MAX;
 }
 
@@ -698,7 +986,7 @@ void grouped_free(GroupedMatrix* G, cudaStream_t st) {
   for (void* p : {(void*)G->groups, (void*)G->table, (void*)G->loc, (void*)G->wide,
                   (void*)G->cg_ptr,
                   (void*)G->cg_slot, (void*)G->ones, (void*)G->partial, (void*)G->val16,
-                  (void*)G->val32, (void*)G->row_ptr, (void*)G->scale})
+                  (void*)G->val32, (void*)G->strips, (void*)G->scale})
     if (p) dev_free(p, st);
   *G = GroupedMatrix{};
 }
@@ -710,24 +998,15 @@ void grouped_drop_fp32(GroupedMatrix* G, cudaStream_t st) {
   }
 }
 
-// Where the first round of form_groups lays out the first cuts that fit
-// (k_group_tables' first launch): the padded row pointers, the scratch
-// tables (kGroupCap per first cut) and the padded values and ranks.
-struct FirstCuts {
-  const int64_t* ptr;
-  int32_t* ftab;
-  float* pval;
-  uint16_t* ploc;
-};
-
 // Groups of consecutive rows of A (row pointers on the device) whose
 // distinct columns fit kGroupCap: first cuts of kGroupFirstRows rows, halved
 // while too wide; a single row wider than that is a group of its own, its
-// table the row's columns padded to whole 4-entry chunks.  The first round
-// measures the first cuts and lays out those that fit (FirstCuts); the
-// halves are measured by k_group_distinct.
-static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, const FirstCuts& fc,
-                               std::vector<GroupDesc>* out, cudaStream_t st) {
+// table the row's columns.  The first round measures the first cuts and lays
+// out those that fit (k_group_tables' first launch: tables in ftab, strips in
+// fstrips, entries in out); the halves are measured by k_group_distinct.
+static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, int32_t* ftab,
+                               const EntryOut& entries, std::vector<GroupDesc>* out,
+                               cudaStream_t st) {
   const int nwords = bitmap_words(ncols);
   const int64_t ncut = (m + kGroupFirstRows - 1) / kGroupFirstRows;
   EPET_CUDA(cudaFuncSetAttribute(k_group_distinct, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -739,7 +1018,7 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, con
     cudaError_t e = dev_alloc((void**)&nd, std::max<int64_t>(ncut, 1) * 4, st);
     if (e == cudaSuccess && ncut > 0) {
       k_group_tables<<<(unsigned)ncut, kGroupThreads, table_smem(nwords), st>>>(
-          A, nullptr, m, nwords, fc.ptr, fc.ftab, nullptr, nd, fc.pval, fc.ploc);
+          A, nullptr, m, nwords, 1, ftab, nullptr, nullptr, nd, entries);
       note_launch();
       e = cudaGetLastError();
       if (e == cudaSuccess)
@@ -752,9 +1031,9 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, con
   // The wider cuts, halved until their pieces fit or are one row; only
   // those pieces are counted again.  A split cut s keeps its pieces as bits
   // of mask[s] (a piece starting at row j of the cut) and their counts at
-  // sub[32 s + j].
+  // sub[kGroupFirstRows s + j].
   std::vector<int32_t> slot(ncut, -1);
-  std::vector<uint32_t> mask;
+  std::vector<uint64_t> mask;
   std::vector<int32_t> sub;
   std::vector<int2> pend, nextp;
   for (int64_t c = 0; c < ncut; c++) {
@@ -762,7 +1041,7 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, con
     const int32_t r1 = (int32_t)std::min<int64_t>(m, r0 + kGroupFirstRows);
     if (cut_nd[c] > kGroupCap && r1 - r0 > 1) {
       slot[c] = (int32_t)mask.size();
-      mask.push_back(0u);
+      mask.push_back(0);
       const int32_t mid = r0 + (r1 - r0) / 2;
       pend.push_back(make_int2(r0, mid));
       pend.push_back(make_int2(mid, r1));
@@ -799,7 +1078,7 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, con
         nextp.push_back(make_int2(mid, p.y));
       } else {
         const int32_t s = slot[p.x / kGroupFirstRows], j = p.x % kGroupFirstRows;
-        mask[s] |= 1u << j;
+        mask[s] |= uint64_t(1) << j;
         sub[(size_t)s * kGroupFirstRows + j] = hn[k];
       }
     }
@@ -808,38 +1087,103 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, con
   // the groups in row order: the cuts kept whole, and a split cut's pieces
   out->clear();
   out->reserve(ncut + sub.size() / 8);
-  int64_t tb = 0;
+  int64_t tb = 0, qb = 0;
   for (int64_t c = 0; c < ncut; c++) {
     const int32_t r0 = (int32_t)(c * kGroupFirstRows);
     const int32_t r1 = (int32_t)std::min<int64_t>(m, r0 + kGroupFirstRows);
-    uint32_t msk = slot[c] < 0 ? 1u : mask[slot[c]];
+    uint64_t msk = slot[c] < 0 ? 1u : mask[slot[c]];
     if (!(msk & 1u)) return set_error(EPET_ERR_INVALID, "internal: row groups unmeasured");
     while (msk) {
-      const int j = __builtin_ctz(msk);
+      const int j = __builtin_ctzll(msk);
       msk &= msk - 1u;
-      const int32_t e = msk ? r0 + __builtin_ctz(msk) : r1;
+      const int32_t e = msk ? r0 + __builtin_ctzll(msk) : r1;
       const int32_t ndv = slot[c] < 0 ? cut_nd[c] : sub[(size_t)slot[c] * kGroupFirstRows + j];
-      const int32_t n = ndv > kGroupCap ? (ndv + 3) & ~3 : ndv;  // wide: padded like its row
-      if (tb + n > INT32_MAX)
+      const int32_t nq = (e - (r0 + j) + kStrip - 1) / kStrip;
+      if (tb + ndv > INT32_MAX || qb + nq > INT32_MAX)
         return set_error(EPET_ERR_UNSUPPORTED, "row-group tables exceed int32");
-      out->push_back(GroupDesc{r0 + j, e, (int32_t)tb, n});
-      tb += n;
+      out->push_back(GroupDesc{r0 + j, e, (int32_t)tb, ndv, (int32_t)qb});
+      tb += ndv;
+      qb += nq;
     }
   }
   return EPET_OK;
 }
 
+// Launch shape of the pass: chunks per lane in registers (two sets of 10
+// registers each) and warps of a block (one per SM), by the mean entries of a
+// strip and the widest group.  Long strips want them whole in registers (what
+// is beyond is loaded twice, on the warp's path), short ones more warps.
+// Measured: 52^3 voxels, 100 rays (510 entries a strip; 20 iterations of 5.1M
+// rows): 5 chunks and 12 warps 73.2 ms, 4 and 12 80.4, 4 and 16 84.0, 6 and 12
+// (spilling) 94; 24^3 and 32^3, 20 to 100 rays (16 problems, 10 iterations):
+// 5 and 12 20.1 ms, 4 and 12 17.5, by this rule 16.5; 24^3, 20 rays (one
+// iteration): 5 and 12 67 us, 2 and 20 55.
+struct PassShape {
+  int rounds, warps;
+  size_t smem() const { return (size_t)warps * 2 * pass_stride(warps) * 4; }
+};
+static PassShape pass_shape(int64_t entries, int64_t strips, int max_nd) {
+  const double mean = strips > 0 ? (double)entries / strips : 0.0;
+  // (the tables hold the group's columns and the padding's rank)
+  if (mean <= 220 && max_nd < pass_stride(20)) return PassShape{2, 20};
+  if (mean <= 340 && max_nd < pass_stride(16)) return PassShape{3, 16};
+  return PassShape{5, 12};
+}
+static_assert(pass_stride(12) > kGroupCap, "the largest groups");
+static_assert(12 * 8 * (size_t)pass_stride(12) <= kMaxPassSmem, "shared tables");
+static_assert(16 * 8 * (size_t)pass_stride(16) <= kMaxPassSmem, "shared tables");
+static_assert(20 * 8 * (size_t)pass_stride(20) <= kMaxPassSmem, "shared tables");
+
+// f(integral_constant<ROUNDS>, integral_constant<WARPS>) for the shape.
+template <class F>
+static void dispatch_shape(const PassShape& s, F&& f) {
+  using std::integral_constant;
+  if (s.rounds == 2) f(integral_constant<int, 2>{}, integral_constant<int, 20>{});
+  else if (s.rounds == 3) f(integral_constant<int, 3>{}, integral_constant<int, 16>{});
+  else f(integral_constant<int, 5>{}, integral_constant<int, 12>{});
+}
+
+// Shared memory of every instantiation (set when a layout is built: the
+// launches may be captured in a graph).
+static cudaError_t allow_pass_smem() {
+  cudaError_t e = cudaSuccess;
+  auto allow = [&](const void* k, size_t bytes) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  for (int r : {2, 3, 5})
+    dispatch_shape(PassShape{r, 0}, [&](auto R, auto W) {
+      constexpr int rounds = decltype(R)::value, warps = decltype(W)::value;
+      allow((const void*)k_group_mlem<0, rounds, warps>, kMaxPassSmem);
+      allow((const void*)k_group_mlem<1, rounds, warps>, kMaxPassSmem);
+      allow((const void*)k_group_mlem<2, rounds, warps>, kMaxPassSmem);
+      allow((const void*)k_group_mlem_batch<rounds, warps>, kMaxPassSmem);
+    });
+  allow((const void*)k_group_colsum<0>, kColsumSmem);
+  allow((const void*)k_group_colsum<1>, kColsumSmem);
+  allow((const void*)k_group_colsum<2>, kColsumSmem);
+  return e;
+}
+
 epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t nnz,
                           int value_format, GroupedMatrix* G, cudaStream_t st) {
-  (void)nnz;
   *G = GroupedMatrix{};
   G->fmt = value_format;
   G->n = ncols;
   if (!grouped_supported(ncols, m))
     return set_error(EPET_ERR_UNSUPPORTED, "grouped layout: %lld columns", (long long)ncols);
-  int32_t* ftab = nullptr;  // first cuts' tables (scratch)
+  int32_t* ftab = nullptr;              // first cuts' tables (scratch)
+  StripDesc* fstrips = nullptr;         // first cuts' strips (scratch)
+  unsigned long long* cursor = nullptr; // entries reserved
+  auto drop_scratch = [&]() {
+    for (void* p : {(void*)ftab, (void*)fstrips, (void*)cursor})
+      if (p) dev_free(p, st);
+    ftab = nullptr;
+    fstrips = nullptr;
+    cursor = nullptr;
+  };
   auto fail = [&](epet_status rc) {
-    if (ftab) dev_free(ftab, st);
+    drop_scratch();
     grouped_free(G, st);
     return rc;
   };
@@ -853,58 +1197,92 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
                                        (int)table_smem(nwords));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_group_tables, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  for (const void* k : {(const void*)k_group_mlem<0>, (const void*)k_group_mlem<1>,
-                        (const void*)k_group_mlem<2>, (const void*)k_group_mlem_batch,
-                        (const void*)k_group_colsum<0>, (const void*)k_group_colsum<1>,
-                        (const void*)k_group_colsum<2>})
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGroupSmem);
+  if (e == cudaSuccess) e = allow_pass_smem();
   if (e != cudaSuccess) return fail(cuda_status(e, "grouped kernels"));
-  // the padded row pointers (rows padded to whole 4-entry chunks)
-  GALLOC(G->row_ptr, (m + 1) * 8);
-  {
-    int64_t *len = nullptr, *tmp = nullptr;
-    GALLOC(len, std::max<int64_t>(m, 1) * 8);
-    GALLOC(tmp, scan_tmp_elems(m) * 8);
-    epet_status rc = EPET_OK;
-    if (m > 0) {
-      k_padded_len<<<ceil_div(m, 256), 256, 0, st>>>(A, m, len);
+  const int64_t ncut = ceil_div(std::max<int64_t>(m, 1), (int64_t)kGroupFirstRows);
+  GALLOC(cursor, 8);
+  GALLOC(ftab, ncut * kGroupCap * 4);
+  GALLOC(fstrips, ncut * kGroupStrips * sizeof(StripDesc));
+  auto read_cursor = [&](int64_t* n) -> epet_status {
+    unsigned long long v = 0;
+    EPET_CUDA(cudaMemcpyAsync(&v, cursor, 8, cudaMemcpyDeviceToHost, st));
+    EPET_CUDA(cudaStreamSynchronize(st));
+    *n = (int64_t)v;
+    return EPET_OK;
+  };
+  // The entries' arrays: how far the rows of a strip share columns is only
+  // known once they are merged (0.6 entries per non-zero in scans).  Up to
+  // 2^26 non-zeros the arrays are sized as if none were shared (0.7 GB at
+  // most, and a small reconstruction saves a launch and a round trip: 0.1 of
+  // 4.1 ms); beyond, a sample of the first cuts sizes them, and should the
+  // entries not fit after all, the layout is made again at the size it asked
+  // for.
+  int64_t cap = nnz + 3 * std::max<int64_t>(m, 1);
+  if (m > 0 && nnz > (int64_t(1) << 26)) {
+    const int64_t every = std::max<int64_t>(1, ncut / kSampleCuts);
+    const int64_t sampled = (ncut + every - 1) / every;
+    e = cudaMemsetAsync(cursor, 0, 8, st);
+    if (e == cudaSuccess) {
+      k_group_tables<<<(unsigned)sampled, kGroupThreads, table_smem(nwords), st>>>(
+          A, nullptr, m, nwords, every, nullptr, nullptr, nullptr, nullptr,
+          EntryOut{cursor, 0, nullptr, nullptr, nullptr});
       note_launch();
-      rc = exclusive_scan_i64(len, G->row_ptr, m, tmp, st);
-    } else {
-      cudaMemsetAsync(G->row_ptr, 0, 8, st);
+      e = cudaGetLastError();
     }
-    if (rc == EPET_OK) {
-      e = cudaMemcpyAsync(&G->npad, G->row_ptr + m, 8, cudaMemcpyDeviceToHost, st);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-      if (e != cudaSuccess) rc = cuda_status(e, "padded layout");
-    }
-    dev_free(len, st);
-    dev_free(tmp, st);
+    int64_t n = 0;
+    const epet_status rc = e == cudaSuccess ? read_cursor(&n) : cuda_status(e, "group sample");
     if (rc != EPET_OK) return fail(rc);
+    cap = (int64_t)((double)n / sampled * ncut * 1.03) + 65536;
   }
-  GALLOC(G->val32, std::max<int64_t>(G->npad, 4) * 4);
-  GALLOC(G->loc, std::max<int64_t>(G->npad, 4) * 2);
-  // the groups; the first cuts that fit are laid out on the way
-  GALLOC(ftab, ceil_div(std::max<int64_t>(m, 1), (int64_t)kGroupFirstRows) * kGroupCap * 4);
   std::vector<GroupDesc> hg;
-  {
-    const epet_status rc = form_groups(A, m, ncols, FirstCuts{G->row_ptr, ftab, G->val32, G->loc},
-                                       &hg, st);
+  for (int attempt = 0;; attempt++) {
+    GALLOC(G->val32, cap * sizeof(StripF));
+    GALLOC(G->loc, cap * 2);
+    e = cudaMemsetAsync(cursor, 0, 8, st);
+    if (e != cudaSuccess) return fail(cuda_status(e, "group entries"));
+    // the groups; the first cuts that fit are laid out on the way
+    epet_status rc = form_groups(A, m, ncols, ftab, EntryOut{cursor, cap, G->val32, G->loc, fstrips},
+                                 &hg, st);
     if (rc != EPET_OK) return fail(rc);
+    G->ngroups = (int64_t)hg.size();
+    G->nslots = hg.empty() ? 0 : (int64_t)hg.back().tb + hg.back().nd;
+    G->nstrips =
+        hg.empty() ? 0 : (int64_t)hg.back().qb + (hg.back().r1 - hg.back().r0 + kStrip - 1) / kStrip;
+    if (attempt == 0) {  // (the groups do not depend on the entries' place)
+      GALLOC(G->groups, hg.size() * sizeof(GroupDesc));
+      GALLOC(G->strips, std::max<int64_t>(G->nstrips, 1) * sizeof(StripDesc));
+      GALLOC(G->table, std::max<int64_t>(G->nslots, 1) * 4);
+    }
+    // the tables and strips at their places and the layout of the groups
+    // split from wider cuts
+    if (!hg.empty()) {
+      e = cudaMemcpyAsync(G->groups, hg.data(), hg.size() * sizeof(GroupDesc),
+                          cudaMemcpyHostToDevice, st);
+      if (e == cudaSuccess) {
+        k_group_tables<<<(unsigned)hg.size(), kGroupThreads, table_smem(nwords), st>>>(
+            A, G->groups, m, nwords, 1, G->table, ftab, fstrips, nullptr,
+            EntryOut{cursor, cap, G->val32, G->loc, G->strips});
+        note_launch();
+        e = cudaGetLastError();
+      }
+      if (e != cudaSuccess) return fail(cuda_status(e, "group tables"));
+    }
+    rc = read_cursor(&G->nent);
+    if (rc != EPET_OK) return fail(rc);
+    if (G->nent <= cap) break;
+    if (attempt > 0) return fail(set_error(EPET_ERR_INVALID, "internal: group entries"));
+    dev_free(G->val32, st);
+    dev_free(G->loc, st);
+    G->val32 = nullptr;
+    G->loc = nullptr;
+    cap = G->nent;
   }
-  G->ngroups = (int64_t)hg.size();
-  G->nslots = hg.empty() ? 0 : (int64_t)hg.back().tb + hg.back().nd;
+  drop_scratch();
+  for (const GroupDesc& g : hg)
+    if (g.nd <= kGroupCap) G->max_nd = std::max(G->max_nd, g.nd);
   const int64_t ns = std::max<int64_t>(G->nslots, 1);
-  GALLOC(G->groups, hg.size() * sizeof(GroupDesc));
-  GALLOC(G->table, ns * 4);
   GALLOC(G->partial, ns * 4);
   GALLOC(G->cg_ptr, (ncols + 1) * 8);
-  if (!hg.empty()) {
-    e = cudaMemcpyAsync(G->groups, hg.data(), hg.size() * sizeof(GroupDesc),
-                        cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return fail(cuda_status(e, "group table"));
-  }
   {
     std::vector<int32_t> wide;
     for (size_t i = 0; i < hg.size(); i++)
@@ -918,18 +1296,8 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
       if (e != cudaSuccess) return fail(cuda_status(e, "wide groups"));
     }
   }
-  // the tables at their slots and the layout of the groups split from wider cuts
-  if (!hg.empty()) {
-    k_group_tables<<<(unsigned)hg.size(), kGroupThreads, table_smem(nwords), st>>>(
-        A, G->groups, m, nwords, G->row_ptr, G->table, ftab, nullptr, G->val32, G->loc);
-    note_launch();
-    if (cudaGetLastError() != cudaSuccess) return fail(set_error(EPET_ERR_CUDA, "group tables"));
-  }
-  dev_free(ftab, st);
-  ftab = nullptr;
   // the slots of each column in group order: the column-major order of the
-  // (group x column) table's entries, i.e. their positions (a wide group's
-  // padding slots sit in column 0 and hold zero corrections)
+  // (group x column) table's entries, i.e. their positions
   GALLOC(G->cg_slot, ns * 4);
   {
     const epet_status rc = csr_to_csc_positions(G->nslots, ncols, G->table, G->cg_ptr,
@@ -937,15 +1305,16 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     if (rc != EPET_OK) return fail(rc);
   }
   if (value_format != EPET_VALUES_FP32) {
-    GALLOC(G->val16, std::max<int64_t>(G->npad, 4) * 2);
+    GALLOC(G->val16, std::max<int64_t>(G->nent, 1) * sizeof(StripH));
     GALLOC(G->scale, std::max<int64_t>(m, 1) * 4);
     if (m > 0) {
+      const unsigned nb = (unsigned)ceil_div(G->nstrips * 32, 256);
       if (value_format == EPET_VALUES_BF16)
-        k_group_quantise<1><<<ceil_div(m * 32, 256), 256, 0, st>>>(G->row_ptr, G->val32, m,
-                                                                     G->scale, G->val16);
+        k_group_quantise<1><<<nb, 256, 0, st>>>(G->strips, G->nstrips, G->val32, m, G->scale,
+                                                G->val16);
       else
-        k_group_quantise<2><<<ceil_div(m * 32, 256), 256, 0, st>>>(G->row_ptr, G->val32, m,
-                                                                     G->scale, G->val16);
+        k_group_quantise<2><<<nb, 256, 0, st>>>(G->strips, G->nstrips, G->val32, m, G->scale,
+                                                G->val16);
       note_launch();
       if (cudaGetLastError() != cudaSuccess) return fail(set_error(EPET_ERR_CUDA, "quantise"));
     }
@@ -957,7 +1326,7 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
 
 static GroupIterArgs iter_args(const GroupedMatrix& G, const float* x, const float* y,
                                float* ybar) {
-  return GroupIterArgs{G.groups, G.ngroups, G.row_ptr,
+  return GroupIterArgs{G.groups, G.ngroups, G.strips,
                        G.fmt == EPET_VALUES_FP32 ? (const void*)G.val32 : (const void*)G.val16,
                        G.scale, G.loc, G.table, x, y, ybar, G.partial};
 }
@@ -969,17 +1338,21 @@ void grouped_batch_desc(const GroupedMatrix& G, const float* x, const float* y, 
   *static_cast<GroupIterArgs*>(out) = iter_args(G, x, y, ybar);
 }
 
-static unsigned pass_grid(int64_t ngroups) {
+static unsigned pass_grid(int64_t ngroups, int warps) {
   return (unsigned)std::max<int64_t>(
-      1, std::min<int64_t>((ngroups + kGroupWarps - 1) / kGroupWarps, (int64_t)num_sms()));
+      1, std::min<int64_t>((ngroups + warps - 1) / warps, (int64_t)num_sms()));
 }
 
 epet_status grouped_pass_batch(const void* desc, const int64_t* gstart, int np,
-                               int64_t total_groups, const int32_t* wide, int64_t nwide,
+                               const BatchGroups& total, const int32_t* wide, int64_t nwide,
                                cudaStream_t st) {
-  if (total_groups <= 0) return EPET_OK;
-  k_group_mlem_batch<<<pass_grid(total_groups), kGroupWarps * 32, kGroupSmem, st>>>(
-      static_cast<const GroupIterArgs*>(desc), gstart, np);
+  if (total.groups <= 0) return EPET_OK;
+  const PassShape s = pass_shape(total.entries, total.strips, total.max_nd);
+  dispatch_shape(s, [&](auto R, auto W) {
+    k_group_mlem_batch<decltype(R)::value, decltype(W)::value>
+        <<<pass_grid(total.groups, s.warps), s.warps * 32, s.smem(), st>>>(
+            static_cast<const GroupIterArgs*>(desc), gstart, np);
+  });
   EPET_LAUNCHED();
   if (nwide > 0) {
     k_group_mlem_batch_wide<<<(unsigned)ceil_div(nwide * 32, (int64_t)128), 128, 0, st>>>(
@@ -999,11 +1372,11 @@ epet_status grouped_column_sums(const GroupedMatrix& G, bool quantised, float* o
       a.val = G.val32;
       fmt = EPET_VALUES_FP32;
     }
-    const unsigned grid = pass_grid(G.ngroups);
+    const unsigned grid = 3 * pass_grid(G.ngroups, kColsumWarps), T = kColsumWarps * 32;
     switch (fmt) {
-      case EPET_VALUES_BF16: k_group_colsum<1><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a); break;
-      case EPET_VALUES_FP16: k_group_colsum<2><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a); break;
-      default: k_group_colsum<0><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a);
+      case EPET_VALUES_BF16: k_group_colsum<1><<<grid, T, kColsumSmem, st>>>(a); break;
+      case EPET_VALUES_FP16: k_group_colsum<2><<<grid, T, kColsumSmem, st>>>(a); break;
+      default: k_group_colsum<0><<<grid, T, kColsumSmem, st>>>(a);
     }
     EPET_LAUNCHED();
   }
@@ -1019,14 +1392,20 @@ epet_status grouped_pass(const GroupedMatrix& G, const float* x, const float* y,
                          cudaStream_t st) {
   if (G.ngroups == 0) return EPET_OK;
   const GroupIterArgs a = iter_args(G, x, y, ybar);
-  const unsigned grid = pass_grid(G.ngroups);
-  // (the shared-memory size was allowed when the layout was built: this
-  // launch may be captured in a graph)
-  switch (G.fmt) {
-    case EPET_VALUES_BF16: k_group_mlem<1><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a); break;
-    case EPET_VALUES_FP16: k_group_mlem<2><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a); break;
-    default: k_group_mlem<0><<<grid, kGroupWarps * 32, kGroupSmem, st>>>(a);
-  }
+  const PassShape s = pass_shape(G.nent, G.nstrips, G.max_nd);
+  const unsigned grid = pass_grid(G.ngroups, s.warps), T = s.warps * 32;
+  dispatch_shape(s, [&](auto R, auto W) {
+    constexpr int rounds = decltype(R)::value, warps = decltype(W)::value;
+    switch (G.fmt) {
+      case EPET_VALUES_BF16:
+        k_group_mlem<1, rounds, warps><<<grid, T, s.smem(), st>>>(a);
+        break;
+      case EPET_VALUES_FP16:
+        k_group_mlem<2, rounds, warps><<<grid, T, s.smem(), st>>>(a);
+        break;
+      default: k_group_mlem<0, rounds, warps><<<grid, T, s.smem(), st>>>(a);
+    }
+  });
   EPET_LAUNCHED();
   if (G.nwide > 0) {
     const unsigned wgrid = (unsigned)ceil_div(G.nwide * 32, (int64_t)128);

@@ -701,15 +701,16 @@ epet_status epet_mlem_stats(const epet_mlem* h, int64_t* nnz_h, int64_t* bytes_h
   if (!h) return set_error(EPET_ERR_INVALID, "bad arguments");
   if (nnz_h) *nnz_h = h->A.nnz;
   if (bytes_h && h->grouped) {
-    // pass: values (4 or 2 bytes) and ranks (2) per entry, row pointers,
-    // y, ybar, row scales (16-bit), per slot the table, the x gather and
-    // the correction written; slot sums: column pointers, per slot the slot
-    // index, a one and the correction, x and s read, xnew written; image
-    // sum and normalisation: xnew read twice, x written
-    const int64_t np = h->G.npad, m = h->m, V = h->V, ns = h->G.nslots;  // (padded entries)
+    // pass: values (4 or 2 bytes per row of the strip) and ranks (2) per
+    // entry, strip descriptors, y, ybar, row scales (16-bit), per slot the
+    // table, the x gather and the correction written; slot sums: column
+    // pointers, per slot the slot index, a one and the correction, x and s
+    // read, xnew written; image sum and normalisation: xnew read twice, x
+    // written
+    const int64_t ne = h->G.nent, m = h->m, V = h->V, ns = h->G.nslots;
     const int64_t bv = h->G.fmt == EPET_VALUES_FP32 ? 4 : 2;
-    *bytes_h = (bv + 2) * np + 8 * (m + 1) + 8 * m + (bv == 2 ? 4 * m : 0) + 12 * ns +
-               8 * (V + 1) + 12 * ns + 8 * V + 4 * V + 8 * V + 4 * V;
+    *bytes_h = (kStrip * bv + 2) * ne + 16 * h->G.nstrips + 8 * m + (bv == 2 ? 4 * m : 0) +
+               12 * ns + 8 * (V + 1) + 12 * ns + 8 * V + 4 * V + 8 * V + 4 * V;
   } else if (bytes_h && h->opt.matrix_free) {
     // no matrix: the pass writes and reads the rays (24 bytes each) and the
     // channel geometry (224 bytes per row), reads y and writes ybar, reads x

@@ -8,22 +8,40 @@
 namespace epet {
 // Grouped layout of a reconstruction's matrix (grouped.cu): consecutive rows
 // in groups whose distinct columns fit a per-warp shared table.
-constexpr int kGroupCap = 1536;  // distinct columns of a group held in shared memory
-constexpr int kGroupWarps = 16;  // warps (groups in flight) per block of the iteration
+constexpr int kGroupCap = 2048;  // distinct columns of a group held in shared memory
 struct GroupDesc {
   int32_t r0, r1;  // rows [r0, r1)
   int32_t tb, nd;  // table slots [tb, tb + nd)
+  int32_t qb;      // first strip; ceil((r1 - r0) / kStrip) of them
+};
+// Rows merged per entry, and an entry's values: one per row of its strip (zero
+// where the row does not touch the entry's column).
+constexpr int kStrip = 2;
+struct alignas(4 * kStrip) StripF {
+  float v[kStrip];
+};
+struct alignas(2 * kStrip) StripH {
+  uint16_t v[kStrip];
+};
+// kStrip consecutive rows of a group (fewer at its end) merged: entries
+// [start, start + n), one per column that any of them touches.
+struct StripDesc {
+  int64_t start;
+  int32_t n;
+  int32_t r0;  // first row
 };
 struct GroupedMatrix {
   int fmt = 0;  // EPET_VALUES_*
   int64_t n = 0;                // columns (voxels)
-  int64_t ngroups = 0, nslots = 0, npad = 0;
+  int64_t ngroups = 0, nstrips = 0, nslots = 0, nent = 0;
+  int max_nd = 0;               // most columns of a group in shared memory
   GroupDesc* groups = nullptr;
+  StripDesc* strips = nullptr;
   int32_t* table = nullptr;     // each group's distinct columns, ascending
-  int64_t* row_ptr = nullptr;   // rows padded to whole 4-entry chunks
-  float* val32 = nullptr;       // values (FP32 form; 16-bit forms: until the sensitivity is fixed)
-  uint16_t* val16 = nullptr;    // 16-bit forms: values / row scale
-  float* scale = nullptr;
+  StripF* val32 = nullptr;      // per entry its rows' values (FP32 form; 16-bit forms: until the
+                                // sensitivity is fixed)
+  StripH* val16 = nullptr;      // 16-bit forms: values / row scale
+  float* scale = nullptr;       // per row
   uint16_t* loc = nullptr;      // per entry: rank of its column in its group's table
   int64_t* cg_ptr = nullptr;    // per column: its slots (group order) at cg_slot[cg_ptr[v] ..]
   int32_t* cg_slot = nullptr;
@@ -80,8 +98,14 @@ epet_status grouped_column_sums(const GroupedMatrix& G, bool quantised, float* o
 size_t grouped_batch_desc_bytes();
 void grouped_batch_desc(const GroupedMatrix& G, const float* x, const float* y, float* ybar,
                         void* out);
+// groups/strips/entries/columns: totals over the problems and the most columns
+// of any group (the launch shape's rule).
+struct BatchGroups {
+  int64_t groups = 0, strips = 0, entries = 0;
+  int max_nd = 0;
+};
 epet_status grouped_pass_batch(const void* desc, const int64_t* gstart, int np,
-                               int64_t total_groups, const int32_t* wide, int64_t nwide,
+                               const BatchGroups& total, const int32_t* wide, int64_t nwide,
                                cudaStream_t st);
 }  // namespace epet
 
