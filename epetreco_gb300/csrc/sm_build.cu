@@ -39,7 +39,11 @@
 
 namespace epet {
 
-constexpr int kWalkThreads = 128;
+// Threads of a walk CTA (one channel): half as many for few rays, where the
+// phases around the walk weigh most and a CTA's threads share little work
+// (walk_threads).
+constexpr int kWalkThreads = 128, kWalkThreadsFew = 64;
+constexpr int kFewRays = 80;     // rays of a channel up to which a CTA has kWalkThreadsFew threads
 constexpr int kGeomFloats = 56;  // per-channel geometry record (k_channel_geom)
 constexpr int kMaxSlabs = 1024;  // nx limit of the walk kernel
 constexpr float kWinPad = 1e-3f;  // window padding margin, in voxels (slab_window)
@@ -139,9 +143,10 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) {
   return v < lo ? lo : (v > hi ? hi : v);
 }
 
-// Block-wide exclusive scan of one int per thread (kWalkThreads threads) with
-// one barrier; warp_tot (kWalkThreads / 32 ints) is the call's own: it must
-// not be reused before another barrier.
+// Block-wide exclusive scan of one int per thread (kT threads) with one
+// barrier; warp_tot (kT / 32 ints) is the call's own: it must not be reused
+// before another barrier.
+template <int kT>
 __device__ __forceinline__ int block_excl_scan(int v, int* warp_tot, int* total) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int inc = warp_incl_scan(v);
@@ -149,7 +154,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int* warp_tot, int* total)
   __syncthreads();
   int before = 0, all = 0;
 #pragma unroll
-  for (int k = 0; k < kWalkThreads / 32; k++) {
+  for (int k = 0; k < kT / 32; k++) {
     const int t = warp_tot[k];
     before += k < w ? t : 0;
     all += t;
@@ -542,10 +547,15 @@ static epet_status launch_channel_geom(const Geo& G, const int32_t* rows, int64_
 // walk, lo and hi sums apart, the hull from 16 lines, the z runs of a column
 // from per-x and per-y slab runs, one barrier per scan.  Registers are held
 // to 64 for 8 CTAs per SM (9 with 56 registers: 11.4 ms, 10 with 48: 12.3).
-template <int kMode>
-__global__ void __launch_bounds__(kWalkThreads, 8)
+template <int kMode, int kT>
+__global__ void __launch_bounds__(kT, 1024 / kT)
 k_walk(WalkArgs args) {
   extern __shared__ __align__(16) unsigned char smem[];
+  // Ranges of the extraction: one per thread; a projection's sum is cut into
+  // kWalkThreads of them whatever the CTA (its order of additions, hence
+  // every bit of A x, does not depend on the launch shape).
+  constexpr int kRanges = kMode == kModeForward || kMode == kModeMlem ? kWalkThreads : kT;
+  constexpr int kMine = kRanges / kT;
   const Geo& G = args.G;
   const epet_grid& g = G.p.grid;
   const WalkLayout lay = walk_layout(g, args.cap_cells);
@@ -556,12 +566,12 @@ k_walk(WalkArgs args) {
   const float(*c0)[3] = reinterpret_cast<const float(*)[3]>(s_geom);
   const float(*c1)[3] = reinterpret_cast<const float(*)[3]>(s_geom + 24);
   const ChannelLine& line = *reinterpret_cast<const ChannelLine*>(s_geom + 48);
-  __shared__ int tot_cells[kWalkThreads / 32], tot_kept[kWalkThreads / 32];
+  __shared__ int tot_cells[kT / 32], tot_kept[kT / 32];
   __shared__ int s_exact, s_box[4], s_nospan;
-  __shared__ double red_d[kWalkThreads / 32];
-  __shared__ float red_f[kWalkThreads / 32];
+  __shared__ double red_d[kT / 32];
+  __shared__ float red_f[kRanges / 32];
   __shared__ float s_e;
-  __shared__ int s_col[kWalkThreads];
+  __shared__ int s_col[kRanges];
 
   if ((int64_t)blockIdx.x >= args.m) return;
   const int64_t row = args.sel ? (int64_t)args.sel[blockIdx.x] : (int64_t)blockIdx.x;
@@ -617,7 +627,7 @@ k_walk(WalkArgs args) {
     spans = s_nospan == 0;
     const float ya0 = c0[0][1], yb0 = c0[2][1], dya = c1[0][1] - ya0, dyb = c1[2][1] - yb0;
     const int half = threadIdx.x & 1, l0 = half * (kHullLines / 2);
-    for (int k0 = 0; k0 <= ns; k0 += kWalkThreads / 2) {
+    for (int k0 = 0; k0 <= ns; k0 += kT / 2) {
       const int k = k0 + (threadIdx.x >> 1);
       const float X = voxel_plane(g, sa, min(k, ns));
       float tlo = INFINITY, thi = -INFINITY, hlo = INFINITY, hhi = -INFINITY;
@@ -666,8 +676,8 @@ k_walk(WalkArgs args) {
   int* yr0 = xr1 + g.n[0];
   int* yr1 = yr0 + g.n[1];
   if (sa == 2) {
-    for (int i = threadIdx.x; i < g.n[0]; i += kWalkThreads) { xr0[i] = INT_MAX; xr1[i] = INT_MIN; }
-    for (int i = threadIdx.x; i < g.n[1]; i += kWalkThreads) { yr0[i] = INT_MAX; yr1[i] = INT_MIN; }
+    for (int i = threadIdx.x; i < g.n[0]; i += kT) { xr0[i] = INT_MAX; xr1[i] = INT_MIN; }
+    for (int i = threadIdx.x; i < g.n[1]; i += kT) { yr0[i] = INT_MAX; yr1[i] = INT_MIN; }
   }
   __syncthreads();
 
@@ -675,7 +685,7 @@ k_walk(WalkArgs args) {
   // bounding box of all of them
   {
     int xlo = INT_MAX, xhi = INT_MIN, ylo = INT_MAX, yhi = INT_MIN;
-    for (int i = threadIdx.x; i < ns; i += kWalkThreads) {
+    for (int i = threadIdx.x; i < ns; i += kT) {
       Slab sl;
       slab_window(G, c0, c1, pext, spans, sa, i, &sl);
       slabs[i] = sl;
@@ -709,7 +719,7 @@ k_walk(WalkArgs args) {
   win.wby = s_box[3] >= s_box[2] ? s_box[3] - s_box[2] + 1 : 0;
   win.wbyp = win.wby + 1;
   const int A = (win.wbx + 1) * win.wbyp;  // table entries (with the empty border)
-  const int kper = (A + kWalkThreads - 1) / kWalkThreads;
+  const int kper = (A + kT - 1) / kT;
   const int kbeg = min(A, (int)threadIdx.x * kper), kend = min(A, kbeg + kper);
   // The z runs of the thread's columns k = (ix, iy), f(k, first, last) in
   // order (empty: last < first): for x slabs the range of slab ix's rectangle
@@ -756,7 +766,7 @@ k_walk(WalkArgs args) {
     // columns + cells, computed without the table
     int n = 0, W;
     for_cols([&](int, int zlo, int zhi) { n += max(zhi - zlo + 1, 0); });
-    block_excl_scan(n, tot_cells, &W);
+    block_excl_scan<kT>(n, tot_cells, &W);
     // + the cell that counts hits outside, and one
     if (threadIdx.x == 0) args.win_cells[row] = A + W + 2;
     return;
@@ -774,7 +784,7 @@ k_walk(WalkArgs args) {
     });
   // column lengths -> first cells (exclusive scan)
   int W;  // window cells
-  const int cexcl = block_excl_scan(n_mine, tot_cells, &W);
+  const int cexcl = block_excl_scan<kT>(n_mine, tot_cells, &W);
   if (!table_fits || A + W + 2 > args.cap_cells) {
     if (threadIdx.x == 0) {
       int k = atomicAdd(args.overflow_count, 1);
@@ -788,12 +798,12 @@ k_walk(WalkArgs args) {
   win.hi = win.lo + W + 2;
   win.hioff = 4u * (uint32_t)(W + 2);
   const uint32_t lo_s = (uint32_t)__cvta_generic_to_shared(win.lo);
-  // Extraction: thread t takes the cells [t cpt, (t + 1) cpt) (an odd count:
+  // Extraction: range t of the cells is [t cpt, (t + 1) cpt) (an odd count:
   // the lanes' concurrent reads fall in distinct shared-memory banks), from
-  // column s_col[t] on.
-  const int cpt = ((W + kWalkThreads - 1) / kWalkThreads) | 1;
+  // column s_col[t] on; thread t takes the ranges t, t + kT, ...
+  const int cpt = ((W + kRanges - 1) / kRanges) | 1;
   const float inv_cpt = __fdividef(1.f, (float)cpt);
-  auto first_thread = [&](int o) { return (int)(((float)(o + cpt) - 0.5f) * inv_cpt); };  // ceil(o / cpt)
+  auto first_range = [&](int o) { return (int)(((float)(o + cpt) - 0.5f) * inv_cpt); };  // ceil(o / cpt)
   {
     int o = cexcl;
     for (int k = kbeg; k < kend; k++) {
@@ -801,12 +811,12 @@ k_walk(WalkArgs args) {
       const int zn = max(z1 - z0 + 1, 0);
       cz0[k] = (int)(lo_s + 4u * (uint32_t)(zn > 0 ? o - z0 : o));  // (o - z0 may be < 0)
       cz1[k] = zn > 0 ? z0 | (zn << 16) : 0;
-      // the threads whose cells start in this column
-      for (int t = first_thread(o); t < kWalkThreads && t * cpt < o + zn; t++) s_col[t] = k;
+      // the ranges that start in this column
+      for (int t = first_range(o); t < kRanges && t * cpt < o + zn; t++) s_col[t] = k;
       o += zn;
     }
     uint32_t* guard = reinterpret_cast<uint32_t*>(smem + lay.pool);
-    for (int i = threadIdx.x; i < lay.gcol / 4; i += kWalkThreads) guard[i] = lo_s;
+    for (int i = threadIdx.x; i < lay.gcol / 4; i += kT) guard[i] = lo_s;
   }
   win.cbase = reinterpret_cast<const uint32_t*>(cz0);
   win.zrun = reinterpret_cast<const uint32_t*>(cz1);
@@ -821,24 +831,24 @@ k_walk(WalkArgs args) {
   win.poff1 = g.n[0] + 1;
   win.poff2 = g.n[0] + g.n[1] + 2;
   if (threadIdx.x == 0) planes[-1] = planes[nplanes] = 0.f;
-  for (int i = threadIdx.x; i < nplanes; i += kWalkThreads) {
+  for (int i = threadIdx.x; i < nplanes; i += kT) {
     const int a = i < win.poff1 ? 0 : (i < win.poff2 ? 1 : 2);
     planes[i] = voxel_plane(g, a, i - (a == 0 ? 0 : (a == 1 ? win.poff1 : win.poff2)));
   }
   // per z cell the candidate test's z terms ab1 * ap2 and ab0 * ap2
   // (ap = voxel centre - a; the other terms are constant along a column)
   float2* ztab = reinterpret_cast<float2*>(smem + lay.ztab);
-  for (int iz = threadIdx.x; iz < g.n[2]; iz += kWalkThreads) {
+  for (int iz = threadIdx.x; iz < g.n[2]; iz += kT) {
     const float ap2 = fsub(voxel_centre(g, 2, iz), line.a[2]);
     ztab[iz] = make_float2(fmul(line.ab[1], ap2), fmul(line.ab[0], ap2));
   }
   // ---- zero the window, walk the rays
-  for (int i = threadIdx.x; i < W + 2; i += kWalkThreads)  // lo, then hi words
+  for (int i = threadIdx.x; i < W + 2; i += kT)  // lo, then hi words
     reinterpret_cast<uint2*>(win.lo)[i] = make_uint2(0u, 0u);
   __syncthreads();
   const int R = G.p.nrays;
   const float* rays = args.rays + row * (int64_t)R * 6;
-  // Rays to lanes: whole rays, one per lane, in rounds of kWalkThreads;
+  // Rays to lanes: whole rays, one per lane, in rounds of kT;
   // in the last round, whole warps take one ray per lane and the remaining
   // rays are cut into equal pieces over the remaining lanes (100 rays: 3
   // warps of whole rays, 4 rays in 8 pieces each on the fourth warp).
@@ -852,17 +862,17 @@ k_walk(WalkArgs args) {
     };
     // one call site, so each form of the walk loop is compiled once
     const int t = threadIdx.x;
-    const int rounds = R / kWalkThreads;
-    const int rr = R - rounds * kWalkThreads, r0 = rounds * kWalkThreads;
+    const int rounds = R / kT;
+    const int rr = R - rounds * kT, r0 = rounds * kT;
     const int fw = rr / 32;  // warps of whole rays in the last round
     for (int k = 0; k <= rounds; k++) {
-      int r = k * kWalkThreads + t, piece = 0, np = 1;
+      int r = k * kT + t, piece = 0, np = 1;
       bool act = true;
       if (k == rounds) {
         if (t < fw * 32) {
           r = r0 + t;
         } else {
-          const int rem = rr - fw * 32, lanes = kWalkThreads - fw * 32;
+          const int rem = rr - fw * 32, lanes = kT - fw * 32;
           np = rem > 0 ? lanes / rem : 1;
           const int l = t - fw * 32;
           act = rem > 0 && l < rem * np;
@@ -885,12 +895,12 @@ k_walk(WalkArgs args) {
   }
 
   // ---- ordered extraction: the cells are stored in voxel-id order
-  const int cbeg = min(W, (int)threadIdx.x * cpt), cend = min(W, cbeg + cpt);
-  // Visits the thread's range in order: fcol(ix, iy) on entering a column,
+  // Visits range q's cells in order: fcol(ix, iy) on entering a column,
   // f(cell, ix, iy, iz) per cell.
-  auto for_cells = [&](auto&& fcol, auto&& f) {
+  auto for_cells = [&](int q, auto&& fcol, auto&& f) {
+    const int cbeg = min(W, q * cpt), cend = min(W, cbeg + cpt);
     if (cbeg >= cend) return;
-    int k = s_col[threadIdx.x];
+    int k = s_col[q];
     uint32_t e = win.zrun[k];
     int zhi = (int)(e & 0xffffu) + (int)(e >> 16) - 1;
     int cx = k / win.wbyp, cy = k - cx * win.wbyp;
@@ -921,50 +931,60 @@ k_walk(WalkArgs args) {
   // value are computed for all of them and the result selected).  The
   // candidate test is the reference's |ab x ap|^2 with the same operations:
   // its x and y terms come per column, its z terms from the table.
-  int cnt = 0;
-  float fsum = 0.f;
+  int cnts[kMine];
+  float fsums[kMine];
   const float inv_fR = __frcp_rn(fR);
-  float K0 = 0.f, K1 = 0.f, c2sq = 0.f;
-  int colvox = 0;
-  for_cells(
-      [&](int ix, int iy) {
-        const float ap0 = fsub(voxel_centre(g, 0, ix), L.a[0]);
-        const float ap1 = fsub(voxel_centre(g, 1, iy), L.a[1]);
-        K0 = fmul(L.ab[2], ap1);
-        K1 = fmul(L.ab[2], ap0);
-        const float c2 = fsub(fmul(L.ab[0], ap1), fmul(L.ab[1], ap0));
-        c2sq = fmul(c2, c2);
-        colvox = ix * G.nyz + iy * g.n[2];
-      },
-      [&](int cidx, int ix, int iy, int iz) {
-    const unsigned long long u =
-        ((unsigned long long)win.hi[cidx] << win.split) + (unsigned long long)win.lo[cidx];
-    const float2 zt = ztab[iz];
-    const float c0 = fsub(zt.x, K0), c1 = fsub(K1, zt.y);
-    // not a candidate: dropped
-    const bool cand = fadd(fadd(fmul(c0, c0), fmul(c1, c1)), c2sq) < L.s_max;
-    const bool keep = (u != 0ull) & cand;
-    const float v = div_cr(fmul(__ull2float_rn(u), G.fx_inv), fR, inv_fR);
-    if (kMode == kModeCsr || kMode == kModeMlem) {
-      // kept entries compacted at the start of the thread's range: the slot
-      // written is this cell's or an earlier one, already read
-      win.lo[cbeg + cnt] = __float_as_uint(v);
-      win.hi[cbeg + cnt] = (uint32_t)(colvox + iz);
-    }
-    cnt += keep ? 1 : 0;
-    if (kMode != kModeCsr && keep) {
-      const int vox = colvox + iz;
-      if (kMode == kModeForward || kMode == kModeMlem) fsum = fadd(fsum, fmul(v, args.x[vox]));
-      if (kMode == kModeBack) {
-        const float ev = args.e[row];
-        if (ev != 0.f) atomicAdd(&args.c[vox], fmul(v, ev));
+#pragma unroll
+  for (int i = 0; i < kMine; i++) {
+    const int q = (int)threadIdx.x + i * kT, cbeg = min(W, q * cpt);
+    int cnt = 0;
+    float fsum = 0.f;
+    float K0 = 0.f, K1 = 0.f, c2sq = 0.f;
+    int colvox = 0;
+    for_cells(
+        q,
+        [&](int ix, int iy) {
+          const float ap0 = fsub(voxel_centre(g, 0, ix), L.a[0]);
+          const float ap1 = fsub(voxel_centre(g, 1, iy), L.a[1]);
+          K0 = fmul(L.ab[2], ap1);
+          K1 = fmul(L.ab[2], ap0);
+          const float c2 = fsub(fmul(L.ab[0], ap1), fmul(L.ab[1], ap0));
+          c2sq = fmul(c2, c2);
+          colvox = ix * G.nyz + iy * g.n[2];
+        },
+        [&](int cidx, int ix, int iy, int iz) {
+      const unsigned long long u =
+          ((unsigned long long)win.hi[cidx] << win.split) + (unsigned long long)win.lo[cidx];
+      const float2 zt = ztab[iz];
+      const float c0 = fsub(zt.x, K0), c1 = fsub(K1, zt.y);
+      // not a candidate: dropped
+      const bool cand = fadd(fadd(fmul(c0, c0), fmul(c1, c1)), c2sq) < L.s_max;
+      const bool keep = (u != 0ull) & cand;
+      const float v = div_cr(fmul(__ull2float_rn(u), G.fx_inv), fR, inv_fR);
+      if (kMode == kModeCsr || kMode == kModeMlem) {
+        // kept entries compacted at the start of the thread's range: the slot
+        // written is this cell's or an earlier one, already read
+        win.lo[cbeg + cnt] = __float_as_uint(v);
+        win.hi[cbeg + cnt] = (uint32_t)(colvox + iz);
       }
-      if (kMode == kModeColSum) atomicAdd(&args.s64[vox], (double)v);
-    }
-  });
+      cnt += keep ? 1 : 0;
+      if (kMode != kModeCsr && keep) {
+        const int vox = colvox + iz;
+        if (kMode == kModeForward || kMode == kModeMlem) fsum = fadd(fsum, fmul(v, args.x[vox]));
+        if (kMode == kModeBack) {
+          const float ev = args.e[row];
+          if (ev != 0.f) atomicAdd(&args.c[vox], fmul(v, ev));
+        }
+        if (kMode == kModeColSum) atomicAdd(&args.s64[vox], (double)v);
+      }
+    });
+    cnts[i] = cnt;
+    fsums[i] = fsum;
+  }
   if (kMode == kModeCsr) {
     int kept;
-    const int pos = block_excl_scan(cnt, tot_kept, &kept);
+    const int cnt = cnts[0], cbeg = min(W, (int)threadIdx.x * cpt);
+    const int pos = block_excl_scan<kT>(cnt, tot_kept, &kept);
     const int64_t o = slot * args.stride + pos;
     for (int j = 0; j < cnt; j++) {
       args.stage_col[o + j] = (int32_t)win.hi[cbeg + j];
@@ -975,16 +995,19 @@ k_walk(WalkArgs args) {
       if (args.sel) args.ovf_idx[row] = (int32_t)slot;
     }
   } else if (kMode == kModeForward || kMode == kModeMlem) {
-    // deterministic block reduction in thread order
+    // deterministic block reduction in the order of the ranges
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    float v = fsum;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fadd(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) red_f[w] = v;
+    for (int i = 0; i < kMine; i++) {
+      float v = fsums[i];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v = fadd(v, __shfl_down_sync(0xffffffffu, v, o));
+      if (lane == 0) red_f[i * (kT / 32) + w] = v;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
       float t = 0.f;
-      for (int k = 0; k < kWalkThreads / 32; k++) t = fadd(t, red_f[k]);
+      for (int k = 0; k < kRanges / 32; k++) t = fadd(t, red_f[k]);
       if (args.y) args.y[row] = t;
       // e = y / (A x) (mlemOperations.hpp:22-32, 0 where A x == 0)
       if (kMode == kModeMlem) s_e = t > 0.f ? __fdiv_rn(args.ycnt[row], t) : 0.f;
@@ -993,11 +1016,15 @@ k_walk(WalkArgs args) {
       // the row's share of A^T e: its kept entries, compacted in pass 1
       __syncthreads();
       const float ev = s_e;
-      if (ev != 0.f)
-        for (int j = 0; j < cnt; j++) {
-          atomicAdd(&args.c64[win.hi[cbeg + j]],
-                    (double)fmul(__uint_as_float(win.lo[cbeg + j]), ev));
+      if (ev != 0.f) {
+#pragma unroll
+        for (int i = 0; i < kMine; i++) {
+          const int cbeg = min(W, ((int)threadIdx.x + i * kT) * cpt);
+          for (int j = 0; j < cnts[i]; j++)
+            atomicAdd(&args.c64[win.hi[cbeg + j]],
+                      (double)fmul(__uint_as_float(win.lo[cbeg + j]), ev));
         }
+      }
     }
   }
   (void)red_d;
@@ -1075,14 +1102,29 @@ static int max_dyn_smem() {
   return v;
 }
 
-template <int kMode>
-static epet_status launch_walk(WalkArgs a, size_t smem, cudaStream_t st) {
-  if (a.m == 0) return EPET_OK;
-  EPET_CUDA(cudaFuncSetAttribute(k_walk<kMode>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+// Measured, 122,412 channels (every 7th of 30 angles), forward projection, 64
+// against 128 threads: 32^3 voxels and 10 rays 1.26 / 1.59 ms, 20 rays 1.38 /
+// 1.69, 60 rays 1.77 / 2.21, 80 rays 2.09 / 2.32; 64^3 voxels and 60 rays 3.06
+// / 3.25, 80 rays 3.54 / 3.48, 100 rays 4.42 / 3.80 (52^3: 3.55 / 3.25).  32
+// threads win only at 24^3 (10 rays: 1.01).
+static int walk_threads(const Geo& G) {
+  return G.p.nrays <= kFewRays ? kWalkThreadsFew : kWalkThreads;
+}
+
+template <int kMode, int kT>
+static epet_status launch_walk_as(const WalkArgs& a, size_t smem, cudaStream_t st) {
+  EPET_CUDA(cudaFuncSetAttribute(k_walk<kMode, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
-  k_walk<kMode><<<(unsigned)a.m, kWalkThreads, smem, st>>>(a);
+  k_walk<kMode, kT><<<(unsigned)a.m, kT, smem, st>>>(a);
   EPET_LAUNCHED();
   return EPET_OK;
+}
+
+template <int kMode>
+static epet_status launch_walk(const WalkArgs& a, size_t smem, cudaStream_t st) {
+  if (a.m == 0) return EPET_OK;
+  if (walk_threads(a.G) == kWalkThreads) return launch_walk_as<kMode, kWalkThreads>(a, smem, st);
+  return launch_walk_as<kMode, kWalkThreadsFew>(a, smem, st);
 }
 
 // Rows processed per chunk (rays and staging are chunk-sized).
@@ -1154,8 +1196,11 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
   int cap = std::max(256, (int)(p90 * 1.10) + 64);
   auto resident = [&](int c) {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_walk<kModeCsr>, kWalkThreads,
-                                                      walk_smem(G, c)) != cudaSuccess)
+    const bool few = walk_threads(G) == kWalkThreadsFew;
+    const void* k = few ? (const void*)k_walk<kModeCsr, kWalkThreadsFew>
+                        : (const void*)k_walk<kModeCsr, kWalkThreads>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, walk_threads(G), walk_smem(G, c)) !=
+        cudaSuccess)
       n = 0;
     return n;
   };
