@@ -124,18 +124,25 @@ static int bits_for(int64_t maxval) {
 // Stable LSD radix sort with BITS-bit digits, reduce-then-scan over chunks:
 // the input is cut into nchunks equal runs of whole tiles (a few per SM);
 // the histogram kernel counts each chunk's digits (BINS x nchunks counts),
-// an exclusive scan of the digit-major counts gives every (digit, chunk) its
-// output start, and the scatter kernel walks its chunk's tiles in order,
-// keeping a running output offset per digit.  Within a tile, items are
-// ranked stably -- warp w owns items [w*512, (w+1)*512) and ranks them in 16
-// rounds of 32 consecutive items with __match_any_sync -- and staged in
-// shared memory in digit order, so each digit's global writes are
-// contiguous runs.  Input and output go through adapters, so the first pass
-// of the column-major copy reads a CSR directly and the last one writes the
-// CSC arrays and its column starts.
-constexpr int kRsThreads = 256, kRsItems = 16, kRsTile = kRsThreads * kRsItems;
+// a scan of each digit's counts over the chunks and one of the digits' totals
+// (in the scatter kernel) give every (digit, chunk) its output start, and the
+// scatter kernel walks its chunk's tiles in order, keeping a running output
+// offset per digit.  Within a tile, items are ranked stably -- warp w owns
+// items [w*256, (w+1)*256) and ranks them in 8 rounds of 32 consecutive items
+// -- and staged in shared memory in digit order, so each digit's global
+// writes are contiguous runs.  Input and output go through adapters, so the
+// first pass of the column-major copy reads a CSR directly and the last one
+// writes the CSC arrays and its column starts, and likewise for COO triples.
+// The scatter is bound by the latency of its phases (rank, scan, stage,
+// write), not by bytes (2.4 TB/s): a tile of 4096 items has 16 warps and
+// 16-bit counts, its items are loaded while the tile before it is written,
+// two blocks an SM.  A pass over 20M (8-byte key, 4-byte value) pairs takes
+// 171 us with 9-bit digits (8 warps, 16 rounds of matches and 8-bit digits:
+// 190; three blocks an SM spill: 247).
+constexpr int kRsThreads = 512, kRsItems = 8, kRsTile = kRsThreads * kRsItems;
 constexpr int kRsWarps = kRsThreads / 32;
 constexpr int kRsMaxChunks = 2048;
+constexpr int kRsBlocks = 2;  // resident blocks per SM
 
 struct RsGrid {
   int64_t tiles, tpc;  // tiles, tiles per chunk
@@ -147,7 +154,7 @@ static RsGrid rs_grid(int64_t n) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t want = std::min<int64_t>(kRsMaxChunks, 3 * (int64_t)sms);
+  const int64_t want = std::min<int64_t>(kRsMaxChunks, kRsBlocks * (int64_t)sms);
   g.tpc = (g.tiles + want - 1) / want;
   g.nchunks = (int)((g.tiles + g.tpc - 1) / g.tpc);
   return g;
@@ -199,6 +206,27 @@ struct ArrOut {
   }
 };
 
+// COO triples in (key = row above the column's bits) and out.
+struct CooIn {
+  const int32_t *row, *col;
+  const float* v;
+  int colbits;
+  __device__ uint64_t key(int64_t i) const {
+    return ((uint64_t)(uint32_t)row[i] << colbits) | (uint32_t)col[i];
+  }
+  __device__ uint32_t val(int64_t i) const { return __float_as_uint(v[i]); }
+};
+struct CooOut {
+  int32_t *row, *col;
+  float* v;
+  int colbits;
+  __device__ void put(int64_t pos, uint64_t key, uint32_t val, bool) const {
+    row[pos] = (int32_t)(key >> colbits);
+    col[pos] = (int32_t)(key & ((uint64_t(1) << colbits) - 1));
+    v[pos] = __uint_as_float(val);
+  }
+};
+
 // CSR in, with the row of every entry precomputed (k_row_ids): key =
 // column, value = (row << 32) | value bits.
 struct CsrIn {
@@ -217,14 +245,6 @@ struct PosIn {
   __device__ uint32_t key(int64_t i) const { return (uint32_t)col[i]; }
   __device__ uint32_t val(int64_t i) const { return (uint32_t)i; }
 };
-// CSR-ordered keys (runs of ascending columns): ranked by ballots.
-template <typename In>
-struct IsCsrIn : std::false_type {};
-template <>
-struct IsCsrIn<CsrIn> : std::true_type {};
-template <>
-struct IsCsrIn<PosIn> : std::true_type {};
-
 // Row id of every CSR entry (a warp per row).
 __global__ void k_row_ids(const int64_t* __restrict__ row_ptr, int64_t m,
                           int32_t* __restrict__ row) {
@@ -262,10 +282,12 @@ struct CscOut {
 };
 
 template <int BITS, typename K, typename V, typename In, typename Out>
-__global__ void __launch_bounds__(kRsThreads, 3)
+__global__ void __launch_bounds__(kRsThreads, kRsBlocks)
 k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
-                const int64_t* __restrict__ offs, const uint64_t* __restrict__ vary) {
+                const int64_t* __restrict__ offs, const int64_t* __restrict__ totals,
+                const uint64_t* __restrict__ vary) {
   constexpr int BINS = 1 << BITS;
+  static_assert(BINS <= kRsThreads, "a digit per thread");
   if (!pass_active(vary, shift, BINS - 1)) {
     const int64_t beg = (int64_t)blockIdx.x * tpc * kRsTile;
     const int64_t end = min(n, beg + tpc * kRsTile);
@@ -273,7 +295,7 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
       out.put(i, in.key(i), in.val(i), false);
     return;
   }
-  __shared__ unsigned wcnt[kRsWarps][BINS];
+  __shared__ uint16_t wcnt[kRsWarps][BINS];  // (a tile holds 4096 items)
   __shared__ unsigned dstart[BINS + 1];
   __shared__ unsigned warp_tot[kRsWarps];
   __shared__ int64_t run[BINS];  // output position of the chunk's next item of each digit
@@ -281,9 +303,37 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
   V* sv = reinterpret_cast<V*>(rs_dyn);
   K* sk = reinterpret_cast<K*>(rs_dyn + sizeof(V) * kRsTile);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int d = threadIdx.x; d < BINS; d += kRsThreads) run[d] = offs[(int64_t)d * nchunks + blockIdx.x];
-  constexpr int DPT = (BINS + kRsThreads - 1) / kRsThreads;  // digits per thread
+  {
+    // the digits' first positions: exclusive scan of their totals
+    __shared__ int64_t tot64[kRsWarps];
+    const int d = threadIdx.x;
+    const int64_t mine = d < BINS ? totals[(int64_t)d * nchunks] : 0;
+    int64_t inc = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (lane == 31) tot64[w] = inc;
+    __syncthreads();
+    int64_t before = 0;
+    for (int k = 0; k < w; k++) before += tot64[k];
+    if (d < BINS) run[d] = before + inc - mine + offs[(int64_t)d * nchunks + blockIdx.x];
+  }
   const unsigned lt = (1u << lane) - 1u;
+  // a tile's items in registers, loaded while the tile before is written
+  K kk[kRsItems];
+  V vv[kRsItems];
+  auto load = [&](int64_t tile0) {
+    const int64_t wbase = tile0 + (int64_t)w * (kRsItems * 32);
+#pragma unroll
+    for (int r = 0; r < kRsItems; r++) {
+      const int64_t i = wbase + r * 32 + lane;
+      kk[r] = i < n ? in.key(i) : K(0);
+      vv[r] = i < n ? in.val(i) : V(0);
+    }
+  };
+  load((int64_t)blockIdx.x * tpc * kRsTile);
   for (int64_t t = 0; t < tpc; t++) {
     const int64_t tile0 = ((int64_t)blockIdx.x * tpc + t) * kRsTile;
     if (tile0 >= n) break;
@@ -291,61 +341,42 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
     for (int d = lane; d < BINS; d += 32) wcnt[w][d] = 0;
     __syncwarp();
     const int64_t wbase = tile0 + (int64_t)w * (kRsItems * 32);
-    // keys only in registers (ranking); values are read once, when staged
-    K kk[kRsItems];
     unsigned rank[kRsItems];
 #pragma unroll
     for (int r = 0; r < kRsItems; r++) {
       const int64_t i = wbase + r * 32 + lane;
-      kk[r] = i < n ? in.key(i) : K(0);
-    }
-#pragma unroll
-    for (int r = 0; r < kRsItems; r++) {
-      const int64_t i = wbase + r * 32 + lane;
       const bool ok = i < n;
-      const unsigned dig = ok ? ((unsigned)(kk[r] >> shift) & (BINS - 1)) : BINS + lane;
-      unsigned peers;
-      if constexpr (IsCsrIn<In>::value) {
-        // rows of a CSR: consecutive columns, up to 32 distinct digits per
-        // round, where one ballot per digit bit is cheaper than a match
-        peers = __ballot_sync(0xffffffffu, ok);
-        peers = ok ? peers : (1u << lane);
+      const unsigned dig = (unsigned)(kk[r] >> shift) & (BINS - 1);
+      // the lanes with the same digit, one ballot per digit bit (with many
+      // distinct digits in a round cheaper than a match)
+      unsigned peers = __ballot_sync(0xffffffffu, ok);
+      peers = ok ? peers : (1u << lane);
 #pragma unroll
-        for (int b = 0; b < BITS; b++) {
-          const bool bit = (dig >> b) & 1u;
-          const unsigned bal = __ballot_sync(0xffffffffu, bit);
-          peers &= bit ? bal : ~bal;
-        }
-      } else {
-        peers = __match_any_sync(0xffffffffu, dig);
+      for (int b = 0; b < BITS; b++) {
+        const bool bit = (dig >> b) & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, bit);
+        peers &= bit ? bal : ~bal;
       }
       unsigned before = 0;
       if (ok) before = wcnt[w][dig];
       rank[r] = before + __popc(peers & lt);
       __syncwarp();
       const int leader = 31 - __clz(peers);
-      if (ok && lane == leader) wcnt[w][dig] = before + __popc(peers);
+      if (ok && lane == leader) wcnt[w][dig] = (uint16_t)(before + __popc(peers));
       __syncwarp();
     }
     __syncthreads();
-    // per digit: warp offsets (exclusive over warps) and the digit total
-    unsigned tot[DPT];
+    // per digit (a thread each): warp offsets (exclusive over warps) and the
+    // digit's total, then an exclusive scan of the totals
     unsigned mysum = 0;
+    if (threadIdx.x < BINS) {
 #pragma unroll
-    for (int q = 0; q < DPT; q++) {
-      const int d = threadIdx.x * DPT + q;
-      unsigned acc = 0;
-      if (d < BINS) {
-        for (int ww = 0; ww < kRsWarps; ww++) {
-          const unsigned c = wcnt[ww][d];
-          wcnt[ww][d] = acc;
-          acc += c;
-        }
+      for (int ww = 0; ww < kRsWarps; ww++) {
+        const unsigned c = wcnt[ww][threadIdx.x];
+        wcnt[ww][threadIdx.x] = (uint16_t)mysum;
+        mysum += c;
       }
-      tot[q] = acc;
-      mysum += acc;
     }
-    // exclusive scan of the digit totals (block-wide, digits in thread order)
     unsigned inc = mysum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -354,26 +385,12 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
     }
     if (lane == 31) warp_tot[w] = inc;
     __syncthreads();
-    if (w == 0) {
-      const unsigned u = lane < kRsWarps ? warp_tot[lane] : 0u;
-      unsigned ti = u;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned x = __shfl_up_sync(0xffffffffu, ti, o);
-        if (lane >= o) ti += x;
-      }
-      if (lane < kRsWarps) warp_tot[lane] = ti - u;
-    }
-    __syncthreads();
     {
-      unsigned acc = warp_tot[w] + inc - mysum;
+      unsigned before = 0;
 #pragma unroll
-      for (int q = 0; q < DPT; q++) {
-        const int d = threadIdx.x * DPT + q;
-        if (d < BINS) dstart[d] = acc;
-        acc += tot[q];
-      }
-      if (threadIdx.x == kRsThreads - 1) dstart[BINS] = acc;
+      for (int k = 0; k < kRsWarps; k++) before += k < w ? warp_tot[k] : 0u;
+      if (threadIdx.x < BINS) dstart[threadIdx.x] = before + inc - mysum;
+      if (threadIdx.x == kRsThreads - 1) dstart[BINS] = before + inc;
     }
     __syncthreads();
     // stage in digit order
@@ -384,9 +401,10 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
         const unsigned dig = (unsigned)(kk[r] >> shift) & (BINS - 1);
         const unsigned lp = dstart[dig] + wcnt[w][dig] + rank[r];
         sk[lp] = kk[r];
-        sv[lp] = in.val(i);
+        sv[lp] = vv[r];
       }
     }
+    if (t + 1 < tpc) load(tile0 + kRsTile);
     __syncthreads();
     // contiguous runs per digit
     for (int j = threadIdx.x; j < tile_n; j += kRsThreads) {
@@ -396,14 +414,47 @@ k_radix_scatter(In in, Out out, int64_t n, int shift, int64_t tpc, int nchunks,
       out.put(run[dig] + (j - (int)dstart[dig]), key, sv[j], first);
     }
     __syncthreads();
+    // (the next tile's writes come several barriers later)
     for (int d = threadIdx.x; d < BINS; d += kRsThreads) run[d] += dstart[d + 1] - dstart[d];
-    __syncthreads();
   }
 }
 
 size_t radix_hist_elems(int64_t n) {
   const int64_t tiles = std::max<int64_t>(1, (n + kRsTile - 1) / kRsTile);
   return (size_t)512 * (size_t)std::min<int64_t>(tiles, kRsMaxChunks);
+}
+
+// Per digit (a block each) the exclusive scan of its counts over the chunks;
+// the digit's total replaces its first count.
+__global__ void __launch_bounds__(256)
+k_digit_scan(int64_t* __restrict__ hist, int64_t* __restrict__ offs, int nchunks) {
+  __shared__ int64_t tot[256 / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int64_t* h = hist + (int64_t)blockIdx.x * nchunks;
+  int64_t* o = offs + (int64_t)blockIdx.x * nchunks;
+  int64_t run = 0;
+  for (int c0 = 0; c0 < nchunks; c0 += 256) {
+    const int c = c0 + threadIdx.x;
+    const int64_t v = c < nchunks ? h[c] : 0;
+    int64_t inc = v;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, inc, k);
+      if (lane >= k) inc += u;
+    }
+    if (lane == 31) tot[w] = inc;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < 256 / 32; k++) {
+      before += k < w ? tot[k] : 0;
+      all += tot[k];
+    }
+    if (c < nchunks) o[c] = run + before + inc - v;
+    run += all;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) h[0] = run;
 }
 
 // One pass: histogram of `in`'s keys, scan, scatter from `in` to `out`.
@@ -414,48 +465,28 @@ epet_status radix_pass(In in, Out out, int64_t n, int shift, int64_t* hist, int6
   k_radix_hist<BITS, In><<<(unsigned)g.nchunks, kRsThreads, 0, st>>>(in, n, shift, g.tpc,
                                                                      g.nchunks, hist, vary);
   EPET_LAUNCHED();
-  EPET_CHECK(exclusive_scan_i64(hist, hist_scan, (int64_t)(1 << BITS) * g.nchunks, scan_tmp, st));
+  (void)scan_tmp;
+  k_digit_scan<<<1 << BITS, 256, 0, st>>>(hist, hist_scan, g.nchunks);
+  EPET_LAUNCHED();
   const size_t dyn = (sizeof(K) + sizeof(V)) * (size_t)kRsTile;
   EPET_CUDA(cudaFuncSetAttribute(k_radix_scatter<BITS, K, V, In, Out>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
   k_radix_scatter<BITS, K, V, In, Out><<<(unsigned)g.nchunks, kRsThreads, dyn, st>>>(
-      in, out, n, shift, g.tpc, g.nchunks, hist_scan, vary);
+      in, out, n, shift, g.tpc, g.nchunks, hist_scan, hist, vary);
   EPET_LAUNCHED();
   return EPET_OK;
 }
 
-// Sorts (keys, vals) in place on the low `bits` bits (8-bit digits).
-template <typename K, typename Vt>
-epet_status radix_sort(K* keys, Vt* vals, K* alt_keys, Vt* alt_vals, int64_t n, int bits,
-                       int64_t* hist, int64_t* hist_scan, int64_t* scan_tmp,
-                       cudaStream_t st) {
-  if (n <= 1 || bits <= 0) return EPET_OK;
-  K *src_k = keys, *dst_k = alt_keys;
-  Vt *src_v = vals, *dst_v = alt_vals;
-  int passes = 0;
-  for (int shift = 0; shift < bits; shift += 8, passes++) {
-    EPET_CHECK((radix_pass<8, K, Vt>(ArrIn<K, Vt>{src_k, src_v}, ArrOut<K, Vt>{dst_k, dst_v},
-                                      n, shift, hist, hist_scan, scan_tmp, st)));
-    std::swap(src_k, dst_k);
-    std::swap(src_v, dst_v);
-  }
-  if (passes & 1) {
-    EPET_CUDA(cudaMemcpyAsync(keys, src_k, n * sizeof(K), cudaMemcpyDeviceToDevice, st));
-    EPET_CUDA(cudaMemcpyAsync(vals, src_v, n * sizeof(Vt), cudaMemcpyDeviceToDevice, st));
-  }
-  return EPET_OK;
-}
+// Sorts COO triples in place by their `bits`-bit keys: the first pass reads the
+// triples, the last one writes them (packing and unpacking them in passes of
+// their own took 196 of 2590 us for 20M); a single pass goes through the
+// scratch pairs (a pass cannot scatter onto its input).
+template <int BITS>
+static epet_status coo_passes(const CooIn& in, const CooOut& out, int64_t n, int bits,
+                              uint64_t* keys[2], uint32_t* vals[2], int64_t* hist,
+                              int64_t* hist_scan, cudaStream_t st);
 
 // ----------------------------------------------------------- COO helpers
-__global__ void k_pack_coo(const int32_t* row, const int32_t* col, const float* val,
-                           int64_t n, int colbits, uint64_t* key, uint32_t* v) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    key[i] = ((uint64_t)(uint32_t)row[i] << colbits) | (uint32_t)col[i];
-    v[i] = __float_as_uint(val[i]);
-  }
-}
-
 __global__ void k_unpack_coo(const uint64_t* key, const uint32_t* v, int64_t n, int colbits,
                              int32_t* row, int32_t* col, float* val) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -466,37 +497,37 @@ __global__ void k_unpack_coo(const uint64_t* key, const uint32_t* v, int64_t n, 
   }
 }
 
-__global__ void k_max2(const int32_t* a, const int32_t* b, int64_t n, int* out) {
-  int ma = 0, mb = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    ma = max(ma, a[i]);
-    mb = max(mb, b[i]);
+// out = {max a, max b, min a, min b}, initialised to 0 (the ids' lower bound);
+// four loads of each array in flight per thread.
+__global__ void __launch_bounds__(256)
+k_range2(const int32_t* __restrict__ a, const int32_t* __restrict__ b, int64_t n, int* out) {
+  int xa = 0, xb = 0, na = 0, nb = 0;
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * step) {
+    int va[4], vb[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int64_t j = i + k * step;
+      va[k] = j < n ? a[j] : 0;
+      vb[k] = j < n ? b[j] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      xa = max(xa, va[k]);
+      na = min(na, va[k]);
+      xb = max(xb, vb[k]);
+      nb = min(nb, vb[k]);
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    ma = max(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-    mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-  }
+  xa = __reduce_max_sync(0xffffffffu, xa);
+  xb = __reduce_max_sync(0xffffffffu, xb);
+  na = __reduce_min_sync(0xffffffffu, na);
+  nb = __reduce_min_sync(0xffffffffu, nb);
   if ((threadIdx.x & 31) == 0) {
-    atomicMax(&out[0], ma);
-    atomicMax(&out[1], mb);
-  }
-}
-
-__global__ void k_min2(const int32_t* a, const int32_t* b, int64_t n, int* out) {
-  int ma = 0, mb = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    ma = min(ma, a[i]);
-    mb = min(mb, b[i]);
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    ma = min(ma, __shfl_xor_sync(0xffffffffu, ma, o));
-    mb = min(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-  }
-  if ((threadIdx.x & 31) == 0) {
-    atomicMin(&out[0], ma);
-    atomicMin(&out[1], mb);
+    atomicMax(&out[0], xa);
+    atomicMax(&out[1], xb);
+    atomicMin(&out[2], na);
+    atomicMin(&out[3], nb);
   }
 }
 
@@ -527,28 +558,92 @@ __global__ void k_fill_i64(int64_t* p, int64_t n, int64_t v) {
   if (i < n) p[i] = v;
 }
 
-// p[i] = min(p[i..n-1]) by one block: per-thread chunk minima, a block-wide
-// suffix scan of them, then the chunks.
-__global__ void __launch_bounds__(1024) k_suffix_min_i64(int64_t* p, int64_t n) {
-  __shared__ int64_t cm[1024];
-  const int t = threadIdx.x;
-  const int64_t per = (n + 1023) / 1024;
-  const int64_t b = min(n, t * per), e = min(n, b + per);
+// p[i] = min(p[i..n-1]), blocks of `per` entries: first each block's minimum,
+// then each block's suffix minima on top of the later blocks' (one block over
+// 140,609 column starts took 139 us).
+constexpr int kSuffixBlocks = 512;  // scratch entries (a radix histogram holds as many)
+__global__ void __launch_bounds__(256)
+k_block_min_i64(const int64_t* __restrict__ p, int64_t n, int64_t per, int64_t* __restrict__ bm) {
+  __shared__ int64_t wm[8];
+  const int64_t b = (int64_t)blockIdx.x * per, e = min(n, b + per);
   int64_t m = INT64_MAX;
-  for (int64_t i = e - 1; i >= b; i--) m = min(m, p[i]);
-  cm[t] = m;
+  for (int64_t i = b + threadIdx.x; i < e; i += 256) m = min(m, p[i]);
+  for (int o = 16; o > 0; o >>= 1) m = min(m, (int64_t)__shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
   __syncthreads();
-  for (int o = 1; o < 1024; o <<= 1) {
-    const int64_t v = t + o < 1024 ? cm[t + o] : INT64_MAX;
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < 8; k++) m = min(m, wm[k]);
+    bm[blockIdx.x] = m;
+  }
+}
+
+__global__ void __launch_bounds__(256)
+k_suffix_min_i64(int64_t* p, int64_t n, int64_t per, const int64_t* __restrict__ bm) {
+  __shared__ int64_t wm[8];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  // the later blocks' minimum
+  int64_t after = INT64_MAX;
+  for (int k = blockIdx.x + 1 + threadIdx.x; k < (int)gridDim.x; k += 256) after = min(after, bm[k]);
+  for (int o = 16; o > 0; o >>= 1)
+    after = min(after, (int64_t)__shfl_xor_sync(0xffffffffu, after, o));
+  if (lane == 0) wm[w] = after;
+  __syncthreads();
+  for (int k = 0; k < 8; k++) after = min(after, wm[k]);
+  __syncthreads();
+  // the block's entries, 256 at a time from its end
+  const int64_t b = (int64_t)blockIdx.x * per, e = min(n, b + per);
+  for (int64_t t0 = e; t0 > b; t0 -= 256) {
+    const int64_t i = t0 - 1 - threadIdx.x;  // thread order = from the end
+    int64_t m = i >= b ? p[i] : INT64_MAX;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t u = __shfl_up_sync(0xffffffffu, m, o);
+      if (lane >= o) m = min(m, u);
+    }
+    if (lane == 31) wm[w] = m;
     __syncthreads();
-    cm[t] = min(cm[t], v);
+    for (int k = 0; k < w; k++) m = min(m, wm[k]);
+    m = min(m, after);
+    if (i >= b) p[i] = m;
+    for (int k = 0; k < 8; k++) after = min(after, wm[k]);
     __syncthreads();
   }
-  int64_t run = t + 1 < 1024 ? cm[t + 1] : INT64_MAX;
-  for (int64_t i = e - 1; i >= b; i--) {
-    run = min(run, p[i]);
-    p[i] = run;
+}
+
+static epet_status suffix_min(int64_t* p, int64_t n, int64_t* scratch, cudaStream_t st) {
+  const int64_t per = std::max<int64_t>(1024, (n + kSuffixBlocks - 1) / kSuffixBlocks);
+  const unsigned nb = (unsigned)((n + per - 1) / per);
+  k_block_min_i64<<<nb, 256, 0, st>>>(p, n, per, scratch);
+  EPET_LAUNCHED();
+  k_suffix_min_i64<<<nb, 256, 0, st>>>(p, n, per, scratch);
+  EPET_LAUNCHED();
+  return EPET_OK;
+}
+
+template <int BITS>
+static epet_status coo_passes(const CooIn& in, const CooOut& out, int64_t n, int bits,
+                              uint64_t* keys[2], uint32_t* vals[2], int64_t* hist,
+                              int64_t* hist_scan, cudaStream_t st) {
+  using Pairs = ArrOut<uint64_t, uint32_t>;
+  using From = ArrIn<uint64_t, uint32_t>;
+  const int passes = (bits + BITS - 1) / BITS;
+  EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(in, Pairs{keys[0], vals[0]}, n, 0, hist,
+                                                   hist_scan, nullptr, st)));
+  if (passes == 1) {
+    k_unpack_coo<<<ceil_div(n, 256), 256, 0, st>>>(keys[0], vals[0], n, out.colbits, out.row,
+                                                   out.col, out.v);
+    EPET_LAUNCHED();
+    return EPET_OK;
   }
+  for (int p = 1; p < passes; p++) {
+    const From src{keys[(p - 1) & 1], vals[(p - 1) & 1]};
+    if (p + 1 < passes)
+      EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(src, Pairs{keys[p & 1], vals[p & 1]}, n,
+                                                       BITS * p, hist, hist_scan, nullptr, st)));
+    else
+      EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(src, out, n, BITS * p, hist, hist_scan,
+                                                       nullptr, st)));
+  }
+  return EPET_OK;
 }
 
 }  // namespace epet
@@ -582,27 +677,27 @@ epet_status epet_coo_sort(float* val_d, int32_t* row_d, int32_t* col_d, int64_t 
   int* mx = scr.take<int>(4);
   if (scr.overrun) return set_error(EPET_ERR_INVALID, "internal: workspace size");
   // index ranges (ids must be non-negative)
-  int h_mx[2] = {0, 0}, h_mn[2] = {0, 0};
   EPET_CUDA(cudaMemsetAsync(mx, 0, 16, st));
-  k_max2<<<std::min(ceil_div(n, 256), 1024), 256, 0, st>>>(row_d, col_d, n, mx);
+  k_range2<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 8 * (int64_t)num_sms()), 256, 0, st>>>(
+      row_d, col_d, n, mx);
   EPET_LAUNCHED();
-  k_min2<<<std::min(ceil_div(n, 256), 1024), 256, 0, st>>>(row_d, col_d, n, mx + 2);
-  EPET_LAUNCHED();
-  EPET_CUDA(cudaMemcpyAsync(h_mx, mx, 8, cudaMemcpyDeviceToHost, st));
-  EPET_CUDA(cudaMemcpyAsync(h_mn, mx + 2, 8, cudaMemcpyDeviceToHost, st));
+  int h_rng[4] = {0, 0, 0, 0};
+  EPET_CUDA(cudaMemcpyAsync(h_rng, mx, 16, cudaMemcpyDeviceToHost, st));
   EPET_CUDA(cudaStreamSynchronize(st));
-  if (h_mn[0] < 0 || h_mn[1] < 0)
+  if (h_rng[2] < 0 || h_rng[3] < 0)
     return set_error(EPET_ERR_INVALID, "negative row/column index");
-  const int colbits = std::max(1, bits_for(h_mx[1]));
-  const int rowbits = std::max(1, bits_for(h_mx[0]));
-  const int T = 256;
-  k_pack_coo<<<ceil_div(n, T), T, 0, st>>>(row_d, col_d, val_d, n, colbits, key, v);
-  EPET_LAUNCHED();
-  EPET_CHECK((radix_sort<uint64_t, uint32_t>(key, v, key2, v2, n, colbits + rowbits, hist,
-                                             hist_scan, tmp, st)));
-  k_unpack_coo<<<ceil_div(n, T), T, 0, st>>>(key, v, n, colbits, row_d, col_d, val_d);
-  EPET_LAUNCHED();
-  return EPET_OK;
+  const int colbits = std::max(1, bits_for(h_rng[1]));
+  const int rowbits = std::max(1, bits_for(h_rng[0]));
+  (void)tmp;
+  // 8-bit digits, or 9-bit ones where they save a pass
+  const int bits = colbits + rowbits;
+  uint64_t* keys[2] = {key, key2};
+  uint32_t* vals[2] = {v, v2};
+  const CooIn in{row_d, col_d, val_d, colbits};
+  const CooOut out{row_d, col_d, val_d, colbits};
+  if ((bits + 8) / 9 < (bits + 7) / 8)
+    return coo_passes<9>(in, out, n, bits, keys, vals, hist, hist_scan, st);
+  return coo_passes<8>(in, out, n, bits, keys, vals, hist, hist_scan, st);
 }
 
 epet_status epet_coo2csr(const int32_t* row_d, int64_t nnz, int64_t m, int64_t* csr_d,
@@ -711,9 +806,7 @@ static epet_status csr_to_csc_impl(const epet_csr* a, epet_csc* out, void* ws, s
     }
   }
   // empty columns start where the next non-empty one does
-  k_suffix_min_i64<<<1, 1024, 0, st>>>(out->col_ptr, a->n + 1);
-  EPET_LAUNCHED();
-  return EPET_OK;
+  return suffix_min(out->col_ptr, a->n + 1, hist, st);
 }
 
 epet_status csr_to_csc_positions(int64_t nnz, int64_t n, const int32_t* col, int64_t* col_ptr,
@@ -766,9 +859,7 @@ epet_status csr_to_csc_positions(int64_t nnz, int64_t n, const int32_t* col, int
         EPET_CHECK((radix_pass<9, K, V>(src, co, nnz, 9 * k, hist, hist_scan, tmp, st)));
     }
   }
-  k_suffix_min_i64<<<1, 1024, 0, st>>>(col_ptr, n + 1);
-  EPET_LAUNCHED();
-  return EPET_OK;
+  return suffix_min(col_ptr, n + 1, hist, st);
 }
 }  // namespace epet
 
