@@ -94,6 +94,7 @@ SIGNATURES = {
     "epet_csr16_count": [C.POINTER(CsrC), VP, C.POINTER(C.c_int64), VP],
     "epet_csr_compress": [C.POINTER(CsrC), I32, C.POINTER(Csr16C), VP],
     "epet_csr16_mv": [C.POINTER(Csr16C), F, VP, F, VP, VP],
+    "epet_csrmv2": [C.c_int, C.POINTER(CsrC), C.POINTER(CscC), F, VP, F, VP, VP, VP],
     "epet_csrmv": [C.c_int, C.POINTER(CsrC), C.POINTER(CscC), F, VP, F, VP, VP],
     "epet_divides": [VP, VP, VP, I64, VP],
     "epet_divides_multiplies": [VP, VP, VP, VP, I64, VP],

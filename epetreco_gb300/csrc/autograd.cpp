@@ -50,7 +50,15 @@ torch::Tensor apply_stored(const Stored& S, const torch::Tensor& x, bool trans) 
   auto y = torch::empty({x2.size(0), out}, x2.options());
   epet_csr a = S.csr();
   epet_csc c = S.csc();
-  for (int64_t b = 0; b < x2.size(0); b++)
+  // two vectors at a time, stored pairwise, so that the matrix is read once
+  // for both (same bits as one at a time)
+  int64_t b = 0;
+  for (; b + 1 < x2.size(0); b += 2) {
+    auto pair = x2.slice(0, b, b + 2).t().contiguous();
+    check(epet_csrmv2(trans ? 1 : 0, &a, &c, 1.f, pair.data_ptr<float>(), 0.f,
+                      y[b].data_ptr<float>(), y[b + 1].data_ptr<float>(), stream()));
+  }
+  if (b < x2.size(0))
     check(epet_csrmv(trans ? 1 : 0, &a, &c, 1.f, x2[b].data_ptr<float>(), 0.f,
                      y[b].data_ptr<float>(), stream()));
   auto shape = x.sizes().vec();

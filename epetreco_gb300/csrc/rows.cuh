@@ -119,6 +119,123 @@ __device__ __forceinline__ float group_dot_vec(const int32_t* __restrict__ idx,
   return a;
 }
 
+// The dot products of one row with two vectors stored pairwise (x[c] = both
+// vectors' element c), the matrix read once: the same additions in the same
+// order as the single-vector forms above, so both results have the same bits.
+template <int G>
+__device__ __forceinline__ float2 group_dot2_scalar(const int32_t* __restrict__ idx,
+                                                    const float* __restrict__ val,
+                                                    const float2* __restrict__ x, int64_t beg,
+                                                    int64_t end, int lg) {
+  float a[4] = {}, b[4] = {};
+  int64_t k = beg + lg;
+  for (; k + 3 * G < end; k += 4 * G) {
+    float v[4];
+    int c[4];
+    float2 q[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] = ld_stream(val + k + i * G);
+#pragma unroll
+    for (int i = 0; i < 4; i++) c[i] = ld_stream(idx + k + i * G);
+#pragma unroll
+    for (int i = 0; i < 4; i++) q[i] = __ldg(x + c[i]);
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      a[i] = fmaf(v[i], q[i].x, a[i]);
+      b[i] = fmaf(v[i], q[i].y, b[i]);
+    }
+  }
+  for (; k < end; k += G) {
+    const float v = ld_stream(val + k);
+    const float2 q = __ldg(x + ld_stream(idx + k));
+    a[0] = fmaf(v, q.x, a[0]);
+    b[0] = fmaf(v, q.y, b[0]);
+  }
+  float2 d = make_float2((a[0] + a[1]) + (a[2] + a[3]), (b[0] + b[1]) + (b[2] + b[3]));
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    d.x += __shfl_xor_sync(0xffffffffu, d.x, o, G);
+    d.y += __shfl_xor_sync(0xffffffffu, d.y, o, G);
+  }
+  return d;
+}
+
+template <int G, int U>
+__device__ __forceinline__ float2 group_dot2_vec(const int32_t* __restrict__ idx,
+                                                 const float* __restrict__ val,
+                                                 const float2* __restrict__ x, int64_t beg,
+                                                 int64_t end, int lg) {
+  const int64_t h = min(end, (beg + 3) & ~int64_t(3));
+  const int64_t t = max(h, end & ~int64_t(3));
+  float a[U] = {}, b[U] = {};
+  if (lg < h - beg) {
+    const float v = ld_stream(val + beg + lg);
+    const float2 q = __ldg(x + ld_stream(idx + beg + lg));
+    a[0] = v * q.x;
+    b[0] = v * q.y;
+  }
+  if (lg < end - t) {
+    const float v = ld_stream(val + t + lg);
+    const float2 q = __ldg(x + ld_stream(idx + t + lg));
+    a[U - 1] = fmaf(v, q.x, a[U - 1]);
+    b[U - 1] = fmaf(v, q.y, b[U - 1]);
+  }
+  const float4* __restrict__ v4 = reinterpret_cast<const float4*>(val + h);
+  const int4* __restrict__ c4 = reinterpret_cast<const int4*>(idx + h);
+  const int64_t nc = (t - h) >> 2;
+  float4 v[U];
+  int4 c[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int64_t jj = lg + u * G;
+    if (jj < nc) {
+      v[u] = __ldcs(v4 + jj);
+      c[u] = __ldcs(c4 + jj);
+    }
+  }
+  for (int64_t j = lg; j < nc; j += U * G) {
+    float4 vn[U];
+    int4 cn[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int64_t jj = j + (U + u) * G;
+      if (jj < nc) {
+        vn[u] = __ldcs(v4 + jj);
+        cn[u] = __ldcs(c4 + jj);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (j + u * G < nc) {
+        const float2 q0 = __ldg(x + c[u].x), q1 = __ldg(x + c[u].y);
+        const float2 q2 = __ldg(x + c[u].z), q3 = __ldg(x + c[u].w);
+        a[u] = fmaf(v[u].x, q0.x, a[u]);
+        b[u] = fmaf(v[u].x, q0.y, b[u]);
+        a[u] = fmaf(v[u].y, q1.x, a[u]);
+        b[u] = fmaf(v[u].y, q1.y, b[u]);
+        a[u] = fmaf(v[u].z, q2.x, a[u]);
+        b[u] = fmaf(v[u].z, q2.y, b[u]);
+        a[u] = fmaf(v[u].w, q3.x, a[u]);
+        b[u] = fmaf(v[u].w, q3.y, b[u]);
+      }
+      v[u] = vn[u];
+      c[u] = cn[u];
+    }
+  }
+  float2 d = make_float2(a[0], b[0]);
+#pragma unroll
+  for (int u = 1; u < U; u++) {
+    d.x += a[u];
+    d.y += b[u];
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) {
+    d.x += __shfl_xor_sync(0xffffffffu, d.x, o, G);
+    d.y += __shfl_xor_sync(0xffffffffu, d.y, o, G);
+  }
+  return d;
+}
+
 // The same sums with every value 1 (no value stream): sum of x over the
 // row's indices, in the same order as the dot products above (a product by
 // 1 is exact, so the results equal theirs).

@@ -65,6 +65,28 @@ k_sums(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
   }
 }
 
+// y0, y1 = alpha A x + beta y for two vectors stored pairwise.
+template <int G, int U, bool VEC>
+__global__ void __launch_bounds__(kSpmvThreads)
+k_rows_pair(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
+            const float* __restrict__ val, const float2* __restrict__ x, int64_t nrows,
+            float alpha, float beta, float* __restrict__ y0, float* __restrict__ y1) {
+  constexpr int RPT = kSpmvThreads / G;
+  const int lg = threadIdx.x % G;
+  const int64_t ntiles = (nrows + RPT - 1) / RPT;
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const int64_t row = tile * RPT + threadIdx.x / G;
+    if (row >= nrows) continue;
+    float2 d;
+    if constexpr (VEC) d = group_dot2_vec<G, U>(idx, val, x, ptr[row], ptr[row + 1], lg);
+    else d = group_dot2_scalar<G>(idx, val, x, ptr[row], ptr[row + 1], lg);
+    if (lg == 0) {
+      y0[row] = beta == 0.f ? alpha * d.x : alpha * d.x + beta * y0[row];
+      y1[row] = beta == 0.f ? alpha * d.y : alpha * d.y + beta * y1[row];
+    }
+  }
+}
+
 // Fixed-order sum of the block partials.
 __global__ void k_sum_partials(const double* __restrict__ p, int64_t n, double* out) {
   __shared__ double red[32];
@@ -364,6 +386,34 @@ epet_status epet_csrmv(int trans, const epet_csr* a, const epet_csc* csc, float 
                                                                a->m, alpha, y_d);
     EPET_LAUNCHED();
   }
+  return EPET_OK;
+}
+
+epet_status epet_csrmv2(int trans, const epet_csr* a, const epet_csc* csc, float alpha,
+                        const float* x_d, float beta, float* y0_d, float* y1_d,
+                        epet_stream_t stream) {
+  if (!a || (trans && !csc)) return set_error(EPET_ERR_INVALID, "bad arguments");
+  const int64_t out_len = trans ? a->n : a->m, in_len = trans ? a->m : a->n;
+  if ((out_len > 0 && (!y0_d || !y1_d)) || (in_len > 0 && !x_d) ||
+      (reinterpret_cast<uintptr_t>(x_d) & 7) != 0)
+    return set_error(EPET_ERR_INVALID, "bad arguments");
+  const int64_t* ptr = trans ? csc->col_ptr : a->row_ptr;
+  const int32_t* idx = trans ? csc->row : a->col;
+  const float* val = trans ? csc->val : a->val;
+  const int64_t nrows = trans ? csc->n : a->m, ncols = trans ? csc->m : a->n;
+  if (nrows <= 0) return EPET_OK;
+  cudaStream_t st = (cudaStream_t)stream;
+  RowPlan pl;  // (tuned on the first elements of x_d as one vector)
+  EPET_CHECK(dropin_plan(trans ? 3 : 2, ptr, idx, val, x_d, nrows, trans ? csc->nnz : a->nnz, ncols,
+                         st, &pl));
+  const int64_t nt = plan_tiles(pl, nrows);
+  const unsigned grid = (unsigned)(pl.grid > 0 ? std::min<int64_t>(nt, pl.grid) : nt);
+  dispatch_plan(pl, aligned16(idx, val), [&](auto g, auto u, auto v) {
+    k_rows_pair<decltype(g)::value, decltype(u)::value, decltype(v)::value>
+        <<<grid, kSpmvThreads, 0, st>>>(ptr, idx, val, reinterpret_cast<const float2*>(x_d), nrows,
+                                        alpha, beta, y0_d, y1_d);
+  });
+  EPET_LAUNCHED();
   return EPET_OK;
 }
 

@@ -309,6 +309,14 @@ epet_status epet_csrmv(int trans, const epet_csr* a, const epet_csc* csc,
                        float alpha, const float* x_d, float beta, float* y_d,
                        epet_stream_t stream);
 
+/* The same for two vectors at once, stored pairwise (x_d[2 i + k] = element i
+ * of vector k, 8-byte aligned), into y0_d and y1_d: the matrix is read once,
+ * and each result has the bits of its own epet_csrmv (same launch shape).  The
+ * transpose needs the CSC. */
+epet_status epet_csrmv2(int trans, const epet_csr* a, const epet_csc* csc,
+                        float alpha, const float* x_d, float beta, float* y0_d,
+                        float* y1_d, epet_stream_t stream);
+
 /* 16-bit layout: per-row stored-entry counts (row_len16_d[m]) and their
  * total. */
 epet_status epet_csr16_count(const epet_csr* a, int64_t* row_len16_d,
