@@ -96,25 +96,82 @@ __global__ void __launch_bounds__(128) k_uniforms(Geo G, const int32_t* __restri
 // state advanced c subsequences, so this yields the same states while a
 // typical step (consecutive channel ids) applies one jump matrix instead of
 // one per set bit of the channel id.
-constexpr int kRaysPerThread = 4;
-__global__ void __launch_bounds__(128) k_rays(Geo G, const int32_t* __restrict__ rows,
-                                              int64_t m, float* __restrict__ out) {
-  const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * kRaysPerThread;
-  if (i0 >= m) return;
+//
+// A thread's own stores would be 16 bytes into 32 rows at a time, half a
+// sector each; a warp stages kStageRays rays of its 32 rows in shared memory
+// and writes each row's share as one run of whole sectors (rows of an even
+// number of rays on 16-byte boundaries; others keep the thread's own stores).
+// 395,460 rows of 100 rays: 0.88 -> 0.66 ms.
+constexpr int kRaysPerThread = 4, kRaysThreads = 128;
+constexpr int kStageRays = 8, kStageVec = kStageRays * 24 / 16;  // rays and 16-byte pieces a row
+__global__ void __launch_bounds__(kRaysThreads)
+k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ out) {
+  // (a row of 13 pieces: the lanes' 16-byte stores fall in distinct banks)
+  __shared__ float4 stage[kRaysThreads / 32][32][kStageVec + 1];
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t i0 = t * kRaysPerThread;
   const int64_t i1 = i0 + kRaysPerThread < m ? i0 + kRaysPerThread : m;
   const bool regular = G.p.ray_mode == EPET_RAYS_REGULAR;
+  const int R = G.p.nrays;
   curandState base = {};
-  int prev = rows[i0];
-  if (!regular) curand_init(G.p.seed, (unsigned long long)prev, 0ull, &base);
-  for (int64_t i = i0; i < i1; i++) {
-    const int cnl = rows[i];
-    if (i > i0 && !regular) {
-      if (cnl > prev) skipahead_sequence((unsigned long long)(cnl - prev), &base);
-      else if (cnl != prev) curand_init(G.p.seed, (unsigned long long)cnl, 0ull, &base);
-      prev = cnl;
+  int prev = 0;
+  if (i0 < m) {
+    prev = rows[i0];
+    if (!regular) curand_init(G.p.seed, (unsigned long long)prev, 0ull, &base);
+  }
+  const bool staged = (R & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  const int lane = threadIdx.x & 31;
+  float4(*st)[kStageVec + 1] = stage[threadIdx.x >> 5];
+  for (int j = 0; j < kRaysPerThread; j++) {
+    const int64_t i = i0 + j;
+    const bool live = i < i1;
+    int cnl = 0;
+    if (live) {
+      cnl = rows[i];
+      if (j > 0 && !regular) {
+        if (cnl > prev) skipahead_sequence((unsigned long long)(cnl - prev), &base);
+        else if (cnl != prev) curand_init(G.p.seed, (unsigned long long)cnl, 0ull, &base);
+        prev = cnl;
+      }
     }
-    emit_rays(G, cnl, base, false,
-              reinterpret_cast<float2*>(out + i * (int64_t)G.p.nrays * 6));
+    if (!staged) {
+      if (live) emit_rays(G, cnl, base, false, reinterpret_cast<float2*>(out + i * (int64_t)R * 6));
+      continue;
+    }
+    curandState state = base;
+    int id[5];
+    channel_decode(G.p.setup, cnl, id);
+    float sn, cs;
+    angle_sincos(G.p.setup, id[0], &sn, &cs);
+    const CrystalMat m0 = crystal_matrix(G.p.setup, sn, cs, 0, id[1], id[2]);
+    const CrystalMat m1 = crystal_matrix(G.p.setup, sn, cs, 1, id[3], id[4]);
+    const int64_t row0 = (t - lane) * kRaysPerThread + j;  // lane r's row: row0 + r kRaysPerThread
+    for (int r0 = 0; r0 < R; r0 += kStageRays) {
+      const int nr = min(kStageRays, R - r0);  // even
+#pragma unroll 1
+      for (int r = 0; r < nr; r += 2) {
+        float u[6], w[12];
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+          draw6(state, regular, u);
+          crystal_apply(m0, u[0], u[1], u[2], w + 6 * k);
+          crystal_apply(m1, u[3], u[4], u[5], w + 6 * k + 3);
+        }
+        float4* q = &st[lane][r * 3 / 2];
+        q[0] = make_float4(w[0], w[1], w[2], w[3]);
+        q[1] = make_float4(w[4], w[5], w[6], w[7]);
+        q[2] = make_float4(w[8], w[9], w[10], w[11]);
+      }
+      __syncwarp();
+      const int nv = nr * 3 / 2;  // pieces of a row
+      for (int k = lane; k < 32 * nv; k += 32) {
+        const int r = nv == kStageVec ? k / kStageVec : k / nv, c = k - r * nv;
+        const int64_t row = row0 + (int64_t)r * kRaysPerThread;
+        if (row < m)
+          reinterpret_cast<float4*>(out + (row * R + r0) * 6)[c] = st[r][c];
+      }
+      __syncwarp();
+    }
   }
 }
 
@@ -180,7 +237,7 @@ epet_status launch_rays(const Geo& G, const int32_t* rows, int64_t m, float* out
   if (uniforms_only)
     k_uniforms<<<ceil_div(m, T), T, 0, st>>>(G, rows, m, out);
   else
-    k_rays<<<ceil_div(ceil_div(m, kRaysPerThread), T), T, 0, st>>>(G, rows, m, out);
+    k_rays<<<ceil_div(ceil_div(m, kRaysPerThread), kRaysThreads), kRaysThreads, 0, st>>>(G, rows, m, out);
   EPET_LAUNCHED();
   return EPET_OK;
 }
