@@ -521,7 +521,7 @@ class Mlem:
 
 class MlemBatch:
     """Many independent reconstructions iterated together: each step of an
-    iteration is one launch over all problems, the iteration one CUDA graph.
+    iteration runs over all problems together, the iteration one CUDA graph.
     ``problems`` is a list of (Problem, rows, y, s) with device tensors."""
 
     def __init__(self, problems, use_graph: bool = True, autotune: bool = True,

@@ -3,11 +3,12 @@
 // Each problem is an ordinary epet_mlem (its own matrix, CSC copy, counts,
 // sensitivity and image, all in separate allocations).  The batch adds a
 // device array of per-problem descriptors and tile tables, and runs every
-// step of an iteration as ONE launch over all problems: a tile of rows (or
+// step of an iteration as one launch over all problems: a tile of rows (or
 // voxels) finds its problem by binary search in the tile table, then works
-// on that problem's arrays.  The four launches of an iteration (five with
-// wide row groups) are captured
-// in one CUDA graph.  Partial image sums are written per tile; a problem's
+// on that problem's arrays.  The grouped layout's pass takes a launch per
+// launch shape and one for each problem that fills the device by itself
+// (grouped_batch_order), and one for wide row groups.  An iteration's launches
+// are captured in one CUDA graph.  Partial image sums are written per tile; a problem's
 // tiles are contiguous, so its image sum is a fixed-order sum over its own
 // tile range (deterministic, as in the single-problem driver).
 #include <algorithm>
@@ -127,7 +128,8 @@ struct epet_mlem_batch {
   bool grouped = false;
   void* gdesc = nullptr;      // device, nprob descriptors of the pass
   int64_t* gstart = nullptr;  // device, prefix of the problems' group counts
-  BatchGroups total;
+  std::vector<BatchRun> runs;        // the pass's launches
+  std::vector<unsigned char> gdesc_h;  // host copy of gdesc
   int32_t* gwide = nullptr;   // device, global ids of the wide groups
   int64_t nwide = 0;
   int graph_kernels = 0;      // kernels in the captured iteration
@@ -176,8 +178,8 @@ epet_status launch_batch_rows(const epet_mlem_batch* h, const RowPlan& plan, boo
 
 epet_status batch_iteration(const epet_mlem_batch* h, cudaStream_t st) {
   if (h->grouped)
-    EPET_CHECK(grouped_pass_batch(h->gdesc, h->gstart, h->np(), h->total, h->gwide,
-                                  h->nwide, st));
+    EPET_CHECK(grouped_pass_batch(h->gdesc, h->gdesc_h.data(), h->gstart, h->np(), h->runs,
+                                  h->gwide, h->nwide, st));
   else
     EPET_CHECK(launch_batch_rows(h, h->plan_fwd, true, st));
   EPET_CHECK(launch_batch_rows(h, h->plan_bwd, false, st));
@@ -220,8 +222,8 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
   };
   epet_mlem_options po = o;  // members iterated alone: graph as asked, heuristic shapes
   po.autotune = 0;
-  // every member in the grouped layout where all support it (6 bytes per
-  // entry), else every member with its CSR and column-major copy
+  // every member in the grouped layout where all support it (strips of
+  // merged rows), else every member with its CSR and column-major copy
   bool all_grouped = o.layout != EPET_LAYOUT_CSC;
   for (int i = 0; i < nprob && all_grouped; i++) {
     const epet_grid& g = problems[i].grid;
@@ -244,9 +246,24 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
   std::vector<BatchDesc> dh(np);
   h->tiles_h.assign(9 * (np + 1), 0);
   h->grouped = all_grouped;
-  std::vector<unsigned char> gd_h(all_grouped ? np * grouped_batch_desc_bytes() : 0);
   std::vector<int64_t> gs_h(np + 1, 0);
   std::vector<int32_t> gw_h;  // global ids of the wide groups
+  if (all_grouped) {
+    // the pass's descriptors and group ids in the order of its launches
+    std::vector<const GroupedMatrix*> gm;
+    for (const epet_mlem* p : h->probs) gm.push_back(&p->G);
+    const std::vector<int> order = grouped_batch_order(gm, &h->runs);
+    h->gdesc_h.resize(np * grouped_batch_desc_bytes());
+    for (int k = 0; k < np; k++) {
+      const epet_mlem* p = h->probs[order[k]];
+      grouped_batch_desc(p->G, p->x, p->y, p->ybar,
+                         h->gdesc_h.data() + k * grouped_batch_desc_bytes());
+      gs_h[k + 1] = gs_h[k] + p->G.ngroups;
+      if (gs_h[k + 1] > INT32_MAX)
+        return fail(set_error(EPET_ERR_UNSUPPORTED, "batch: more than 2^31 row groups"));
+      for (int32_t w : p->G.wide_h) gw_h.push_back((int32_t)(gs_h[k] + w));
+    }
+  }
   for (int i = 0; i < np; i++) {
     epet_mlem* p = h->probs[i];
     if (all_grouped) {
@@ -256,9 +273,6 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
       if (rc != EPET_OK) return fail(rc);
       dh[i] = BatchDesc{nullptr, nullptr, nullptr, p->G.cg_ptr, p->G.cg_slot, p->G.ones,
                         p->y, p->G.partial, p->ybar, p->s, p->x, p->xnew, p->m, p->V};
-      grouped_batch_desc(p->G, p->x, p->y, p->ybar, gd_h.data() + i * grouped_batch_desc_bytes());
-      for (int32_t w : p->G.wide_h) gw_h.push_back((int32_t)(gs_h[i] + w));
-      gs_h[i + 1] = gs_h[i] + p->G.ngroups;
       if (!aligned16(p->G.cg_slot, p->G.ones))
         return fail(set_error(EPET_ERR_UNSUPPORTED, "batch: slot streams not 16-byte aligned"));
     } else {
@@ -287,16 +301,8 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
   ALLOC(h->partial, std::max<int64_t>(h->host_total(4), 1) * 8);  // 8 rows per tile: most
   ALLOC(h->sums, np * 8);
   if (all_grouped) {
-    ALLOC(h->gdesc, gd_h.size());
+    ALLOC(h->gdesc, h->gdesc_h.size());
     ALLOC(h->gstart, (np + 1) * 8);
-    for (const epet_mlem* p : h->probs) {
-      h->total.groups += p->G.ngroups;
-      h->total.strips += p->G.nstrips;
-      h->total.entries += p->G.nent;
-      h->total.max_nd = std::max(h->total.max_nd, p->G.max_nd);
-    }
-    if (h->total.groups > INT32_MAX)
-      return fail(set_error(EPET_ERR_UNSUPPORTED, "batch: more than 2^31 row groups"));
     h->nwide = (int64_t)gw_h.size();
     if (h->nwide > 0) ALLOC(h->gwide, h->nwide * 4);
   }
@@ -307,7 +313,7 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
     e = cudaMemcpyAsync(h->tiles, h->tiles_h.data(), h->tiles_h.size() * 8,
                         cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && all_grouped)
-    e = cudaMemcpyAsync(h->gdesc, gd_h.data(), gd_h.size(), cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(h->gdesc, h->gdesc_h.data(), h->gdesc_h.size(), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && all_grouped)
     e = cudaMemcpyAsync(h->gstart, gs_h.data(), (np + 1) * 8, cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess && h->nwide > 0)
@@ -328,8 +334,8 @@ epet_status epet_mlem_batch_create(int32_t nprob, const epet_problem* problems,
       // one pass fills the slots (unless the plan is cached); the slot
       // sums' candidates rerun the (idempotent) update epilogue
       if (!tune_lookup(7, h->voxels, nslots, np, &h->plan_bwd))
-        rc = grouped_pass_batch(h->gdesc, h->gstart, np, h->total, h->gwide, h->nwide,
-                                st);
+        rc = grouped_pass_batch(h->gdesc, h->gdesc_h.data(), h->gstart, np, h->runs, h->gwide,
+                                h->nwide, st);
       if (rc == EPET_OK)
         rc = tune_rows(
             7, h->voxels, nslots, np, avg_col,

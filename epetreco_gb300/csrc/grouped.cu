@@ -4,12 +4,12 @@
 // The rows (in the reconstruction's crystal-pair order) are cut into groups
 // of consecutive rows whose distinct columns fit a per-warp table in shared
 // memory.  Consecutive rows in that order are a fan of lines through nearly
-// one point, so a group touches few voxels, and four consecutive rows (a
+// one point, so a group touches few voxels, and two consecutive rows (a
 // strip) touch few more than one of them.  A strip is stored as the merged list
-// of its rows' columns: per entry the four rows' values (zero where a row
+// of its rows' columns: per entry the two rows' values (zero where a row
 // does not touch the column) and a 2-byte rank of the column among the
-// group's sorted distinct columns (the group's table), 18 bytes in FP32 for
-// about 3 non-zeros and 10 in the 16-bit forms, instead of a CSR plus a
+// group's sorted distinct columns (the group's table), 10 bytes in FP32 and 6
+// in the 16-bit forms for about 1.7 non-zeros, instead of a CSR plus a
 // column-major copy (16 bytes per non-zero).
 //
 // One iteration reads every entry once (k_group_mlem): a warp takes a group,
@@ -870,7 +870,7 @@ k_group_mlem_batch(const GroupIterArgs* __restrict__ desc, const int64_t* __rest
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float* xs = gsm + (size_t)w * 2 * kStride;
   float* cs = xs + kStride;
-  const int64_t total = gstart[np];
+  const int64_t total = gstart[np];  // (gstart[0]: the groups of the runs before)
   const int64_t step = (int64_t)gridDim.x * WARPS;
   auto locate = [&](int64_t g) {  // gstart[lo] <= g < gstart[lo + 1]
     int lo = 0, hi = np;
@@ -881,7 +881,7 @@ k_group_mlem_batch(const GroupIterArgs* __restrict__ desc, const int64_t* __rest
     }
     return lo;
   };
-  int64_t g = (int64_t)blockIdx.x * WARPS + w;
+  int64_t g = gstart[0] + (int64_t)blockIdx.x * WARPS + w;
   if (g >= total) return;
   // the next group's problem and head loaded one group ahead
   int p = locate(g);
@@ -1343,17 +1343,60 @@ static unsigned pass_grid(int64_t ngroups, int warps) {
       1, std::min<int64_t>((ngroups + warps - 1) / warps, (int64_t)num_sms()));
 }
 
-epet_status grouped_pass_batch(const void* desc, const int64_t* gstart, int np,
-                               const BatchGroups& total, const int32_t* wide, int64_t nwide,
-                               cudaStream_t st) {
-  if (total.groups <= 0) return EPET_OK;
-  const PassShape s = pass_shape(total.entries, total.strips, total.max_nd);
-  dispatch_shape(s, [&](auto R, auto W) {
-    k_group_mlem_batch<decltype(R)::value, decltype(W)::value>
-        <<<pass_grid(total.groups, s.warps), s.warps * 32, s.smem(), st>>>(
-            static_cast<const GroupIterArgs*>(desc), gstart, np);
-  });
-  EPET_LAUNCHED();
+// The launches of a batch's pass: the problems of one launch shape together,
+// a problem with kAloneWaves groups or more for every warp of the device in a
+// launch of its own (it fills the device by itself, and its descriptor is then
+// a kernel parameter: in memory, its loads stand before every strip's).
+// Measured, 10 iterations: 64 problems of 24^3 to 64^3 and up to 5.1M rows, one
+// launch for all in the shape of the widest 691 ms, a launch a shape 654, alone
+// from 1, 4, 16 waves 578, 577, 579; 64 of 24^3 and 32^3, 8 angles: 66.9, 50.7,
+// and 56.8, 50.7, 50.7.
+constexpr int kAloneWaves = 4;
+
+std::vector<int> grouped_batch_order(const std::vector<const GroupedMatrix*>& G,
+                                     std::vector<BatchRun>* runs) {
+  runs->clear();
+  std::vector<int> order;
+  auto shape = [&](int i) { return pass_shape(G[i]->nent, G[i]->nstrips, G[i]->max_nd); };
+  auto alone = [&](int i) {
+    return G[i]->ngroups >= (int64_t)kAloneWaves * shape(i).warps * num_sms();
+  };
+  for (int rounds : {5, 3, 2}) {
+    BatchRun run{(int)order.size(), 0, 0, nullptr};
+    for (int i = 0; i < (int)G.size(); i++) {
+      if (G[i]->ngroups == 0 || alone(i) || shape(i).rounds != rounds) continue;
+      order.push_back(i);
+      run.np++;
+      run.groups += G[i]->ngroups;
+      run.rep = G[i];
+    }
+    if (run.np > 0) runs->push_back(run);
+  }
+  for (int i = 0; i < (int)G.size(); i++) {
+    if (G[i]->ngroups > 0 && !alone(i)) continue;  // (without groups: last, in no run)
+    if (G[i]->ngroups > 0) runs->push_back(BatchRun{(int)order.size(), 1, G[i]->ngroups, G[i]});
+    order.push_back(i);
+  }
+  return order;
+}
+
+epet_status grouped_pass_batch(const void* desc, const void* desc_h, const int64_t* gstart, int np,
+                               const std::vector<BatchRun>& runs, const int32_t* wide,
+                               int64_t nwide, cudaStream_t st) {
+  for (const BatchRun& run : runs) {
+    const PassShape s = pass_shape(run.rep->nent, run.rep->nstrips, run.rep->max_nd);
+    const unsigned grid = pass_grid(run.groups, s.warps), T = s.warps * 32;
+    dispatch_shape(s, [&](auto R, auto W) {
+      constexpr int rounds = decltype(R)::value, warps = decltype(W)::value;
+      if (run.np == 1)
+        k_group_mlem<0, rounds, warps><<<grid, T, s.smem(), st>>>(
+            static_cast<const GroupIterArgs*>(desc_h)[run.p0]);
+      else
+        k_group_mlem_batch<rounds, warps><<<grid, T, s.smem(), st>>>(
+            static_cast<const GroupIterArgs*>(desc) + run.p0, gstart + run.p0, run.np);
+    });
+    EPET_LAUNCHED();
+  }
   if (nwide > 0) {
     k_group_mlem_batch_wide<<<(unsigned)ceil_div(nwide * 32, (int64_t)128), 128, 0, st>>>(
         static_cast<const GroupIterArgs*>(desc), gstart, np, wide, nwide);

@@ -92,21 +92,26 @@ epet_status grouped_column_sums(const GroupedMatrix& G, bool quantised, float* o
                                 cudaStream_t st);
 // Batched form: a descriptor per problem (grouped_batch_desc_bytes() each,
 // written by grouped_batch_desc into a host buffer and copied to the
-// device) and one pass over all problems' groups (gstart: device prefix of
-// the problems' group counts, np + 1 entries; wide: the global ids of the
-// wide groups, nwide of them, passed by a second kernel).
+// device) and the pass over all problems' groups, in the order and the runs
+// that grouped_batch_order gives (gstart: device prefix of the problems'
+// group counts in that order, np + 1 entries; wide: the global ids of the
+// wide groups, nwide of them, passed by a kernel of their own).
 size_t grouped_batch_desc_bytes();
 void grouped_batch_desc(const GroupedMatrix& G, const float* x, const float* y, float* ybar,
                         void* out);
-// groups/strips/entries/columns: totals over the problems and the most columns
-// of any group (the launch shape's rule).
-struct BatchGroups {
-  int64_t groups = 0, strips = 0, entries = 0;
-  int max_nd = 0;
+// A launch of the pass: problems [p0, p0 + np) of the order, `groups` groups,
+// all of them with the launch shape of rep.
+struct BatchRun {
+  int p0, np;
+  int64_t groups;
+  const GroupedMatrix* rep;
 };
-epet_status grouped_pass_batch(const void* desc, const int64_t* gstart, int np,
-                               const BatchGroups& total, const int32_t* wide, int64_t nwide,
-                               cudaStream_t st);
+std::vector<int> grouped_batch_order(const std::vector<const GroupedMatrix*>& G,
+                                     std::vector<BatchRun>* runs);
+// desc_h: the descriptors' host copy.
+epet_status grouped_pass_batch(const void* desc, const void* desc_h, const int64_t* gstart, int np,
+                               const std::vector<BatchRun>& runs, const int32_t* wide,
+                               int64_t nwide, cudaStream_t st);
 }  // namespace epet
 
 struct epet_mlem {

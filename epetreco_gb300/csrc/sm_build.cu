@@ -17,8 +17,8 @@
 //    chord length is bit-identical to intersectionLength(); a voxel is never
 //    evaluated more than once per ray;
 //  * chords accumulate in a dense shared-memory window covering the ray
-//    bundle slab by slab along x (bounded by the 64 crystal-corner lines, an
-//    exact convex-hull bound), as 64-bit fixed-point integers: the sum is
+//    bundle slab by slab along x (bounded by lines between the crystals'
+//    corners, an exact convex-hull bound), as 64-bit fixed-point integers: the sum is
 //    exact and independent of the order of the atomic adds, so results are
 //    deterministic; it is rounded once to float.  Versus the reference's
 //    sequential fp32 sum the difference is below (nrays-1)*2^-24 relative;

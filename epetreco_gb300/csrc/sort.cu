@@ -4,9 +4,11 @@
 // The reference sorts COO triples with thrust's comparison sort_by_key
 // (cooSort.hpp:53-71, a merge sort) and converts with cusparseXcoo2csr
 // (cusparseWrapper.hpp:38-45) and a host loop of three synchronous copies per
-// row (convertCsr2Ecsr.hpp:34-47).  Here: an 8-bit-digit LSD radix sort on a
-// packed (row, col) key, stable within each tile by warp-ordered ranking
-// (__match_any_sync), a histogram+scan row pointer, and one gather kernel.
+// row (convertCsr2Ecsr.hpp:34-47).  Here: an LSD radix sort on a packed
+// (row, col) key (digits of 8 bits, or 9 where that saves a pass), stable
+// within each tile by warp-ordered ranking (ballots), reading the triples in
+// its first pass and writing them in its last; a histogram+scan row pointer,
+// and one gather kernel.
 #include <algorithm>
 #include <type_traits>
 #include <mutex>

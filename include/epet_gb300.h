@@ -470,10 +470,11 @@ epet_status epet_mlem_layout(const epet_mlem* h, int32_t* layout_h);
 /* ---------------------------------------------- batched reconstructions */
 /* Many independent reconstructions (each its own geometry, grid, rays,
  * measured rows and sensitivity) iterated together: every step of an
- * iteration is ONE kernel launch over all problems' rows or voxels, and the
+ * iteration runs over all problems' rows or voxels together, and the
  * iteration (forward product + e = y/(Ax), transpose product + x*c/s,
- * per-problem fp64 image sums, normalisation: four launches, five when a
- * grouped-layout problem has a row wider than the shared tables) is captured in
+ * per-problem fp64 image sums, normalisation: four launches, in the grouped
+ * layout more for problems of different row lengths or filling the device by
+ * themselves, and one for rows wider than the shared tables) is captured in
  * one CUDA graph.  Launch shapes come from the autotuner unless
  * opt->autotune == 0.  The reference runs one reconstruction per process
  * (reco.cu:209-281); there is no batched counterpart.  FP32 values. */

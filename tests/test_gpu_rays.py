@@ -1,0 +1,43 @@
+"""Endpoint rays at the edges of their staged stores, against the oracle bit
+for bit: ray counts around the staged run of 8 rays (odd ones are stored
+directly), row counts around a thread's 4 rows, a warp's and a block's share,
+and an output off a 16-byte boundary (8-byte aligned, as the entry point asks);
+the words before and after the output keep what they held."""
+import ctypes as C
+
+import numpy as np
+import pytest
+import torch
+
+from epetreco_gb300 import api
+from epetreco_gb300._lib import check, lib
+from epetreco_gb300.problem import Problem, VoxelGrid, two_head_setup
+
+pytestmark = pytest.mark.gpu
+
+GUARD = 64  # floats on either side of the output
+
+
+@pytest.mark.parametrize("shift", [0, 2])  # floats
+@pytest.mark.parametrize("nrays,m", [(1, 5), (2, 1), (6, 129), (7, 33), (8, 127), (10, 513),
+                                     (16, 4), (18, 128), (101, 3)])
+def test_rays_match_oracle_and_stay_inside(gpu_lib, oracle, nrays, m, shift):
+    p = Problem(two_head_setup(8, 45.0, n=5), VoxelGrid((-0.02,) * 3, (0.004,) * 3, (10,) * 3),
+                nrays)
+    rows = np.random.default_rng(nrays).integers(0, p.nchannels, m).astype(np.int32)
+    d = torch.from_numpy(rows).cuda()
+    n = m * nrays * 6
+    buf = torch.full((n + 2 * GUARD + shift,), -7.0, dtype=torch.float32, device="cuda")
+    out = buf[GUARD + shift:]
+    assert out.data_ptr() % 16 == 4 * shift
+    check(lib().epet_rays(C.byref(api.problem_struct(p)), C.c_void_p(d.data_ptr()), m,
+                          C.c_void_p(out.data_ptr()),
+                          C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    got = buf.cpu().numpy()
+    assert (got[:GUARD + shift] == -7.0).all() and (got[GUARD + shift + n:] == -7.0).all()
+    got = got[GUARD + shift:GUARD + shift + n].reshape(m, nrays, 6)
+    trig = api.trig_table(p).cpu().numpy()
+    rnd = api.dump_uniforms(p, d).cpu().numpy()
+    for i in range(m):
+        want = oracle.rays(p, rows[i], rnd[i], trig=trig)
+        assert (got[i].view(np.uint32) == np.asarray(want, np.float32).view(np.uint32)).all(), i
