@@ -42,6 +42,13 @@ struct Stored {
   }
 };
 
+// Non-zeros from which two vectors share a read of the matrix: at twice the
+// size of L2 a second read comes from memory, while below it what the pairs'
+// copies cost the host weighs more.  Forward and backward of two images, pairs
+// / singles: 28M non-zeros 435 / 414 us, 56M 436 / 436 (waited for after each:
+// 521 / 565), 112M 541 / 795; three images, 56M: 487 / 621.
+constexpr int64_t kPairNnz = int64_t(1) << 25;
+
 torch::Tensor apply_stored(const Stored& S, const torch::Tensor& x, bool trans) {
   const int64_t in = trans ? S.m : S.n, out = trans ? S.n : S.m;
   TORCH_CHECK(x.size(-1) == in, "projector: last dimension ", x.size(-1), " != ", in);
@@ -53,12 +60,12 @@ torch::Tensor apply_stored(const Stored& S, const torch::Tensor& x, bool trans) 
   // two vectors at a time, stored pairwise, so that the matrix is read once
   // for both (same bits as one at a time)
   int64_t b = 0;
-  for (; b + 1 < x2.size(0); b += 2) {
+  for (; S.col.numel() >= kPairNnz && b + 1 < x2.size(0); b += 2) {
     auto pair = x2.slice(0, b, b + 2).t().contiguous();
     check(epet_csrmv2(trans ? 1 : 0, &a, &c, 1.f, pair.data_ptr<float>(), 0.f,
                       y[b].data_ptr<float>(), y[b + 1].data_ptr<float>(), stream()));
   }
-  if (b < x2.size(0))
+  for (; b < x2.size(0); b++)
     check(epet_csrmv(trans ? 1 : 0, &a, &c, 1.f, x2[b].data_ptr<float>(), 0.f,
                      y[b].data_ptr<float>(), stream()));
   auto shape = x.sizes().vec();

@@ -63,3 +63,19 @@ def test_projector_batches(gpu_lib, batch):
     for k in range(batch):
         assert torch.equal(y[k], api.CSRmv(0, proj.A, x[k].detach()))
         assert torch.equal(grad[k], api.CSRmv(1, proj.A, w[k], At=proj.At))
+
+
+def test_projector_pairs_of_a_large_matrix(gpu_lib):
+    """Above the size from which the projector takes its vectors in pairs."""
+    from epetreco_gb300.autograd import Projector
+    from epetreco_gb300.problem import config
+    p = config("small")["problem"]
+    proj = Projector(p, torch.arange(p.nchannels, dtype=torch.int32, device="cuda"))
+    assert proj.A.nnz >= 1 << 25
+    x = torch.rand(3, p.nvoxels, device="cuda", requires_grad=True)
+    y = proj(x)
+    w = torch.rand_like(y)
+    (grad,) = torch.autograd.grad((y * w).sum(), x)
+    for k in range(3):
+        assert torch.equal(y[k], api.CSRmv(0, proj.A, x[k].detach()))
+        assert torch.equal(grad[k], api.CSRmv(1, proj.A, w[k], At=proj.At))
