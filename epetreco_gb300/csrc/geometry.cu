@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) k_uniforms(Geo G, const int32_t* __restri
             reinterpret_cast<float2*>(out + i * (int64_t)G.p.nrays * 6));
 }
 
-// World rays.  Thread t handles rows t*K .. t*K+K-1: the first channel's
+// World rays.  Thread t handles rows t*K .. t*K+K-1 (K = kPer): the first channel's
 // generator comes from curand_init, the next ones from the previous
 // channel's initial state advanced by the channel difference in
 // subsequences (skipahead_sequence): curand_init(seed, c, 0) is the seeded
@@ -102,15 +102,23 @@ __global__ void __launch_bounds__(128) k_uniforms(Geo G, const int32_t* __restri
 // and writes each row's share as one run of whole sectors (rows of an even
 // number of rays on 16-byte boundaries; others keep the thread's own stores).
 // 395,460 rows of 100 rays: 0.88 -> 0.66 ms.
+//
+// For few rows a thread has one row and stores its rays itself: the kernel is
+// then bound by the latency of a thread's own rows, and four of them in series
+// took 387 us for 3,000 rows of 20 rays and 451 of 90, against 149 and 162
+// (80,000 rows: 390 and 489 against 304 and 345; 160,000: 443 and 549 against
+// 494 and 566, when the generator's jumps and the stores weigh more).
 constexpr int kRaysPerThread = 4, kRaysThreads = 128;
+constexpr int kRaysThreadsFew = 64, kRaysFewPerSm = 800;
 constexpr int kStageRays = 8, kStageVec = kStageRays * 24 / 16;  // rays and 16-byte pieces a row
-__global__ void __launch_bounds__(kRaysThreads)
+template <int kPer, int kT, bool kStaged>
+__global__ void __launch_bounds__(kT)
 k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ out) {
   // (a row of 13 pieces: the lanes' 16-byte stores fall in distinct banks)
-  __shared__ float4 stage[kRaysThreads / 32][32][kStageVec + 1];
+  __shared__ float4 stage[kStaged ? kT / 32 : 1][32][kStageVec + 1];
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t i0 = t * kRaysPerThread;
-  const int64_t i1 = i0 + kRaysPerThread < m ? i0 + kRaysPerThread : m;
+  const int64_t i0 = t * kPer;
+  const int64_t i1 = i0 + kPer < m ? i0 + kPer : m;
   const bool regular = G.p.ray_mode == EPET_RAYS_REGULAR;
   const int R = G.p.nrays;
   curandState base = {};
@@ -119,10 +127,10 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
     prev = rows[i0];
     if (!regular) curand_init(G.p.seed, (unsigned long long)prev, 0ull, &base);
   }
-  const bool staged = (R & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+  const bool staged = kStaged && (R & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const int lane = threadIdx.x & 31;
-  float4(*st)[kStageVec + 1] = stage[threadIdx.x >> 5];
-  for (int j = 0; j < kRaysPerThread; j++) {
+  float4(*st)[kStageVec + 1] = stage[kStaged ? threadIdx.x >> 5 : 0];
+  for (int j = 0; j < kPer; j++) {
     const int64_t i = i0 + j;
     const bool live = i < i1;
     int cnl = 0;
@@ -145,7 +153,7 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
     angle_sincos(G.p.setup, id[0], &sn, &cs);
     const CrystalMat m0 = crystal_matrix(G.p.setup, sn, cs, 0, id[1], id[2]);
     const CrystalMat m1 = crystal_matrix(G.p.setup, sn, cs, 1, id[3], id[4]);
-    const int64_t row0 = (t - lane) * kRaysPerThread + j;  // lane r's row: row0 + r kRaysPerThread
+    const int64_t row0 = (t - lane) * kPer + j;  // lane r's row: row0 + r kPer
     for (int r0 = 0; r0 < R; r0 += kStageRays) {
       const int nr = min(kStageRays, R - r0);  // even
 #pragma unroll 1
@@ -166,7 +174,7 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
       const int nv = nr * 3 / 2;  // pieces of a row
       for (int k = lane; k < 32 * nv; k += 32) {
         const int r = nv == kStageVec ? k / kStageVec : k / nv, c = k - r * nv;
-        const int64_t row = row0 + (int64_t)r * kRaysPerThread;
+        const int64_t row = row0 + (int64_t)r * kPer;
         if (row < m)
           reinterpret_cast<float4*>(out + (row * R + r0) * 6)[c] = st[r][c];
       }
@@ -236,8 +244,13 @@ epet_status launch_rays(const Geo& G, const int32_t* rows, int64_t m, float* out
   const int T = 128;
   if (uniforms_only)
     k_uniforms<<<ceil_div(m, T), T, 0, st>>>(G, rows, m, out);
+  else if (m <= (int64_t)kRaysFewPerSm * num_sms())
+    k_rays<1, kRaysThreadsFew, false>
+        <<<ceil_div(m, kRaysThreadsFew), kRaysThreadsFew, 0, st>>>(G, rows, m, out);
   else
-    k_rays<<<ceil_div(ceil_div(m, kRaysPerThread), kRaysThreads), kRaysThreads, 0, st>>>(G, rows, m, out);
+    k_rays<kRaysPerThread, kRaysThreads, true>
+        <<<ceil_div(ceil_div(m, kRaysPerThread), kRaysThreads), kRaysThreads, 0, st>>>(G, rows, m,
+                                                                                      out);
   EPET_LAUNCHED();
   return EPET_OK;
 }

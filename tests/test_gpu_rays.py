@@ -41,3 +41,23 @@ def test_rays_match_oracle_and_stay_inside(gpu_lib, oracle, nrays, m, shift):
     for i in range(m):
         want = oracle.rays(p, rows[i], rnd[i], trig=trig)
         assert (got[i].view(np.uint32) == np.asarray(want, np.float32).view(np.uint32)).all(), i
+
+
+@pytest.mark.parametrize("nrays,more", [(2, 0), (2, 1), (10, 517), (7, 3)])
+def test_many_rows_as_few_at_a_time(gpu_lib, oracle, nrays, more):
+    """Around the row count from which a thread has several rows: the rays of a
+    list are those of its pieces, and those of the oracle."""
+    p = Problem(two_head_setup(8, 45.0, n=13), VoxelGrid((-0.02,) * 3, (0.004,) * 3, (10,) * 3),
+                nrays)
+    m = 800 * torch.cuda.get_device_properties(0).multi_processor_count + more
+    rows = torch.arange(m, dtype=torch.int32, device="cuda") * 7 % p.nchannels
+    got = api.rays(p, rows)
+    want = torch.cat([api.rays(p, r.contiguous()) for r in rows.split(30011)])
+    assert torch.equal(got.view(torch.int32), want.view(torch.int32))
+    pick = torch.tensor([0, 1, 3, 4, 127, 128, 511, 512, m // 2, m - 2, m - 1], device="cuda")
+    some = rows[pick].contiguous()
+    trig = api.trig_table(p).cpu().numpy()
+    rnd = api.dump_uniforms(p, some).cpu().numpy()
+    for i, (c, k) in enumerate(zip(some.tolist(), pick.tolist())):
+        w = np.asarray(oracle.rays(p, c, rnd[i], trig=trig), np.float32)
+        assert (got[k].cpu().numpy().view(np.uint32) == w.view(np.uint32)).all(), k
