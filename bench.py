@@ -272,7 +272,7 @@ def batch_measure(args, api, torch, st, nit: int = 10, grids=None, angles=None):
     angles = angles or BATCH_ANGLES
     members = batch_members(args.batch, grids=grids, angles=angles)
     # Problems are taken in draw order while their estimated matrix bytes fit
-    # the budget: the grouped layout holds 6 bytes per non-zero (value and
+    # the budget: the grouped layout holds about 6 bytes per non-zero (values and
     # group-local column rank; the CSR + column-major copy would need 16);
     # non-zeros per row from 512 sampled measured rows.
     free, _ = torch.cuda.mem_get_info()
