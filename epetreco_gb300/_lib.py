@@ -121,6 +121,8 @@ SIGNATURES = {
     "epet_mlem_update": [VP, VP, VP],
     "epet_mlem_loglik": [VP, C.POINTER(C.c_double), VP],
     "epet_trim_memory": [C.c_size_t],
+    "epet_selftest_window_error": [C.POINTER(ProblemC), C.POINTER(C.c_double),
+                                   C.POINTER(C.c_double)],
     "epet_selftest_division": [I64, C.c_uint64, C.POINTER(C.c_int64), VP],
     "epet_build_counters": [C.POINTER(C.c_int64), C.POINTER(C.c_int64)],
     "epet_ray_steps": [P, VP, I64, VP, C.POINTER(C.c_int64), VP],

@@ -71,6 +71,8 @@ void note_launch(int n = 1);
 
 // ------------------------------------------------------------ geometry
 
+constexpr float kWinPad = 1e-3f;  // margin of the walk's windows around the hull, in voxels
+
 // Per-problem constants shared by the kernels (passed by value).
 struct Geo {
   epet_problem p;
@@ -81,7 +83,7 @@ struct Geo {
   float fx_inv;      // 2^-s
   int fx_split;      // units = hi * 2^fx_split + lo, both parts summed in 32 bits
   float inv_pitch[3];  // 1 / grid pitch (approximate)
-  bool check_window;   // grid too fine for the window's margin: every cell tested
+  bool check_window;   // roundings not bound to stay in kWinPad: every cell tested
 };
 
 __device__ __forceinline__ float fmul(float a, float b) { return __fmul_rn(a, b); }

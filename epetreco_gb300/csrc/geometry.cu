@@ -183,6 +183,61 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
   }
 }
 
+// How far, in voxels, rounding can put a cell that a ray visits outside the
+// walk's window of its channel, for a ray that crosses the grid between its
+// end points while every line joining the crystals spans the grid (the only
+// rays whose cells are not tested; k_walk).  u = 2^-24, first order in u:
+//  * a crossing's parameter is RN(RN(P - r0) / RN(r1 - r0)), three roundings,
+//    so at any parameter of a cell's interval the line through the ray's float
+//    end points lies within 3 u |P - r0| <= 3 u D of the cell along every axis
+//    (D: the largest coordinate difference of two points of the heads).  Along
+//    the slab axis that is a way off the slab, and the hull's edges move by
+//    their slope times it: 3 u kappa D (kappa: of one channel, the longest over
+//    the shortest distance along the slab axis between points of its crystals);
+//  * the end points and the hull's corners are affine in the box coordinates,
+//    each rounded by at most u (R + 2 sqrt2 e) (R: the largest coordinate, e:
+//    the largest crystal edge): twice that, and again times the hull's slope S
+//    for its part along the slab axis;
+//  * a hull edge at a slab plane is ah + t w with t = RN(RN(X - as) RN(1 /
+//    RN(ds))): four roundings of t, one of w, one of the product, one of the
+//    sum: u (6 D + R).  (Between the planes the edges are straight, and a hull
+//    is convex: past a corner an edge's extension bounds it.);
+//  * its index, RN(RN(f - o) RN(1 / d)), and the planes RN(o + RN(k d)): u (3 +
+//    1) times the grid's extent, and u R.
+// 1 % more covers the second order.  Two 13 x 13 heads at 0.25 m (kappa 1.12,
+// S 1.12, D 0.52 m): 8.8 m u, so that pitches from 0.53 mm need no test; the
+// workloads' 2 mm leave a factor of 3.8.
+static double window_error(const epet_problem& p) {
+  const epet_setup& s = p.setup;
+  const epet_grid& g = p.grid;
+  const double e = std::max({(double)s.segx, (double)s.segy, (double)s.segz});
+  const double half_z = 0.5 * s.segz * std::max(s.n0z, s.n1z);
+  const double half_y = 0.5 * s.segy * std::max(s.n0y, s.n1y);
+  const double apart = std::fabs((double)s.pos1x - s.pos0x);
+  const double Dy = 0.5 * s.segy * ((double)s.n0y + s.n1y);
+  const double D = std::max(std::hypot(apart + s.segx, 0.5 * s.segz * ((double)s.n0z + s.n1z)), Dy);
+  double R = std::max(half_y, std::hypot(std::max(std::fabs((double)s.pos0x),
+                                                  std::fabs((double)s.pos1x)) + 0.5 * s.segx,
+                                         half_z));
+  double pitch = g.d[0], extent = 0.0;
+  for (int a = 0; a < 3; a++) {
+    const double o = g.o[a], n_d = (double)g.n[a] * g.d[a];
+    pitch = std::min(pitch, (double)g.d[a]);
+    extent = std::max(extent, n_d);
+    R = std::max({R, std::fabs(o), std::fabs(o + n_d)});
+  }
+  // Along the slab axis, the horizontal one that the line follows more closely,
+  // the crystals' centres are at least apart / sqrt2 from each other, and
+  // points of the crystals at most q nearer or farther.
+  const double A = apart * std::sqrt(0.5), q = std::hypot((double)s.segx, (double)s.segz);
+  if (!(A > q)) return INFINITY;
+  const double kappa = (A + q) / (A - q), S = std::max(kappa, Dy / (A - q));
+  const double roundings = (9.0 + 3.0 * kappa) * D +
+                           2.0 * (1.0 + S) * (R + 2.0 * std::sqrt(2.0) * e) + 2.0 * R +
+                           4.0 * extent;
+  return 1.01 * std::ldexp(roundings, -24) / pitch;
+}
+
 Geo make_geo(const epet_problem& p) {
   Geo G;
   G.p = p;
@@ -216,25 +271,7 @@ Geo make_geo(const epet_problem& p) {
   G.fx_inv = ldexpf(1.0f, -s);
   G.fx_split = b;
   for (int a = 0; a < 3; a++) G.inv_pitch[a] = 1.f / p.grid.d[a];
-  // The walk's windows leave a margin of 1e-3 voxel around the crystals'
-  // hull; a crossing's position carries a few roundings of the largest
-  // coordinate (2^-24 of it each).  Cells need no test against the window
-  // while 16 such roundings fit the margin (a pitch of 0.3 mm for heads
-  // 0.25 m away; the workloads' 2 mm leave a factor of 7).
-  double reach = 0.0;
-  for (double v : {(double)p.setup.pos0x, (double)p.setup.pos1x})
-    reach = std::max(reach, std::fabs(v) + p.setup.segx);
-  reach = std::max(reach, 0.5 * p.setup.segy * std::max(p.setup.n0y, p.setup.n1y));
-  reach = std::max(reach, 0.5 * p.setup.segz * std::max(p.setup.n0z, p.setup.n1z)) * 1.5;
-  double pitch = p.grid.d[0];
-  for (int a = 0; a < 3; a++) {
-    pitch = std::min(pitch, (double)p.grid.d[a]);
-    reach = std::max(reach, std::fabs((double)p.grid.o[a]));
-    reach = std::max(reach, std::fabs((double)p.grid.o[a] + (double)p.grid.n[a] * p.grid.d[a]));
-  }
-  // (cell indices from reciprocal pitches carry 2^-23 of their size: up to
-  // 2^11 cells along y; the walk takes at most 2^10 along x and z)
-  G.check_window = !(16.0 * std::ldexp(reach, -24) < 1e-3 * pitch) || p.grid.n[1] > 2048;
+  G.check_window = !(window_error(p) < kWinPad);
   return G;
 }
 
@@ -333,6 +370,15 @@ extern "C" {
 epet_status epet_build_counters(int64_t* overflow_rows_h, int64_t* exact_rows_h) {
   if (overflow_rows_h) *overflow_rows_h = overflow_rows_total();
   if (exact_rows_h) *exact_rows_h = exact_rows_total();
+  return EPET_OK;
+}
+
+epet_status epet_selftest_window_error(const epet_problem* p, double* voxels_h,
+                                       double* margin_h) {
+  EPET_CHECK(epet_problem_validate(p));
+  if (!voxels_h || !margin_h) return set_error(EPET_ERR_INVALID, "NULL output");
+  *voxels_h = window_error(*p);
+  *margin_h = kWinPad;
   return EPET_OK;
 }
 

@@ -46,7 +46,6 @@ constexpr int kWalkThreads = 128, kWalkThreadsFew = 64;
 constexpr int kFewRays = 80;     // rays of a channel up to which a CTA has kWalkThreadsFew threads
 constexpr int kGeomFloats = 56;  // per-channel geometry record (k_channel_geom)
 constexpr int kMaxSlabs = 1024;  // nx limit of the walk kernel
-constexpr float kWinPad = 1e-3f;  // window padding margin, in voxels (slab_window)
 
 enum WalkMode { kModeCsr = 0, kModeForward = 1, kModeBack = 2, kModeColSum = 3,
                 kModeWindow = 4, kModeMlem = 5 };
@@ -178,8 +177,8 @@ __device__ __forceinline__ float fval(int k) {
 // corners) inside the slab.  An index range is widened by one only on a side
 // whose extreme lies within kWinPad (in voxels) of a grid plane, where the
 // rounding of the hull's or a ray's arithmetic could put a hit in the
-// neighbouring cell (a few 1e-6 voxel here, a few 1e-4 at the largest index
-// counts: Geo::check_window); the window then holds about 1.7x a row's
+// neighbouring cell (at most 2.7e-4 voxel in the workloads: window_error,
+// geometry.cu); the window then holds about 1.7x a row's
 // non-zeros instead of 3.9x with a voxel of padding on every side (channels
 // of the full workload).
 __device__ void slab_window(const Geo& G, const float (*c0)[3], const float (*c1)[3],
@@ -313,9 +312,11 @@ struct WalkAxis {
 // grid, an endpoint inside the grid) must be reported.  A ray that crosses
 // the grid between its two endpoints stays inside the crystals' convex hull,
 // which the window of a channel whose crystals lie on both sides of the grid
-// covers with kWinPad of a voxel to spare, so its cells need no test; every
-// other ray (`chk`, also when the grid is too fine for that margin,
-// Geo::check_window) tests each cell and stops at the first one outside.  An untested ray's addresses stay in the pool whatever the window
+// covers with kWinPad of a voxel to spare; where the roundings of the ray's
+// and the hull's arithmetic are bound to stay below that margin (window_error,
+// geometry.cu) its cells need no test.  Every other ray (`chk`, also where
+// they are not, Geo::check_window) tests each cell and stops at the first one
+// outside.  An untested ray's addresses stay in the pool whatever the window
 // is: its columns lie between those of its entry and its exit, which are
 // checked against the table's box here (a column just off the box falls on
 // the border or the guard entries), and every table entry puts all z cells

@@ -177,6 +177,13 @@ epet_status epet_ray_steps(const epet_problem* p, const int32_t* rows_d, int64_t
  * results (0 expected).  Synchronous. */
 epet_status epet_selftest_division(int64_t n, uint64_t seed, int64_t* mismatches_h,
                                    epet_stream_t stream);
+/* Library self-test (no counterpart in the reference): how far, in voxels, the
+ * roundings of the walk can put a cell outside a channel's window (an upper
+ * bound; infinite where there is none), and the windows' margin.  Rays that
+ * cross the grid between the heads are walked without a test of their cells
+ * where the bound is below the margin.  Host only. */
+epet_status epet_selftest_window_error(const epet_problem* p, double* voxels_h,
+                                       double* margin_h);
 /* World-coordinate rays out_d[m][nrays][6] (RandRayGen, RayGenerators.hpp:
  * 15-40 with the per-channel seeding of getSystemMatrixFromWorkqueue.cu;
  * ReguRayGen, :46-66, for EPET_RAYS_REGULAR). */
