@@ -488,6 +488,11 @@ __device__ __forceinline__ float gq_from(uint32_t q) {
   return __half2float(__ushort_as_half((unsigned short)q));
 }
 
+// Whether a row touches an entry's column, from its value there: absent is +0
+// (values are positive; those that a 16-bit form rounds to zero are kept as -0,
+// which adds nothing either, but an infinite x or ratio must meet them).
+__device__ __forceinline__ bool touches(float v) { return __float_as_uint(v) != 0u; }
+
 // 16-bit values of a strip's rows and their scales, a warp per strip.
 template <int FMT>
 __global__ void k_group_quantise(const StripDesc* __restrict__ strips, int64_t nstrips,
@@ -518,7 +523,10 @@ __global__ void k_group_quantise(const StripDesc* __restrict__ strips, int64_t n
     const StripF v = val[d.start + k];
     StripH b;
 #pragma unroll
-    for (int j = 0; j < kStrip; j++) b.v[j] = gq_to<FMT>(__fdiv_rn(v.v[j], sc[j]));
+    for (int j = 0; j < kStrip; j++) {
+      b.v[j] = gq_to<FMT>(__fdiv_rn(v.v[j], sc[j]));
+      if (touches(v.v[j]) && b.v[j] == 0) b.v[j] = 0x8000;
+    }
     // FP32 position k of round u: half h, chunk l, entry 2 h + e of it; the
     // 16-bit values of a chunk lie together
     int to = k;
@@ -721,8 +729,8 @@ __device__ __forceinline__ void group_pass(const GroupIterArgs& a, const GroupHe
         for (int t = 0; t < 4; t++) {
           const float xv = xs[crank(l, t)];
           const float v0 = cvalue<FMT>(v, t, 0), v1 = cvalue<FMT>(v, t, 1);
-          if (v0 != 0.f) s0[0] = fmaf(v0, xv, s0[0]);
-          if (v1 != 0.f) s1[0] = fmaf(v1, xv, s1[0]);
+          if (touches(v0)) s0[0] = fmaf(v0, xv, s0[0]);
+          if (touches(v1)) s1[0] = fmaf(v1, xv, s1[0]);
         }
       }
     }
@@ -775,8 +783,8 @@ __device__ __forceinline__ void group_pass(const GroupIterArgs& a, const GroupHe
         for (int t = 0; t < 4; t++) {
           const float v0 = cvalue<FMT>(v, t, 0), v1 = cvalue<FMT>(v, t, 1);
           float c = cs[crank(l, t)];
-          if (v0 != 0.f) c = fmaf(v0, f0, c);
-          if (v1 != 0.f) c = fmaf(v1, f1, c);
+          if (touches(v0)) c = fmaf(v0, f0, c);
+          if (touches(v1)) c = fmaf(v1, f1, c);
           cs[crank(l, t)] = c;
         }
       }
