@@ -94,6 +94,11 @@ struct WalkArgs {
 // pool wherever the walk can take them (walk_ray): `gcol` bytes before the
 // column tables (a row of the table and an entry, filled like empty columns)
 // and `gz` bytes (the z cells) before and after the cells.
+//
+// The small layout (`lean`) has neither the guard bands nor the slab runs, 2 %
+// of the largest window at 128^3 voxels and most of the SM's memory for 10,000
+// cells along y: it is taken where the other does not fit (walk_lean).  Every
+// ray is then tested, and the columns' z runs are found slab by slab.
 struct WalkLayout {
   size_t planes, ztab, runs, pool, pext, lines, slabs, total;
   int gcol, gz;
@@ -105,16 +110,16 @@ constexpr int kHullLines = 16;  // lines of the hull joining the crystals' verti
 // the slab windows (slabs, at its end) only until the column table is built,
 // so the table must end before them and the cells, written afterwards, may
 // run over them.
-__host__ __device__ inline WalkLayout walk_layout(const epet_grid& g, int cap_cells) {
+__host__ __device__ inline WalkLayout walk_layout(const epet_grid& g, int cap_cells, bool lean) {
   const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
   const int nslab = nx > nz ? nx : nz;
   WalkLayout L;
-  L.gcol = ((ny + 2) * 4 + 15) & ~15;
-  L.gz = ((nz + 4) * 4 + 15) & ~15;
+  L.gcol = lean ? 0 : ((ny + 2) * 4 + 15) & ~15;
+  L.gz = lean ? 0 : ((nz + 4) * 4 + 15) & ~15;
   L.planes = 0;
   L.ztab = L.planes + align256((size_t)(nx + ny + nz + 5) * 4);  // + a guard entry at each end
   L.runs = L.ztab + align256((size_t)nz * 8);
-  L.pool = L.runs + align256((size_t)2 * (nx + ny) * 4);
+  L.pool = L.runs + (lean ? 0 : align256((size_t)2 * (nx + ny) * 4));
   const size_t pext_b = ((size_t)(nslab + 1) * 16 + 15) & ~size_t(15);
   const size_t slab_b = (size_t)16 * nslab;
   const size_t line_b = (size_t)kHullLines * 16;
@@ -548,7 +553,8 @@ static epet_status launch_channel_geom(const Geo& G, const int32_t* rows, int64_
 // walk, lo and hi sums apart, the hull from 16 lines, the z runs of a column
 // from per-x and per-y slab runs, one barrier per scan.  Registers are held
 // to 64 for 8 CTAs per SM (9 with 56 registers: 11.4 ms, 10 with 48: 12.3).
-template <int kMode, int kT>
+// kLean: the small layout of the shared memory (walk_layout).
+template <int kMode, int kT, bool kLean>
 __global__ void __launch_bounds__(kT, 1024 / kT)
 k_walk(WalkArgs args) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -559,7 +565,7 @@ k_walk(WalkArgs args) {
   constexpr int kMine = kRanges / kT;
   const Geo& G = args.G;
   const epet_grid& g = G.p.grid;
-  const WalkLayout lay = walk_layout(g, args.cap_cells);
+  const WalkLayout lay = walk_layout(g, args.cap_cells, kLean);
   Slab* slabs = reinterpret_cast<Slab*>(smem + lay.slabs);
   Window win;
   win.split = G.fx_split;
@@ -676,7 +682,7 @@ k_walk(WalkArgs args) {
   int* xr1 = xr0 + g.n[0];
   int* yr0 = xr1 + g.n[0];
   int* yr1 = yr0 + g.n[1];
-  if (sa == 2) {
+  if (!kLean && sa == 2) {
     for (int i = threadIdx.x; i < g.n[0]; i += kT) { xr0[i] = INT_MAX; xr1[i] = INT_MIN; }
     for (int i = threadIdx.x; i < g.n[1]; i += kT) { yr0[i] = INT_MAX; yr1[i] = INT_MIN; }
   }
@@ -697,13 +703,15 @@ k_walk(WalkArgs args) {
         } else {        // slab = z, rectangle over (x, y)
           xlo = min(xlo, sl.p0); xhi = max(xhi, sl.p0 + sl.wp - 1);
           ylo = min(ylo, sl.q0); yhi = max(yhi, sl.q0 + sl.wq - 1);
-          for (int j = sl.p0; j < sl.p0 + sl.wp; j++) {
-            atomicMin(&xr0[j], i);
-            atomicMax(&xr1[j], i);
-          }
-          for (int j = sl.q0; j < sl.q0 + sl.wq; j++) {
-            atomicMin(&yr0[j], i);
-            atomicMax(&yr1[j], i);
+          if (!kLean) {
+            for (int j = sl.p0; j < sl.p0 + sl.wp; j++) {
+              atomicMin(&xr0[j], i);
+              atomicMax(&xr1[j], i);
+            }
+            for (int j = sl.q0; j < sl.q0 + sl.wq; j++) {
+              atomicMin(&yr0[j], i);
+              atomicMax(&yr1[j], i);
+            }
           }
         }
       }
@@ -739,13 +747,13 @@ k_walk(WalkArgs args) {
             zlo = sl.z;
             zhi = sl.z + sl.w - 1;
           }
-        } else if (spans) {
+        } else if (!kLean && spans) {
           zlo = max(xr0[ix], yr0[iy]);
           zhi = max(min(xr1[ix], yr1[iy]), -1);
           if (zhi < zlo) zlo = 0, zhi = -1;
         } else {
-          // the rectangles of a bundle that ends inside the grid need not
-          // shrink steadily: the first and the last slab that holds (ix, iy)
+          // the first and the last slab that holds (ix, iy) (the rectangles of
+          // a bundle that ends inside the grid need not shrink steadily)
           zlo = 0, zhi = -1;
           for (int iz = ns - 1; iz >= 0; iz--) {
             const int4 sl = reinterpret_cast<const int4*>(slabs)[iz];
@@ -823,7 +831,7 @@ k_walk(WalkArgs args) {
   win.zrun = reinterpret_cast<const uint32_t*>(cz1);
   win.cbase_s = (uint32_t)__cvta_generic_to_shared(cz0);
   win.trash_out = W;
-  win.test_all = G.check_window || !spans;
+  win.test_all = G.check_window || !spans || kLean;
   // grid planes o + k d of the three axes (the walk's quotients read them)
   const int nplanes = g.n[0] + g.n[1] + g.n[2] + 3;
   float* planes = reinterpret_cast<float*>(smem + lay.planes) + 1;  // guards at -1 and nplanes
@@ -1082,11 +1090,6 @@ __global__ void k_offset_rowptr(int64_t* rp, int64_t n, const int64_t* base) {
 
 // ------------------------------------------------------------------ host
 
-static size_t walk_smem(const Geo& G, int cap_cells) {
-  static_assert(sizeof(Slab) == 16, "walk_layout assumes 16-byte slabs");
-  return walk_layout(G.p.grid, cap_cells).total;
-}
-
 // Dynamic shared memory a walk CTA may use on the current device (cached per
 // device; any thread).
 static int max_dyn_smem() {
@@ -1103,6 +1106,20 @@ static int max_dyn_smem() {
   return v;
 }
 
+// Whether a launch with this window capacity takes the small layout, and its
+// dynamic shared memory.
+static bool walk_lean(const Geo& G, int cap_cells) {
+  return walk_layout(G.p.grid, cap_cells, false).total > (size_t)max_dyn_smem();
+}
+static size_t walk_smem(const Geo& G, int cap_cells) {
+  static_assert(sizeof(Slab) == 16, "walk_layout assumes 16-byte slabs");
+  return walk_layout(G.p.grid, cap_cells, walk_lean(G, cap_cells)).total;
+}
+// (the small layout's windows end 4 KB below an SM's shared memory)
+static bool walk_fits(const Geo& G, int cap_cells) {
+  return !walk_lean(G, cap_cells) || walk_smem(G, cap_cells) + 3072 <= (size_t)max_dyn_smem();
+}
+
 // Measured, 122,412 channels (every 7th of 30 angles), forward projection, 64
 // against 128 threads: 32^3 voxels and 10 rays 1.26 / 1.59 ms, 20 rays 1.38 /
 // 1.69, 60 rays 1.77 / 2.21, 80 rays 2.09 / 2.32; 64^3 voxels and 60 rays 3.06
@@ -1112,18 +1129,21 @@ static int walk_threads(const Geo& G) {
   return G.p.nrays <= kFewRays ? kWalkThreadsFew : kWalkThreads;
 }
 
-template <int kMode, int kT>
+template <int kMode, int kT, bool kLean = false>
 static epet_status launch_walk_as(const WalkArgs& a, size_t smem, cudaStream_t st) {
-  EPET_CUDA(cudaFuncSetAttribute(k_walk<kMode, kT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-  k_walk<kMode, kT><<<(unsigned)a.m, kT, smem, st>>>(a);
+  const auto kernel = k_walk<kMode, kT, kLean>;
+  EPET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kernel<<<(unsigned)a.m, kT, smem, st>>>(a);
   EPET_LAUNCHED();
   return EPET_OK;
 }
 
 template <int kMode>
-static epet_status launch_walk(const WalkArgs& a, size_t smem, cudaStream_t st) {
+static epet_status launch_walk(const WalkArgs& a, cudaStream_t st) {
   if (a.m == 0) return EPET_OK;
+  const size_t smem = walk_smem(a.G, a.cap_cells);
+  // (one CTA an SM, whatever the rays)
+  if (walk_lean(a.G, a.cap_cells)) return launch_walk_as<kMode, kWalkThreads, true>(a, smem, st);
   if (walk_threads(a.G) == kWalkThreads) return launch_walk_as<kMode, kWalkThreads>(a, smem, st);
   return launch_walk_as<kMode, kWalkThreadsFew>(a, smem, st);
 }
@@ -1172,7 +1192,7 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
   a.win_cells = d_cells;
   a.geom = d_geom;
   epet_status rc = launch_channel_geom(G, d_rows, n, d_geom, st);
-  if (rc == EPET_OK) rc = launch_walk<kModeWindow>(a, walk_smem(G, 0), st);
+  if (rc == EPET_OK) rc = launch_walk<kModeWindow>(a, st);
   std::vector<int32_t> cells(n);
   if (rc == EPET_OK) {
     cudaError_t e = cudaMemcpyAsync(cells.data(), d_cells, n * 4, cudaMemcpyDeviceToHost, st);
@@ -1196,10 +1216,11 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
   const int p90 = percentile(90);
   int cap = std::max(256, (int)(p90 * 1.10) + 64);
   auto resident = [&](int c) {
+    if (walk_lean(G, c)) return 0;
     int n = 0;
     const bool few = walk_threads(G) == kWalkThreadsFew;
-    const void* k = few ? (const void*)k_walk<kModeCsr, kWalkThreadsFew>
-                        : (const void*)k_walk<kModeCsr, kWalkThreads>;
+    const void* k = few ? (const void*)k_walk<kModeCsr, kWalkThreadsFew, false>
+                        : (const void*)k_walk<kModeCsr, kWalkThreads, false>;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, walk_threads(G), walk_smem(G, c)) !=
         cudaSuccess)
       n = 0;
@@ -1308,19 +1329,19 @@ static epet_status redo_overflow(WalkArgs a, const int32_t* ovf_rows, int n, int
   w.m = n;
   w.win_cells = cells;
   w.geom = geom;
-  EPET_CHECK(launch_walk<kModeWindow>(w, walk_smem(a.G, 0), st));
+  EPET_CHECK(launch_walk<kModeWindow>(w, st));
   std::vector<int32_t> h(n);
   EPET_CUDA(cudaMemcpyAsync(h.data(), cells, n * 4, cudaMemcpyDeviceToHost, st));
   EPET_CUDA(cudaStreamSynchronize(st));
   int mx = 0;
   for (int v : h) mx = std::max(mx, v);
   *cap2 = std::max(mx, 1);
-  if (walk_smem(a.G, *cap2) > (size_t)max_dyn_smem())
+  if (!walk_fits(a.G, *cap2))
     return set_error(EPET_ERR_UNSUPPORTED, "per-row window of %d cells exceeds shared memory",
                      *cap2);
   // the column table must end before the slab windows, whatever the window
   const int room = *cap2 + 2 * std::max(a.G.p.grid.n[0], a.G.p.grid.n[2]);
-  if (walk_smem(a.G, room) <= (size_t)max_dyn_smem()) *cap2 = room;
+  if (walk_fits(a.G, room)) *cap2 = room;
   WalkArgs b = a;
   b.sel = sel;
   b.m = n;
@@ -1334,7 +1355,7 @@ static epet_status redo_overflow(WalkArgs a, const int32_t* ovf_rows, int n, int
     b.stage_val = *s2v;
   }
   EPET_CUDA(cudaMemsetAsync(a.overflow_count, 0, 4, st));
-  EPET_CHECK(launch_walk<kMode>(b, walk_smem(a.G, *cap2), st));
+  EPET_CHECK(launch_walk<kMode>(b, st));
   return EPET_OK;
 }
 
@@ -1431,7 +1452,7 @@ static epet_status run_walk(const Geo& G, const int32_t* rows, int64_t m,
     a.exact_count = flags + 2;
     EPET_CUDA(cudaMemsetAsync(flags, 0, 4, st));
     EPET_CUDA(cudaMemsetAsync(flags + 2, 0, 4, st));
-    EPET_CHECK(launch_walk<kMode>(a, walk_smem(G, cap_cells), st));
+    EPET_CHECK(launch_walk<kMode>(a, st));
     int32_t fl[3] = {0, 0, 0};
     EPET_CUDA(cudaMemcpyAsync(fl, flags, 12, cudaMemcpyDeviceToHost, st));
     EPET_CUDA(cudaStreamSynchronize(st));
@@ -1564,7 +1585,7 @@ static epet_status resolve_capacity(const Geo& G, int32_t max_row_nnz, cudaStrea
   } else {
     EPET_CHECK(sample_capacity(G, st, cap));
   }
-  if (walk_smem(G, *cap) > (size_t)max_dyn_smem())
+  if (!walk_fits(G, *cap))
     return set_error(EPET_ERR_UNSUPPORTED,
                      "per-row window of %d cells exceeds shared memory", *cap);
   if (G.p.grid.n[0] > kMaxSlabs || G.p.grid.n[2] > kMaxSlabs)
