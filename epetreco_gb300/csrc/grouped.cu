@@ -1221,10 +1221,11 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
   // The entries' arrays: how far the rows of a strip share columns is only
   // known once they are merged (0.6 entries per non-zero in scans).  Up to
   // 2^26 non-zeros the arrays are sized as if none were shared (0.7 GB at
-  // most, and a small reconstruction saves a launch and a round trip: 0.1 of
-  // 4.1 ms); beyond, a sample of the first cuts sizes them, and should the
-  // entries not fit after all, the layout is made again at the size it asked
-  // for.
+  // most) and the entries move into smaller ones afterwards: 16 problems of
+  // 24^3 and 32^3 hold 7.8 bytes per non-zero for 11.6, a reconstruction of 36M
+  // takes 3.77 ms for 3.76 (a launch and a round trip that count them first: 0.1
+  // more).  Beyond, a sample of the first cuts sizes them, and should the entries
+  // not fit after all, the layout is made again at the size it asked for.
   int64_t cap = nnz + 3 * std::max<int64_t>(m, 1);
   if (m > 0 && nnz > (int64_t(1) << 26)) {
     const int64_t every = std::max<int64_t>(1, ncut / kSampleCuts);
@@ -1286,6 +1287,25 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     cap = G->nent;
   }
   drop_scratch();
+  // (arrays that are too large are kept where there is no memory for the move)
+  auto fit = [&](auto*& a) -> cudaError_t {
+    auto* was = a;
+    void* p = nullptr;
+    if (dev_alloc(&p, std::max<size_t>(G->nent * sizeof(*a), 16), st) != cudaSuccess) {
+      cudaGetLastError();
+      return cudaSuccess;
+    }
+    a = static_cast<decltype(was)>(p);
+    const cudaError_t c =
+        cudaMemcpyAsync(a, was, G->nent * sizeof(*a), cudaMemcpyDeviceToDevice, st);
+    dev_free(was, st);
+    return c;
+  };
+  if (G->nent < cap - cap / 16) {
+    e = fit(G->val32);
+    if (e == cudaSuccess) e = fit(G->loc);
+    if (e != cudaSuccess) return fail(cuda_status(e, "group entries"));
+  }
   for (const GroupDesc& g : hg)
     if (g.nd <= kGroupCap) G->max_nd = std::max(G->max_nd, g.nd);
   const int64_t ns = std::max<int64_t>(G->nslots, 1);
