@@ -75,12 +75,14 @@ k_batch_rows(const BatchDesc* __restrict__ desc, const int64_t* __restrict__ til
     double part = 0.0;
     if constexpr (FWD) {
       if (r < d.m) {
-        const float v = row_dot<G, U, VEC>(d.col, d.val, d.x, d.row_ptr[r], d.row_ptr[r + 1], lg);
+        const float v = row_dot<G, U, VEC>(d.col, d.val, d.x, d.row_ptr[r], d.row_ptr[r + 1], lg,
+                                           group_mask<G>());
         if (lg == 0) EpiMlemForward{d.y, d.e, d.ybar}(r, v);
       }
     } else {
       if (r < d.V) {
-        const float c = row_dot<G, U, VEC>(d.row, d.cval, d.e, d.col_ptr[r], d.col_ptr[r + 1], lg);
+        const float c = row_dot<G, U, VEC>(d.row, d.cval, d.e, d.col_ptr[r], d.col_ptr[r + 1], lg,
+                                           group_mask<G>());
         if (lg == 0) part = EpiMlemUpdate{d.x, d.s, d.xnew, nullptr}(r, c);
       }
       block_sum_to(part, red, partial + tile);

@@ -28,13 +28,22 @@ inline int64_t plan_tiles(const RowPlan& p, int64_t nrows) {
 __device__ __forceinline__ float ld_stream(const float* p) { return __ldcs(p); }
 __device__ __forceinline__ int ld_stream(const int32_t* p) { return __ldcs(p); }
 
+// The lanes of a row's group, which take part in its shuffles: in the last
+// warp other groups' rows may be past the end, and their lanes skip the row.
+// (Taking them along with no entries cost an iteration of the full workload
+// 74.8 ms for 73.4: it sits in front of every row's first loads.)
+template <int G>
+__device__ __forceinline__ unsigned group_mask() {
+  return G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (threadIdx.x & 31 & ~(G - 1));
+}
+
 // Dot product of row [beg, end) with x by a group of G lanes, element-wise
 // loads (any alignment of idx / val).
 template <int G>
 __device__ __forceinline__ float group_dot_scalar(const int32_t* __restrict__ idx,
                                                   const float* __restrict__ val,
                                                   const float* __restrict__ x, int64_t beg,
-                                                  int64_t end, int lg) {
+                                                  int64_t end, int lg, unsigned mask) {
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
   int64_t k = beg + lg;
   for (; k + 3 * G < end; k += 4 * G) {
@@ -50,7 +59,7 @@ __device__ __forceinline__ float group_dot_scalar(const int32_t* __restrict__ id
   for (; k < end; k += G) a0 = fmaf(ld_stream(val + k), __ldg(x + ld_stream(idx + k)), a0);
   float a = (a0 + a1) + (a2 + a3);
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o, G);
+  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(mask, a, o, G);
   return a;
 }
 
@@ -64,7 +73,7 @@ template <int G, int U>
 __device__ __forceinline__ float group_dot_vec(const int32_t* __restrict__ idx,
                                                const float* __restrict__ val,
                                                const float* __restrict__ x, int64_t beg,
-                                               int64_t end, int lg) {
+                                               int64_t end, int lg, unsigned mask) {
   const int64_t h = min(end, (beg + 3) & ~int64_t(3));
   const int64_t t = max(h, end & ~int64_t(3));
   float acc[U];
@@ -115,7 +124,7 @@ __device__ __forceinline__ float group_dot_vec(const int32_t* __restrict__ idx,
 #pragma unroll
   for (int u = 1; u < U; u++) a += acc[u];
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o, G);
+  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(mask, a, o, G);
   return a;
 }
 
@@ -126,7 +135,7 @@ template <int G>
 __device__ __forceinline__ float2 group_dot2_scalar(const int32_t* __restrict__ idx,
                                                     const float* __restrict__ val,
                                                     const float2* __restrict__ x, int64_t beg,
-                                                    int64_t end, int lg) {
+                                                    int64_t end, int lg, unsigned mask) {
   float a[4] = {}, b[4] = {};
   int64_t k = beg + lg;
   for (; k + 3 * G < end; k += 4 * G) {
@@ -154,8 +163,8 @@ __device__ __forceinline__ float2 group_dot2_scalar(const int32_t* __restrict__ 
   float2 d = make_float2((a[0] + a[1]) + (a[2] + a[3]), (b[0] + b[1]) + (b[2] + b[3]));
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {
-    d.x += __shfl_xor_sync(0xffffffffu, d.x, o, G);
-    d.y += __shfl_xor_sync(0xffffffffu, d.y, o, G);
+    d.x += __shfl_xor_sync(mask, d.x, o, G);
+    d.y += __shfl_xor_sync(mask, d.y, o, G);
   }
   return d;
 }
@@ -164,7 +173,7 @@ template <int G, int U>
 __device__ __forceinline__ float2 group_dot2_vec(const int32_t* __restrict__ idx,
                                                  const float* __restrict__ val,
                                                  const float2* __restrict__ x, int64_t beg,
-                                                 int64_t end, int lg) {
+                                                 int64_t end, int lg, unsigned mask) {
   const int64_t h = min(end, (beg + 3) & ~int64_t(3));
   const int64_t t = max(h, end & ~int64_t(3));
   float a[U] = {}, b[U] = {};
@@ -230,8 +239,8 @@ __device__ __forceinline__ float2 group_dot2_vec(const int32_t* __restrict__ idx
   }
 #pragma unroll
   for (int o = G / 2; o > 0; o >>= 1) {
-    d.x += __shfl_xor_sync(0xffffffffu, d.x, o, G);
-    d.y += __shfl_xor_sync(0xffffffffu, d.y, o, G);
+    d.x += __shfl_xor_sync(mask, d.x, o, G);
+    d.y += __shfl_xor_sync(mask, d.y, o, G);
   }
   return d;
 }
@@ -242,7 +251,7 @@ __device__ __forceinline__ float2 group_dot2_vec(const int32_t* __restrict__ idx
 template <int G>
 __device__ __forceinline__ float group_sum_scalar(const int32_t* __restrict__ idx,
                                                   const float* __restrict__ x, int64_t beg,
-                                                  int64_t end, int lg) {
+                                                  int64_t end, int lg, unsigned mask) {
   float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
   int64_t k = beg + lg;
   for (; k + 3 * G < end; k += 4 * G) {
@@ -256,14 +265,14 @@ __device__ __forceinline__ float group_sum_scalar(const int32_t* __restrict__ id
   for (; k < end; k += G) a0 += __ldg(x + ld_stream(idx + k));
   float a = (a0 + a1) + (a2 + a3);
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o, G);
+  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(mask, a, o, G);
   return a;
 }
 
 template <int G, int U>
 __device__ __forceinline__ float group_sum_vec(const int32_t* __restrict__ idx,
                                                const float* __restrict__ x, int64_t beg,
-                                               int64_t end, int lg) {
+                                               int64_t end, int lg, unsigned mask) {
   const int64_t h = min(end, (beg + 3) & ~int64_t(3));
   const int64_t t = max(h, end & ~int64_t(3));
   float acc[U];
@@ -301,7 +310,7 @@ __device__ __forceinline__ float group_sum_vec(const int32_t* __restrict__ idx,
 #pragma unroll
   for (int u = 1; u < U; u++) a += acc[u];
 #pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o, G);
+  for (int o = G / 2; o > 0; o >>= 1) a += __shfl_xor_sync(mask, a, o, G);
   return a;
 }
 
@@ -310,16 +319,16 @@ template <int G, int U, bool VEC>
 __device__ __forceinline__ float row_dot(const int32_t* __restrict__ idx,
                                          const float* __restrict__ val,
                                          const float* __restrict__ x, int64_t beg, int64_t end,
-                                         int lg) {
-  if constexpr (VEC) return group_dot_vec<G, U>(idx, val, x, beg, end, lg);
-  else return group_dot_scalar<G>(idx, val, x, beg, end, lg);
+                                         int lg, unsigned mask) {
+  if constexpr (VEC) return group_dot_vec<G, U>(idx, val, x, beg, end, lg, mask);
+  else return group_dot_scalar<G>(idx, val, x, beg, end, lg, mask);
 }
 template <int G, int U, bool VEC>
 __device__ __forceinline__ float row_sum(const int32_t* __restrict__ idx,
                                          const float* __restrict__ x, int64_t beg, int64_t end,
-                                         int lg) {
-  if constexpr (VEC) return group_sum_vec<G, U>(idx, x, beg, end, lg);
-  else return group_sum_scalar<G>(idx, x, beg, end, lg);
+                                         int lg, unsigned mask) {
+  if constexpr (VEC) return group_sum_vec<G, U>(idx, x, beg, end, lg, mask);
+  else return group_sum_scalar<G>(idx, x, beg, end, lg, mask);
 }
 
 // Fixed-order block sum of one double per thread into *out (thread 0);

@@ -37,7 +37,8 @@ k_rows(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
     const int64_t row = tile * RPT + threadIdx.x / G;
     double part = 0.0;
     if (row < nrows) {
-      const float d = row_dot<G, U, VEC>(idx, val, x, ptr[row], ptr[row + 1], lg);
+      const float d =
+          row_dot<G, U, VEC>(idx, val, x, ptr[row], ptr[row + 1], lg, group_mask<G>());
       if (lg == 0) part = epi(row, d);
     }
     if (partial) block_sum_to(part, red, partial + tile);
@@ -58,7 +59,7 @@ k_sums(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
     const int64_t row = tile * RPT + threadIdx.x / G;
     double part = 0.0;
     if (row < nrows) {
-      const float d = row_sum<G, U, VEC>(idx, x, ptr[row], ptr[row + 1], lg);
+      const float d = row_sum<G, U, VEC>(idx, x, ptr[row], ptr[row + 1], lg, group_mask<G>());
       if (lg == 0) part = epi(row, d);
     }
     if (partial) block_sum_to(part, red, partial + tile);
@@ -78,8 +79,10 @@ k_rows_pair(const int64_t* __restrict__ ptr, const int32_t* __restrict__ idx,
     const int64_t row = tile * RPT + threadIdx.x / G;
     if (row >= nrows) continue;
     float2 d;
-    if constexpr (VEC) d = group_dot2_vec<G, U>(idx, val, x, ptr[row], ptr[row + 1], lg);
-    else d = group_dot2_scalar<G>(idx, val, x, ptr[row], ptr[row + 1], lg);
+    if constexpr (VEC)
+      d = group_dot2_vec<G, U>(idx, val, x, ptr[row], ptr[row + 1], lg, group_mask<G>());
+    else
+      d = group_dot2_scalar<G>(idx, val, x, ptr[row], ptr[row + 1], lg, group_mask<G>());
     if (lg == 0) {
       y0[row] = beta == 0.f ? alpha * d.x : alpha * d.x + beta * y0[row];
       y1[row] = beta == 0.f ? alpha * d.y : alpha * d.y + beta * y1[row];
