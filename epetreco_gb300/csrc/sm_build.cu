@@ -575,7 +575,6 @@ k_walk(WalkArgs args) {
   const ChannelLine& line = *reinterpret_cast<const ChannelLine*>(s_geom + 48);
   __shared__ int tot_cells[kT / 32], tot_kept[kT / 32];
   __shared__ int s_exact, s_box[4], s_nospan;
-  __shared__ double red_d[kT / 32];
   __shared__ float red_f[kRanges / 32];
   __shared__ float s_e;
   __shared__ int s_col[kRanges];
@@ -1036,7 +1035,6 @@ k_walk(WalkArgs args) {
       }
     }
   }
-  (void)red_d;
 }
 
 // Gather staged rows into their final CSR positions (warp per row).

@@ -480,12 +480,11 @@ k_digit_scan(int64_t* __restrict__ hist, int64_t* __restrict__ offs, int nchunks
 // One pass: histogram of `in`'s keys, scan, scatter from `in` to `out`.
 template <int BITS, typename K, typename V, typename In, typename Out>
 epet_status radix_pass(In in, Out out, int64_t n, int shift, int64_t* hist, int64_t* hist_scan,
-                       int64_t* scan_tmp, cudaStream_t st, const uint64_t* vary = nullptr) {
+                       cudaStream_t st, const uint64_t* vary = nullptr) {
   const RsGrid g = rs_grid(n);
   k_radix_hist<BITS, In><<<(unsigned)g.nchunks, kRsThreads, 0, st>>>(in, n, shift, g.tpc,
                                                                      g.nchunks, hist, vary);
   EPET_LAUNCHED();
-  (void)scan_tmp;
   k_digit_scan<<<1 << BITS, 256, 0, st>>>(hist, hist_scan, g.nchunks);
   EPET_LAUNCHED();
   const size_t dyn = (sizeof(K) + sizeof(V)) * (size_t)kRsTile;
@@ -647,7 +646,7 @@ static epet_status coo_passes(const CooIn& in, const CooOut& out, int64_t n, int
   using From = ArrIn<uint64_t, uint32_t>;
   const int passes = (bits + BITS - 1) / BITS;
   EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(in, Pairs{keys[0], vals[0]}, n, 0, hist,
-                                                   hist_scan, nullptr, st)));
+                                                   hist_scan, st)));
   if (passes == 1) {
     k_unpack_coo<<<ceil_div(n, 256), 256, 0, st>>>(keys[0], vals[0], n, out.colbits, out.row,
                                                    out.col, out.v);
@@ -658,10 +657,10 @@ static epet_status coo_passes(const CooIn& in, const CooOut& out, int64_t n, int
     const From src{keys[(p - 1) & 1], vals[(p - 1) & 1]};
     if (p + 1 < passes)
       EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(src, Pairs{keys[p & 1], vals[p & 1]}, n,
-                                                       BITS * p, hist, hist_scan, nullptr, st)));
+                                                       BITS * p, hist, hist_scan, st)));
     else
       EPET_CHECK((radix_pass<BITS, uint64_t, uint32_t>(src, out, n, BITS * p, hist, hist_scan,
-                                                       nullptr, st)));
+                                                       st)));
   }
   return EPET_OK;
 }
@@ -675,7 +674,7 @@ extern "C" {
 size_t epet_coo_sort_workspace_size(int64_t n) {
   const size_t hist = radix_hist_elems(n);
   return 2 * align256(n * 8) + 2 * align256(n * 4) + align256(hist * 8) +
-         align256((hist + 1) * 8) + align256(scan_tmp_elems(hist) * 8) + 256;
+         align256((hist + 1) * 8) + 256;
 }
 
 epet_status epet_coo_sort(float* val_d, int32_t* row_d, int32_t* col_d, int64_t n,
@@ -693,7 +692,6 @@ epet_status epet_coo_sort(float* val_d, int32_t* row_d, int32_t* col_d, int64_t 
   const size_t hn = radix_hist_elems(n);
   int64_t* hist = scr.take<int64_t>(hn);
   int64_t* hist_scan = scr.take<int64_t>(hn + 1);
-  int64_t* tmp = scr.take<int64_t>(scan_tmp_elems(hn));
   int* mx = scr.take<int>(4);
   if (scr.overrun) return set_error(EPET_ERR_INVALID, "internal: workspace size");
   // index ranges (ids must be non-negative)
@@ -708,7 +706,6 @@ epet_status epet_coo_sort(float* val_d, int32_t* row_d, int32_t* col_d, int64_t 
     return set_error(EPET_ERR_INVALID, "negative row/column index");
   const int colbits = std::max(1, bits_for(h_rng[1]));
   const int rowbits = std::max(1, bits_for(h_rng[0]));
-  (void)tmp;
   // 8-bit digits, or 9-bit ones where they save a pass
   const int bits = colbits + rowbits;
   uint64_t* keys[2] = {key, key2};
@@ -752,8 +749,7 @@ size_t epet_csr_to_csc_workspace_size(int64_t m, int64_t n, int64_t nnz) {
   const size_t hist = radix_hist_elems(nnz);
   const size_t pair = csc_passes(n) > 2 ? 2 : 1;  // key/value pairs between passes
   return 2 * align256(nnz * 4) + align256(nnz * 8) + (pair - 1) * (align256(nnz * 4) +
-         align256(nnz * 8)) + align256(hist * 8) + align256((hist + 1) * 8) +
-         align256(scan_tmp_elems(hist) * 8) + 256;
+         align256(nnz * 8)) + align256(hist * 8) + align256((hist + 1) * 8) + 256;
 }
 
 }  // extern "C"
@@ -785,7 +781,6 @@ static epet_status csr_to_csc_impl(const epet_csr* a, epet_csc* out, void* ws, s
   const size_t hn = radix_hist_elems(nnz);
   int64_t* hist = scr.take<int64_t>(hn);
   int64_t* hist_scan = scr.take<int64_t>(hn + 1);
-  int64_t* tmp = scr.take<int64_t>(scan_tmp_elems(hn));
   int32_t* rid = scr.take<int32_t>(nnz);
   if (scr.overrun) return set_error(EPET_ERR_INVALID, "internal: workspace size");
   const int bits = std::max(1, bits_for(a->n - 1));
@@ -797,32 +792,33 @@ static epet_status csr_to_csc_impl(const epet_csr* a, epet_csc* out, void* ws, s
   EPET_LAUNCHED();
   if (passes == 1) {
     // one pass: CSR -> CSC
-    EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(in, co, nnz, 0, hist, hist_scan, tmp, st)));
+    EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(in, co, nnz, 0, hist, hist_scan, st)));
   } else if (passes == 2) {
     // low digits: CSR -> (key, row|val); high digits -> CSC
     const int b0 = bits - 9;
     ArrOut<uint32_t, uint64_t> mid{key, pv};
     ArrIn<uint32_t, uint64_t> mid_in{key, pv};
-    if (b0 <= 8) EPET_CHECK((radix_pass<8, uint32_t, uint64_t>(in, mid, nnz, 0, hist, hist_scan, tmp, st)));
-    else EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(in, mid, nnz, 0, hist, hist_scan, tmp, st)));
+    if (b0 <= 8)
+      EPET_CHECK((radix_pass<8, uint32_t, uint64_t>(in, mid, nnz, 0, hist, hist_scan, st)));
+    else
+      EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(in, mid, nnz, 0, hist, hist_scan, st)));
     EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(mid_in, co, nnz, b0 <= 8 ? 8 : 9, hist,
-                                                  hist_scan, tmp, st)));
+                                                  hist_scan, st)));
   } else {
     // 9-bit digits from the least significant: CSR -> pair 0, pair k%2 ->
     // pair (k+1)%2, the last one -> CSC
     uint32_t* ks[2] = {key, key2};
     uint64_t* vs[2] = {pv, pv2};
     EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(in, ArrOut<uint32_t, uint64_t>{ks[0], vs[0]},
-                                                  nnz, 0, hist, hist_scan, tmp, st)));
+                                                  nnz, 0, hist, hist_scan, st)));
     for (int k = 1; k < passes; k++) {
       ArrIn<uint32_t, uint64_t> src{ks[(k - 1) & 1], vs[(k - 1) & 1]};
       if (k + 1 < passes)
         EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(src, ArrOut<uint32_t, uint64_t>{ks[k & 1],
                                                       vs[k & 1]}, nnz, 9 * k, hist, hist_scan,
-                                                      tmp, st)));
-      else
-        EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(src, co, nnz, 9 * k, hist, hist_scan, tmp,
                                                       st)));
+      else
+        EPET_CHECK((radix_pass<9, uint32_t, uint64_t>(src, co, nnz, 9 * k, hist, hist_scan, st)));
     }
   }
   // empty columns start where the next non-empty one does
@@ -843,13 +839,12 @@ epet_status csr_to_csc_positions(int64_t nnz, int64_t n, const int32_t* col, int
   Scratch scr;
   EPET_CHECK(scr.init(nullptr, 0,
                       2 * (passes > 2 ? 2 : 1) * align256(nnz * 4) + align256(hn * 8) +
-                          align256((hn + 1) * 8) + align256(scan_tmp_elems(hn) * 8) + 256,
+                          align256((hn + 1) * 8) + 256,
                       st));
   uint32_t* ks[2] = {scr.take<uint32_t>(nnz), passes > 2 ? scr.take<uint32_t>(nnz) : nullptr};
   uint32_t* vs[2] = {scr.take<uint32_t>(nnz), passes > 2 ? scr.take<uint32_t>(nnz) : nullptr};
   int64_t* hist = scr.take<int64_t>(hn);
   int64_t* hist_scan = scr.take<int64_t>(hn + 1);
-  int64_t* tmp = scr.take<int64_t>(scan_tmp_elems(hn));
   if (scr.overrun) return set_error(EPET_ERR_INVALID, "internal: workspace size");
   const int bits = std::max(1, bits_for(n - 1));
   PosIn in{col};
@@ -859,24 +854,23 @@ epet_status csr_to_csc_positions(int64_t nnz, int64_t n, const int32_t* col, int
   using K = uint32_t;
   using V = uint32_t;
   if (passes == 1) {
-    EPET_CHECK((radix_pass<9, K, V>(in, co, nnz, 0, hist, hist_scan, tmp, st)));
+    EPET_CHECK((radix_pass<9, K, V>(in, co, nnz, 0, hist, hist_scan, st)));
   } else if (passes == 2) {
     const int b0 = bits - 9;
     ArrOut<K, V> mid{ks[0], vs[0]};
-    if (b0 <= 8) EPET_CHECK((radix_pass<8, K, V>(in, mid, nnz, 0, hist, hist_scan, tmp, st)));
-    else EPET_CHECK((radix_pass<9, K, V>(in, mid, nnz, 0, hist, hist_scan, tmp, st)));
+    if (b0 <= 8) EPET_CHECK((radix_pass<8, K, V>(in, mid, nnz, 0, hist, hist_scan, st)));
+    else EPET_CHECK((radix_pass<9, K, V>(in, mid, nnz, 0, hist, hist_scan, st)));
     EPET_CHECK((radix_pass<9, K, V>(ArrIn<K, V>{ks[0], vs[0]}, co, nnz, b0 <= 8 ? 8 : 9, hist,
-                                    hist_scan, tmp, st)));
+                                    hist_scan, st)));
   } else {
-    EPET_CHECK((radix_pass<9, K, V>(in, ArrOut<K, V>{ks[0], vs[0]}, nnz, 0, hist, hist_scan, tmp,
-                                    st)));
+    EPET_CHECK((radix_pass<9, K, V>(in, ArrOut<K, V>{ks[0], vs[0]}, nnz, 0, hist, hist_scan, st)));
     for (int k = 1; k < passes; k++) {
       ArrIn<K, V> src{ks[(k - 1) & 1], vs[(k - 1) & 1]};
       if (k + 1 < passes)
         EPET_CHECK((radix_pass<9, K, V>(src, ArrOut<K, V>{ks[k & 1], vs[k & 1]}, nnz, 9 * k,
-                                        hist, hist_scan, tmp, st)));
+                                        hist, hist_scan, st)));
       else
-        EPET_CHECK((radix_pass<9, K, V>(src, co, nnz, 9 * k, hist, hist_scan, tmp, st)));
+        EPET_CHECK((radix_pass<9, K, V>(src, co, nnz, 9 * k, hist, hist_scan, st)));
     }
   }
   return suffix_min(col_ptr, n + 1, hist, st);
@@ -943,7 +937,7 @@ __global__ void k_unpack_coo_signed(const uint64_t* key, const uint32_t* v, int6
 static size_t noalloc_scratch_need(int64_t n) {
   const size_t hn = radix_hist_elems(n);
   return 2 * align256(n * 8) + 2 * align256(n * 4) + align256(hn * 8) + align256((hn + 1) * 8) +
-         align256(scan_tmp_elems(hn) * 8) + align256(16);
+         align256(16);
 }
 
 // Device address of the array, per device, for the context it was looked up
@@ -1009,7 +1003,6 @@ extern "C" epet_status epet_coo_sort_noalloc(float* val_d, int32_t* row_d, int32
   const size_t hn = radix_hist_elems(n);
   int64_t* hist = scr.take<int64_t>(hn);
   int64_t* hist_scan = scr.take<int64_t>(hn + 1);
-  int64_t* tmp = scr.take<int64_t>(scan_tmp_elems(hn));
   uint64_t* vary = scr.take<uint64_t>(2);
   if (scr.overrun) return set_error(EPET_ERR_INVALID, "internal: workspace size");
   // the array keeps the previous call's contents: the OR starts at 0, the AND at all ones
@@ -1025,7 +1018,7 @@ extern "C" epet_status epet_coo_sort_noalloc(float* val_d, int32_t* row_d, int32
   for (int shift = 0; shift < 64; shift += 8) {
     EPET_CHECK((radix_pass<8, uint64_t, uint32_t>(ArrIn<uint64_t, uint32_t>{sk, sv},
                                                   ArrOut<uint64_t, uint32_t>{dk, dv}, n, shift,
-                                                  hist, hist_scan, tmp, st, vary)));
+                                                  hist, hist_scan, st, vary)));
     std::swap(sk, dk);
     std::swap(sv, dv);
   }
