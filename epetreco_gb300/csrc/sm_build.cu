@@ -43,7 +43,8 @@ namespace epet {
 // phases around the walk weigh most and a CTA's threads share little work
 // (walk_threads).
 constexpr int kWalkThreads = 128, kWalkThreadsFew = 64;
-constexpr int kFewRays = 80;     // rays of a channel up to which a CTA has kWalkThreadsFew threads
+constexpr int kFewRays = 80;     // up to so many rays a channel and
+constexpr int kFewCells = 2048;  // cells of window capacity a CTA has kWalkThreadsFew threads
 constexpr int kGeomFloats = 56;  // per-channel geometry record (k_channel_geom)
 constexpr int kMaxSlabs = 1024;  // nx limit of the walk kernel
 
@@ -1118,13 +1119,21 @@ static bool walk_fits(const Geo& G, int cap_cells) {
   return !walk_lean(G, cap_cells) || walk_smem(G, cap_cells) + 3072 <= (size_t)max_dyn_smem();
 }
 
-// Measured, 122,412 channels (every 7th of 30 angles), forward projection, 64
-// against 128 threads: 32^3 voxels and 10 rays 1.26 / 1.59 ms, 20 rays 1.38 /
-// 1.69, 60 rays 1.77 / 2.21, 80 rays 2.09 / 2.32; 64^3 voxels and 60 rays 3.06
-// / 3.25, 80 rays 3.54 / 3.48, 100 rays 4.42 / 3.80 (52^3: 3.55 / 3.25).  32
-// threads win only at 24^3 (10 rays: 1.01).
-static int walk_threads(const Geo& G) {
-  return G.p.nrays <= kFewRays ? kWalkThreadsFew : kWalkThreads;
+// Fewer threads where the window is small: its cells are the threads' to
+// extract, and a large one, which keeps few CTAs resident, would leave an SM
+// with few warps.  Measured, 40,000 channels of 16 angles, 64 / 128 threads,
+// forward projection and build (ms), by voxels (2 mm) and the capacity that
+// the 90th percentile of the windows asks for:
+//   24^3 (672), 40 rays: 0.77 / 0.85, 1.74 / 1.99; 80: 0.90 / 0.93, 2.03 / 2.14
+//   52^3 (1,550), 40: 1.09 / 1.13, 2.37 / 2.63; 80: 1.29 / 1.27, 2.75 / 2.90;
+//                100: 1.52 / 1.35, 3.18 / 3.03
+//   64^3 (1,983), 40: 1.30 / 1.28, 2.75 / 2.95; 80: 1.53 / 1.44, 3.23 / 3.28
+//   80^3 (2,573), 40: 1.66 / 1.51, 3.41 / 3.31
+//   128^3 (4,730), 40: 3.77 / 2.76, 6.62 / 5.98
+//   40^3 of 0.3 mm (12,561), 40: 4.73 / 2.29, 5.50 / 4.50
+// 32 threads win only at 24^3 (10 rays).
+static int walk_threads(const Geo& G, int cap_cells) {
+  return G.p.nrays <= kFewRays && cap_cells <= kFewCells ? kWalkThreadsFew : kWalkThreads;
 }
 
 template <int kMode, int kT, bool kLean = false>
@@ -1142,7 +1151,8 @@ static epet_status launch_walk(const WalkArgs& a, cudaStream_t st) {
   const size_t smem = walk_smem(a.G, a.cap_cells);
   // (one CTA an SM, whatever the rays)
   if (walk_lean(a.G, a.cap_cells)) return launch_walk_as<kMode, kWalkThreads, true>(a, smem, st);
-  if (walk_threads(a.G) == kWalkThreads) return launch_walk_as<kMode, kWalkThreads>(a, smem, st);
+  if (walk_threads(a.G, a.cap_cells) == kWalkThreads)
+    return launch_walk_as<kMode, kWalkThreads>(a, smem, st);
   return launch_walk_as<kMode, kWalkThreadsFew>(a, smem, st);
 }
 
@@ -1216,11 +1226,10 @@ static epet_status sample_capacity(const Geo& G, cudaStream_t st, int* cap_out) 
   auto resident = [&](int c) {
     if (walk_lean(G, c)) return 0;
     int n = 0;
-    const bool few = walk_threads(G) == kWalkThreadsFew;
-    const void* k = few ? (const void*)k_walk<kModeCsr, kWalkThreadsFew, false>
-                        : (const void*)k_walk<kModeCsr, kWalkThreads, false>;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, walk_threads(G), walk_smem(G, c)) !=
-        cudaSuccess)
+    const int T = walk_threads(G, c);
+    const void* k = T == kWalkThreadsFew ? (const void*)k_walk<kModeCsr, kWalkThreadsFew, false>
+                                         : (const void*)k_walk<kModeCsr, kWalkThreads, false>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, T, walk_smem(G, c)) != cudaSuccess)
       n = 0;
     return n;
   };
