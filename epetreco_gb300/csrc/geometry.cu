@@ -97,19 +97,32 @@ __global__ void __launch_bounds__(128) k_uniforms(Geo G, const int32_t* __restri
 // typical step (consecutive channel ids) applies one jump matrix instead of
 // one per set bit of the channel id.
 //
-// A thread's own stores would be 16 bytes into 32 rows at a time, half a
-// sector each; a warp stages kStageRays rays of its 32 rows in shared memory
-// and writes each row's share as one run of whole sectors (rows of an even
-// number of rays on 16-byte boundaries; others keep the thread's own stores).
-// 395,460 rows of 100 rays: 0.88 -> 0.66 ms.
-//
-// For few rows a thread has one row and stores its rays itself: the kernel is
-// then bound by the latency of a thread's own rows, and four of them in series
-// took 387 us for 3,000 rows of 20 rays and 451 of 90, against 149 and 162
-// (80,000 rows: 390 and 489 against 304 and 345; 160,000: 443 and 549 against
-// 494 and 566, when the generator's jumps and the stores weigh more).
-constexpr int kRaysPerThread = 4, kRaysThreads = 128;
-constexpr int kRaysThreadsFew = 64, kRaysFewPerSm = 800;
+// The lines between the forms (launch_rays) are measured, in us, on random
+// rows of 228,488 channels | of 5.1M | on consecutive channels, whose jumps
+// cost least:
+//  * one row a thread: bound by a thread's own latency, which more rows in
+//    series add to (3,000 rows of 20 rays: 149, four rows a thread 248).
+//    30,000 rows of 10 rays with 1 / 2 / 4 rows: 151 / 150 / 201 | 186 / 201 /
+//    286 | 118 / 112 / 111; of 100: 178 / 185 / 285 | 211 / 237 / 382 | 141 /
+//    137 / 170; 50,000 of 10: 162 / 166 / 188 | 201 / 231 / 280 | 152 / 124 /
+//    116.  A single row: 121 / 110 / 106, so it takes the next form;
+//  * two rows: 70,000 of 10 rays 200 / 170 / 180 | 239 / 231 / 271 | 180 / 135
+//    / 120; 120,000 of 100 rays 379 / 331 / 354 | 465 / 441 / 474 | 365 / 278 /
+//    262: the more rays, the farther their stores spread;
+//  * four rows: beyond.  A thread's own stores are 16 bytes into 32 rows at a
+//    time, half a sector each; staged, a warp collects kStageRays rays of its
+//    32 rows in shared memory and writes each row's share as one run of whole
+//    sectors (rows of an even number of rays on 16-byte boundaries).  Direct /
+//    staged, 120,000 rows of 100 rays: 348 / 357 | 471 / 523 | 262 / 253; 200,000
+//    of 100: 441 / 386 | 626 / 603 | 373 / 327; 200,000 and 300,000 of 40: - |
+//    477 / 507, 588 / 599 | 243 / 243, 314 / 300; 500,000 and a million of 20: - |
+//    802 / 827, 1287 / 1278 | 410 / 399, 740 / 674; two million of 10: - | 1888 /
+//    2014 | 1117 / 1151.
+constexpr int kRaysThreads = 128, kRaysThreadsFew = 64;
+constexpr int kRaysOnePerSm = 200;                      // rows an SM up to which a thread has one
+constexpr int kRaysTwoPerSm = 330, kRaysTwoPerRay = 5;  // and two: 330 + 5 a ray (at most 100)
+// Staged beyond so many rows an SM and from so many rays a row and an SM.
+constexpr int kRaysStagedPerSm = 1300, kRaysStagedRays = 20, kRaysStagedSum = 65000;
 constexpr int kStageRays = 8, kStageVec = kStageRays * 24 / 16;  // rays and 16-byte pieces a row
 template <int kPer, int kT, bool kStaged>
 __global__ void __launch_bounds__(kT)
@@ -127,7 +140,6 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
     prev = rows[i0];
     if (!regular) curand_init(G.p.seed, (unsigned long long)prev, 0ull, &base);
   }
-  const bool staged = kStaged && (R & 1) == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0;
   const int lane = threadIdx.x & 31;
   float4(*st)[kStageVec + 1] = stage[kStaged ? threadIdx.x >> 5 : 0];
   for (int j = 0; j < kPer; j++) {
@@ -142,7 +154,7 @@ k_rays(Geo G, const int32_t* __restrict__ rows, int64_t m, float* __restrict__ o
         prev = cnl;
       }
     }
-    if (!staged) {
+    if (!kStaged) {
       if (live) emit_rays(G, cnl, base, false, reinterpret_cast<float2*>(out + i * (int64_t)R * 6));
       continue;
     }
@@ -275,19 +287,28 @@ Geo make_geo(const epet_problem& p) {
   return G;
 }
 
+template <int kPer, int kT, bool kStaged>
+static void launch_rays_as(const Geo& G, const int32_t* rows, int64_t m, float* out,
+                           cudaStream_t st) {
+  k_rays<kPer, kT, kStaged><<<ceil_div(ceil_div(m, kPer), kT), kT, 0, st>>>(G, rows, m, out);
+}
+
 epet_status launch_rays(const Geo& G, const int32_t* rows, int64_t m, float* out,
                         bool uniforms_only, cudaStream_t st) {
   if (m == 0) return EPET_OK;
-  const int T = 128;
+  const int T = 128, R = G.p.nrays;
+  const double per_sm = (double)m / num_sms();
   if (uniforms_only)
     k_uniforms<<<ceil_div(m, T), T, 0, st>>>(G, rows, m, out);
-  else if (m <= (int64_t)kRaysFewPerSm * num_sms())
-    k_rays<1, kRaysThreadsFew, false>
-        <<<ceil_div(m, kRaysThreadsFew), kRaysThreadsFew, 0, st>>>(G, rows, m, out);
+  else if (m > 1 && per_sm <= kRaysOnePerSm)
+    launch_rays_as<1, kRaysThreadsFew, false>(G, rows, m, out, st);
+  else if (per_sm <= kRaysTwoPerSm + kRaysTwoPerRay * std::min(R, 100))
+    launch_rays_as<2, kRaysThreadsFew, false>(G, rows, m, out, st);
+  else if (per_sm <= kRaysStagedPerSm || R < kRaysStagedRays || R * per_sm < kRaysStagedSum ||
+           (R & 1) != 0 || (reinterpret_cast<uintptr_t>(out) & 15) != 0)
+    launch_rays_as<4, kRaysThreads, false>(G, rows, m, out, st);
   else
-    k_rays<kRaysPerThread, kRaysThreads, true>
-        <<<ceil_div(ceil_div(m, kRaysPerThread), kRaysThreads), kRaysThreads, 0, st>>>(G, rows, m,
-                                                                                      out);
+    launch_rays_as<4, kRaysThreads, true>(G, rows, m, out, st);
   EPET_LAUNCHED();
   return EPET_OK;
 }
