@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(128) k_uniforms(Geo G, const int32_t* __restri
 //    802 / 827, 1287 / 1278 | 410 / 399, 740 / 674; two million of 10: - | 1888 /
 //    2014 | 1117 / 1151.
 constexpr int kRaysThreads = 128, kRaysThreadsFew = 64;
-constexpr int kRaysOnePerSm = 200;                      // rows an SM up to which a thread has one
+constexpr int kRaysOnePerSm = 300;                      // rows an SM up to which a thread has one
 constexpr int kRaysTwoPerSm = 330, kRaysTwoPerRay = 5;  // and two: 330 + 5 a ray (at most 100)
 // Staged beyond so many rows an SM and from so many rays a row and an SM.
 constexpr int kRaysStagedPerSm = 1300, kRaysStagedRays = 20, kRaysStagedSum = 65000;

@@ -27,7 +27,7 @@ def rows_and_rays():
     staged += [(3251, 5, 20)]
     direct = [(1300, 0, 50), (1300, 5, 48), (1300, 3, 51), (3249, 2, 20), (3300, 1, 19)]
     two = [(330 + 5 * nrays, more, nrays) for nrays in (2, 7) for more in (-1, 0, 1, 2, 3)]
-    one = [(200, more, nrays) for nrays in (3, 8) for more in (-1, 0, 1, 2)]
+    one = [(300, more, nrays) for nrays in (3, 8) for more in (-1, 0, 1, 2)]
     return staged + direct + two + one + [(0, 1, 10), (0, 2, 10), (0, 3, 11)]
 
 
