@@ -641,8 +641,11 @@ __device__ __forceinline__ GroupHead group_head(const GroupIterArgs& a, const Gr
 // The next strip's entries are in flight while a strip is reduced and added.
 // Bound by the latency of those loads and of the chain from a strip's sums to
 // its corrections.  One row at a time: 120 M instructions, 279 us for the
-// first 400,000 channels of the full workload, 4.24 ms an iteration at full
-// size (the slot sums included); in strips of two 87 M, 255 us, 3.66 ms.
+// first 400,000 channels of the full workload, 4.17 ms an iteration at full
+// size (the slot sums included); in strips of two 87 M, 238 us, 3.59 ms.  Where
+// few channels are measured rows share few columns and strips lose: the full
+// geometry with 1 % of the channels 221 us an iteration for 199, with 10 % 691
+// for 742.
 // Tried: strips of four (more registers than a thread has), a ring in shared
 // memory filled by asynchronous copies ahead of the pass (5.2 ms: a third of
 // the tables' room and twice the instructions).

@@ -90,8 +90,8 @@ struct WalkArgs {
 // and the pool, each on a 256-byte boundary.  The pool holds,
 // per channel, the window's column tables (8 bytes per column, border
 // included) followed by the two 32-bit sum words of every window cell and of
-// the two trash cells (8 bytes per cell): a channel needs columns + cells + 2
-// <= cap_cells.  Guard bands keep a ray's table and cell addresses inside the
+// two more, the first of which counts hits outside the window (8 bytes per
+// cell): a channel needs columns + cells + 2 <= cap_cells.  Guard bands keep a ray's table and cell addresses inside the
 // pool wherever the walk can take them (walk_ray): `gcol` bytes before the
 // column tables (a row of the table and an entry, filled like empty columns)
 // and `gz` bytes (the z cells) before and after the cells.

@@ -415,18 +415,22 @@ typedef struct {
 
 /* Layouts of a reconstruction's stored matrix.  GROUPED: rows cut into
  * groups of consecutive rows (crystal-pair order) whose distinct columns fit
- * a per-warp table in shared memory; each entry keeps its value and a 2-byte
- * rank of its column in the group's table (6 bytes per entry in FP32, 4 in
- * BF16/FP16); one pass over the entries per iteration gives A x, the ratio
- * and A^T e, the latter summed per column in a fixed order; supported up to
- * 819,200 voxels.  CSC: the CSR and its column-major copy (16 bytes per entry
- * in FP32), the transpose product over the copy.  AUTO: GROUPED for FP32
- * values where supported, else CSC (the 16-bit forms run faster in CSC: their
- * grouped pass is bound by shared memory).  Both are deterministic.  The
- * 16-bit forms scale the sensitivity per column by the ratio of the column
- * sums of the values their transpose product uses to the FP32 column sums
- * (over the measured rows), so the iterations do not drift by the rounding
- * of the values. */
+ * a per-warp table in shared memory, neighbouring rows merged in pairs: an
+ * entry is a column that either row touches, the two rows' values and a 2-byte
+ * rank of the column in the group's table (10 bytes in FP32, 6 in BF16/FP16,
+ * for 1.7 non-zeros where most channels are measured, about 1 where few are;
+ * with the tables about 8 bytes held per non-zero in FP32); one pass over the
+ * entries per iteration gives A x, the ratio and A^T e, the latter summed per
+ * column in a fixed order; supported up to 819,200 voxels.  CSC: the CSR and its
+ * column-major copy (16 bytes per non-zero in FP32, 9 in the 16-bit forms), the
+ * transpose product over the copy.  AUTO: GROUPED for FP32 values where
+ * supported, else CSC.  (The 16-bit forms run faster in GROUPED, 3.31 against
+ * 4.13 ms an iteration at 52^3 voxels and 5.1M rows, and nearer to 64-bit
+ * images: ask for it by name.  The two forms' images differ by about 1e-4.)
+ * Both are deterministic.  The 16-bit forms scale the sensitivity per column by
+ * the ratio of the column sums of the values their transpose product uses to
+ * the FP32 column sums (over the measured rows), so the iterations do not drift
+ * by the rounding of the values. */
 enum { EPET_LAYOUT_AUTO = 0, EPET_LAYOUT_GROUPED = 1, EPET_LAYOUT_CSC = 2 };
 
 /* Builds the system matrix for the measured rows (rows_d channel ids, in
