@@ -272,7 +272,7 @@ def batch_measure(args, api, torch, st, nit: int = 10, grids=None, angles=None):
     angles = angles or BATCH_ANGLES
     members = batch_members(args.batch, grids=grids, angles=angles)
     # Problems are taken in draw order while their estimated matrix bytes fit
-    # the budget: the grouped layout holds 7.8 to 8.2 bytes per non-zero (6 of
+    # the budget: the grouped layout holds 7.6 to 8.2 bytes per non-zero (6 of
     # them values and group-local column ranks, the rest the groups' tables and
     # slots; the CSR + column-major copy would need 16), and the set-up of one
     # more problem its matrix besides; non-zeros per row from 512 sampled

@@ -450,7 +450,10 @@ k_group_tables(RowSource A, const GroupDesc* __restrict__ groups, int64_t m, int
   }
 }
 
-constexpr int64_t kSampleCuts = 2048;  // first cuts counted to size the entries' arrays
+// First cuts counted to size the entries' arrays, and the non-zeros from which
+// they are.
+constexpr int64_t kSampleCuts = 2048, kSampleCutsFew = 512;
+constexpr int64_t kSampleNnz = int64_t(1) << 24;
 
 // Dynamic shared memory of k_group_tables: the strips' bitmaps, the group's
 // bitmap and its word ranks, later a list of ranks per warp.
@@ -1222,16 +1225,19 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     return EPET_OK;
   };
   // The entries' arrays: how far the rows of a strip share columns is only
-  // known once they are merged (0.6 entries per non-zero in scans).  Up to
-  // 2^26 non-zeros the arrays are sized as if none were shared (0.7 GB at
-  // most) and the entries move into smaller ones afterwards: 16 problems of
-  // 24^3 and 32^3 hold 7.8 bytes per non-zero for 11.6, a reconstruction of 36M
-  // takes 3.77 ms for 3.76 (a launch and a round trip that count them first: 0.1
-  // more).  Beyond, a sample of the first cuts sizes them, and should the entries
-  // not fit after all, the layout is made again at the size it asked for.
+  // known once they are merged (0.6 entries per non-zero in scans).  A sample of
+  // the first cuts sizes them, one wave of blocks for up to 2^26 non-zeros, where
+  // it weighs; should the entries not fit after all, the layout is made again at
+  // the size it asked for.  Up to 2^24 non-zeros the arrays are sized as if no
+  // columns were shared (0.17 GB at most), and the entries move into smaller ones
+  // afterwards.  16 problems of 24^3 and 32^3 hold 7.6 bytes per non-zero (11.6
+  // in arrays for unshared columns).  Whole reconstructions of 36M, 49M (two
+  // iterations) and 55M non-zeros, in ms, with the sample 3.70, 4.82, 6.00, moved
+  // 3.74, 4.79, 6.01 to 6.08, in arrays for unshared columns 3.71, 4.76, 5.95.
   int64_t cap = nnz + 3 * std::max<int64_t>(m, 1);
-  if (m > 0 && nnz > (int64_t(1) << 26)) {
-    const int64_t every = std::max<int64_t>(1, ncut / kSampleCuts);
+  if (m > 0 && nnz > kSampleNnz) {
+    const bool few = nnz <= (int64_t(1) << 26);
+    const int64_t every = std::max<int64_t>(1, ncut / (few ? kSampleCutsFew : kSampleCuts));
     const int64_t sampled = (ncut + every - 1) / every;
     e = cudaMemsetAsync(cursor, 0, 8, st);
     if (e == cudaSuccess) {
@@ -1244,7 +1250,7 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     int64_t n = 0;
     const epet_status rc = e == cudaSuccess ? read_cursor(&n) : cuda_status(e, "group sample");
     if (rc != EPET_OK) return fail(rc);
-    cap = (int64_t)((double)n / sampled * ncut * 1.03) + 65536;
+    cap = (int64_t)((double)n / sampled * ncut * (few ? 1.08 : 1.03)) + 65536;
   }
   std::vector<GroupDesc> hg;
   for (int attempt = 0;; attempt++) {
@@ -1304,7 +1310,7 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     dev_free(was, st);
     return c;
   };
-  if (G->nent < cap - cap / 16) {
+  if (G->nent < cap - cap / 8) {
     e = fit(G->val32);
     if (e == cudaSuccess) e = fit(G->loc);
     if (e != cudaSuccess) return fail(cuda_status(e, "group entries"));
