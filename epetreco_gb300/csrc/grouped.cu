@@ -991,9 +991,11 @@ k_group_colsum(GroupIterArgs a) {
 
 static int bitmap_words(int64_t V) { return (int)((V + 31) / 32); }
 
-bool grouped_supported(int64_t V, int64_t m) {
-  // a V-bit map and its prefix in a table block's shared memory; int32 rows
-  return V > 0 && (size_t)bitmap_words(V) * 8 <= (size_t)200 * 1024 && m < INT32_MAX;
+// A bitmap over the columns and its prefix in a table block's shared memory.
+constexpr int64_t kMaxColumns = 819200;
+
+bool grouped_supported(int64_t V, int64_t m) {  // (int32 rows)
+  return V > 0 && V <= kMaxColumns && m < INT32_MAX;
 }
 
 void grouped_free(GroupedMatrix* G, cudaStream_t st) {
@@ -1024,7 +1026,7 @@ static epet_status form_groups(const RowSource& A, int64_t m, int64_t ncols, int
   const int nwords = bitmap_words(ncols);
   const int64_t ncut = (m + kGroupFirstRows - 1) / kGroupFirstRows;
   EPET_CUDA(cudaFuncSetAttribute(k_group_distinct, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 nwords * 4));
+                                 bitmap_words(kMaxColumns) * 4));
   // every first cut counted, those that fit laid out
   std::vector<int32_t> cut_nd(ncut);
   {
@@ -1207,8 +1209,9 @@ epet_status grouped_build(const RowSource& A, int64_t m, int64_t ncols, int64_t 
     if (e_ != cudaSuccess) return fail(cuda_status(e_, "grouped allocation " #ptr)); \
   } while (0)
   const int nwords = bitmap_words(ncols);
+  // (limits for any grid: another thread may be between its own and its launch)
   cudaError_t e = cudaFuncSetAttribute(k_group_tables, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)table_smem(nwords));
+                                       (int)table_smem(bitmap_words(kMaxColumns)));
   if (e == cudaSuccess)
     e = cudaFuncSetAttribute(k_group_tables, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
   if (e == cudaSuccess) e = allow_pass_smem();

@@ -23,6 +23,12 @@ size_t radix_hist_elems(int64_t n);
 epet_status csr_to_csc_positions(int64_t nnz, int64_t n, const int32_t* col, int64_t* col_ptr,
                                  uint32_t* pos, cudaStream_t st);
 
+// Dynamic shared memory that a CTA of k_walk or k_values may use on the current
+// device (cached per device; any thread).  A kernel's limit is the process's, so
+// every launch sets it to the same value, never to its own size: another thread's
+// smaller one would come between the setting and the launch.
+int max_dyn_smem();
+
 // Row walk configuration chosen for a problem (per-row accumulator size).
 int auto_row_capacity(const epet_problem& p);
 int64_t exact_rows_total();

@@ -1089,9 +1089,7 @@ __global__ void k_offset_rowptr(int64_t* rp, int64_t n, const int64_t* base) {
 
 // ------------------------------------------------------------------ host
 
-// Dynamic shared memory a walk CTA may use on the current device (cached per
-// device; any thread).
-static int max_dyn_smem() {
+int max_dyn_smem() {
   static std::atomic<int> cache[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -1099,7 +1097,7 @@ static int max_dyn_smem() {
   int v = slot ? slot->load(std::memory_order_relaxed) : 0;
   if (v == 0) {
     cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    v -= 1024;  // static shared memory of the kernel
+    v -= 1024;  // static shared memory of the kernels
     if (slot) slot->store(v, std::memory_order_relaxed);
   }
   return v;
@@ -1139,7 +1137,8 @@ static int walk_threads(const Geo& G, int cap_cells) {
 template <int kMode, int kT, bool kLean = false>
 static epet_status launch_walk_as(const WalkArgs& a, size_t smem, cudaStream_t st) {
   const auto kernel = k_walk<kMode, kT, kLean>;
-  EPET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  EPET_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 max_dyn_smem()));
   kernel<<<(unsigned)a.m, kT, smem, st>>>(a);
   EPET_LAUNCHED();
   return EPET_OK;

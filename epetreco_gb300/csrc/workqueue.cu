@@ -373,11 +373,11 @@ epet_status launch_values(const Geo& G, const float* rays, const int32_t* ray_ro
   const dim3 grid((unsigned)m, slices);
   if (exact) {
     EPET_CUDA(cudaFuncSetAttribute(k_values<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+                                   max_dyn_smem()));
     k_values<true><<<grid, kValThreads, smem, st>>>(G, rays, ray_row, m, row_ptr, col, val);
   } else {
     EPET_CUDA(cudaFuncSetAttribute(k_values<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)smem));
+                                   max_dyn_smem()));
     k_values<false><<<grid, kValThreads, smem, st>>>(G, rays, ray_row, m, row_ptr, col, val);
   }
   EPET_LAUNCHED();
